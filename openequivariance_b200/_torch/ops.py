@@ -315,7 +315,8 @@ def _register_tp_autograd():
         dx, dy, dw = _ops().jit_tp_backward(ctx.kernel, ctx.hash, ctx.L1_in, ctx.L2_in, ctx.W, grad_out)
         return None, None, dx, dy, dw, None
 
-    torch.library.register_autograd(f"{NS}::jit_tp_forward", fwd_backward, setup_context=fwd_setup)
+    if not CPP_OPS:      # (the C++ operators carry their own)
+        torch.library.register_autograd(f"{NS}::jit_tp_forward", fwd_backward, setup_context=fwd_setup)
 
     def bwd_setup(ctx, inputs, output):
         ctx.kernel, ctx.hash, ctx.L1_in, ctx.L2_in, ctx.W, ctx.L3_grad = inputs
@@ -328,7 +329,8 @@ def _register_tp_autograd():
                                                        ctx.L3_grad, a, b, c)
         return None, None, dx, dy, dw, dg
 
-    torch.library.register_autograd(f"{NS}::jit_tp_backward", bwd_backward, setup_context=bwd_setup)
+    if not CPP_OPS:
+        torch.library.register_autograd(f"{NS}::jit_tp_backward", bwd_backward, setup_context=bwd_setup)
 
     def dbl_setup(ctx, inputs, output):
         ctx.kernel, ctx.hash = inputs[0], inputs[1]
@@ -381,7 +383,8 @@ def _register_conv_autograd():
                                               ctx.rows, ctx.cols, ctx.workspace, ctx.perm)
         return None, None, dx, dy, dw, None, None, None, None, None
 
-    torch.library.register_autograd(f"{NS}::jit_conv_forward", fwd_backward, setup_context=fwd_setup)
+    if not CPP_OPS:
+        torch.library.register_autograd(f"{NS}::jit_conv_forward", fwd_backward, setup_context=fwd_setup)
 
     def bwd_setup(ctx, inputs, output):
         (ctx.kernel, ctx.hash, ctx.L1_in, ctx.L2_in, ctx.W, ctx.L3_grad, ctx.rows, ctx.cols, ctx.workspace,
@@ -396,7 +399,8 @@ def _register_conv_autograd():
                                                          ctx.perm)
         return None, None, dx, dy, dw, dg, None, None, None, None
 
-    torch.library.register_autograd(f"{NS}::jit_conv_backward", bwd_backward, setup_context=bwd_setup)
+    if not CPP_OPS:
+        torch.library.register_autograd(f"{NS}::jit_conv_backward", bwd_backward, setup_context=bwd_setup)
 
     def dbl_setup(ctx, inputs, output):
         ctx.kernel, ctx.hash = inputs[0], inputs[1]

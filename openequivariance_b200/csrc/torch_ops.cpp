@@ -5,14 +5,17 @@
 // Same schemas, same argument checks with the same messages, outputs allocated with the inputs' options, launches on
 // the current CUDA stream of the tensors' device.  Being registered in C++, the operators exist in any process that
 // loads this library (an AOTInductor package run from C++ included) and a call costs a few microseconds of host time;
-// the Python module openequivariance_b200/_torch/ops.py adds the fake, autograd and autocast registrations on top and
-// carries an equivalent Python implementation for installations where this file was not built.
+// the autograd chain forward -> backward -> double backward is registered here too, so that recording and running a
+// gradient never enters Python.  The Python module openequivariance_b200/_torch/ops.py adds the fake and autocast
+// registrations and the third order on top and carries an equivalent Python implementation for installations where this
+// file was not built.
 //
 // Built by openequivariance_b200/build_native.py (g++ against the installed torch; links liboeq_b200.so).
 
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/custom_function.h>
 #include <torch/library.h>
 
 #include <memory>
@@ -250,6 +253,175 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> jit_conv_double_backw
     return {dx, dy, dw, dg};
 }
 
+// ---- autograd chain: forward -> backward -> double backward ----------------------------------------------------
+// An op's autograd kernel costs host time on every call, and small calls are nothing but host time: the same chain
+// registered from Python took 125 us for forward + gradients of a 1,000-item product whose two kernels run for 6 us.
+// A kernel with nothing to record redispatches below autograd at once.
+//
+// The index tensors, the workspace and the descriptor travel in saved_data (they are not differentiable); the operands
+// that the next order differentiates are saved variables.
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+typedef std::tuple<at::Tensor, at::Tensor, at::Tensor> Three;
+typedef std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> Four;
+
+typedef at::Tensor TpFwdSig(const at::Tensor&, int64_t, const at::Tensor&, const at::Tensor&, const at::Tensor&, int64_t);
+typedef Three TpBwdSig(const at::Tensor&, int64_t, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&);
+typedef Four TpDblSig(const at::Tensor&, int64_t, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
+                      const at::Tensor&, const at::Tensor&, const at::Tensor&);
+typedef at::Tensor ConvFwdSig(const at::Tensor&, int64_t, const at::Tensor&, const at::Tensor&, const at::Tensor&, int64_t,
+                              const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&);
+typedef Three ConvBwdSig(const at::Tensor&, int64_t, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
+                         const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&);
+typedef Four ConvDblSig(const at::Tensor&, int64_t, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
+                        const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
+                        const at::Tensor&, const at::Tensor&);
+const c10::TypedOperatorHandle<TpFwdSig>& tp_fwd_op() {
+    static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("libtorch_tp_jit::jit_tp_forward", "").typed<TpFwdSig>();
+    return op;
+}
+const c10::TypedOperatorHandle<TpBwdSig>& tp_bwd_op() {
+    static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("libtorch_tp_jit::jit_tp_backward", "").typed<TpBwdSig>();
+    return op;
+}
+const c10::TypedOperatorHandle<TpDblSig>& tp_dbl_op() {
+    static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("libtorch_tp_jit::jit_tp_double_backward", "").typed<TpDblSig>();
+    return op;
+}
+const c10::TypedOperatorHandle<ConvFwdSig>& conv_fwd_op() {
+    static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("libtorch_tp_jit::jit_conv_forward", "").typed<ConvFwdSig>();
+    return op;
+}
+const c10::TypedOperatorHandle<ConvBwdSig>& conv_bwd_op() {
+    static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("libtorch_tp_jit::jit_conv_backward", "").typed<ConvBwdSig>();
+    return op;
+}
+const c10::TypedOperatorHandle<ConvDblSig>& conv_dbl_op() {
+    static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("libtorch_tp_jit::jit_conv_double_backward", "").typed<ConvDblSig>();
+    return op;
+}
+
+template <class... Ts>
+bool records(const Ts&... ts) { return at::GradMode::is_enabled() && (ts.requires_grad() || ...); }
+
+void keep(AutogradContext* ctx, const at::Tensor& json, int64_t hash) {
+    ctx->saved_data["json"] = json;
+    ctx->saved_data["hash"] = hash;
+}
+void keep(AutogradContext* ctx, const at::Tensor& json, int64_t hash, const at::Tensor& rows, const at::Tensor& cols,
+          const at::Tensor& workspace, const at::Tensor& perm) {
+    keep(ctx, json, hash);
+    ctx->saved_data["rows"] = rows;
+    ctx->saved_data["cols"] = cols;
+    ctx->saved_data["workspace"] = workspace;
+    ctx->saved_data["perm"] = perm;
+}
+at::Tensor kept(AutogradContext* ctx, const char* name) { return ctx->saved_data[name].toTensor(); }
+int64_t kept_hash(AutogradContext* ctx) { return ctx->saved_data["hash"].toInt(); }
+
+struct TpForward : torch::autograd::Function<TpForward> {
+    static at::Tensor forward(AutogradContext* ctx, const at::Tensor& json, int64_t hash, const at::Tensor& x, const at::Tensor& y,
+                              const at::Tensor& W, int64_t L3_dim) {
+        keep(ctx, json, hash);
+        ctx->save_for_backward({x, y, W});
+        at::AutoDispatchBelowADInplaceOrView below;
+        return tp_fwd_op().call(json, hash, x, y, W, L3_dim);
+    }
+    static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
+        const variable_list v = ctx->get_saved_variables();
+        auto [dx, dy, dw] = tp_bwd_op().call(kept(ctx, "json"), kept_hash(ctx), v[0], v[1], v[2], grads[0]);
+        return {at::Tensor(), at::Tensor(), dx, dy, dw, at::Tensor()};
+    }
+};
+
+struct TpBackward : torch::autograd::Function<TpBackward> {
+    static variable_list forward(AutogradContext* ctx, const at::Tensor& json, int64_t hash, const at::Tensor& x, const at::Tensor& y,
+                                 const at::Tensor& W, const at::Tensor& g) {
+        keep(ctx, json, hash);
+        ctx->save_for_backward({x, y, W, g});
+        at::AutoDispatchBelowADInplaceOrView below;
+        auto [dx, dy, dw] = tp_bwd_op().call(json, hash, x, y, W, g);
+        return {dx, dy, dw};
+    }
+    static variable_list backward(AutogradContext* ctx, const variable_list& grads) {   // undefined cotangents arrive as zeros
+        const variable_list v = ctx->get_saved_variables();
+        auto [dx, dy, dw, dg] = tp_dbl_op().call(kept(ctx, "json"), kept_hash(ctx), v[0], v[1], v[2], v[3], grads[0], grads[1], grads[2]);
+        return {at::Tensor(), at::Tensor(), dx, dy, dw, dg};
+    }
+};
+
+struct ConvForward : torch::autograd::Function<ConvForward> {
+    static at::Tensor forward(AutogradContext* ctx, const at::Tensor& json, int64_t hash, const at::Tensor& x, const at::Tensor& y,
+                              const at::Tensor& W, int64_t L3_dim, const at::Tensor& rows, const at::Tensor& cols,
+                              const at::Tensor& workspace, const at::Tensor& perm) {
+        keep(ctx, json, hash, rows, cols, workspace, perm);
+        ctx->save_for_backward({x, y, W});
+        at::AutoDispatchBelowADInplaceOrView below;
+        return conv_fwd_op().call(json, hash, x, y, W, L3_dim, rows, cols, workspace, perm);
+    }
+    static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
+        const variable_list v = ctx->get_saved_variables();
+        auto [dx, dy, dw] = conv_bwd_op().call(kept(ctx, "json"), kept_hash(ctx), v[0], v[1], v[2], grads[0], kept(ctx, "rows"),
+                                               kept(ctx, "cols"), kept(ctx, "workspace"), kept(ctx, "perm"));
+        return {at::Tensor(), at::Tensor(), dx, dy, dw, at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor()};
+    }
+};
+
+struct ConvBackward : torch::autograd::Function<ConvBackward> {
+    static variable_list forward(AutogradContext* ctx, const at::Tensor& json, int64_t hash, const at::Tensor& x, const at::Tensor& y,
+                                 const at::Tensor& W, const at::Tensor& g, const at::Tensor& rows, const at::Tensor& cols,
+                                 const at::Tensor& workspace, const at::Tensor& perm) {
+        keep(ctx, json, hash, rows, cols, workspace, perm);
+        ctx->save_for_backward({x, y, W, g});
+        at::AutoDispatchBelowADInplaceOrView below;
+        auto [dx, dy, dw] = conv_bwd_op().call(json, hash, x, y, W, g, rows, cols, workspace, perm);
+        return {dx, dy, dw};
+    }
+    static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
+        const variable_list v = ctx->get_saved_variables();
+        auto [dx, dy, dw, dg] = conv_dbl_op().call(kept(ctx, "json"), kept_hash(ctx), v[0], v[1], v[2], v[3], grads[0], grads[1],
+                                                   grads[2], kept(ctx, "rows"), kept(ctx, "cols"), kept(ctx, "workspace"),
+                                                   kept(ctx, "perm"));
+        return {at::Tensor(), at::Tensor(), dx, dy, dw, dg, at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor()};
+    }
+};
+
+at::Tensor autograd_tp_forward(const at::Tensor& json, int64_t hash, const at::Tensor& x, const at::Tensor& y, const at::Tensor& W,
+                               int64_t L3_dim) {
+    if (records(x, y, W)) return TpForward::apply(json, hash, x, y, W, L3_dim);
+    at::AutoDispatchBelowADInplaceOrView below;
+    return tp_fwd_op().call(json, hash, x, y, W, L3_dim);
+}
+
+Three autograd_tp_backward(const at::Tensor& json, int64_t hash, const at::Tensor& x, const at::Tensor& y, const at::Tensor& W,
+                           const at::Tensor& g) {
+    if (records(x, y, W, g)) {
+        const variable_list out = TpBackward::apply(json, hash, x, y, W, g);
+        return {out[0], out[1], out[2]};
+    }
+    at::AutoDispatchBelowADInplaceOrView below;
+    return tp_bwd_op().call(json, hash, x, y, W, g);
+}
+
+at::Tensor autograd_conv_forward(const at::Tensor& json, int64_t hash, const at::Tensor& x, const at::Tensor& y, const at::Tensor& W,
+                                 int64_t L3_dim, const at::Tensor& rows, const at::Tensor& cols, const at::Tensor& workspace,
+                                 const at::Tensor& perm) {
+    if (records(x, y, W)) return ConvForward::apply(json, hash, x, y, W, L3_dim, rows, cols, workspace, perm);
+    at::AutoDispatchBelowADInplaceOrView below;
+    return conv_fwd_op().call(json, hash, x, y, W, L3_dim, rows, cols, workspace, perm);
+}
+
+Three autograd_conv_backward(const at::Tensor& json, int64_t hash, const at::Tensor& x, const at::Tensor& y, const at::Tensor& W,
+                             const at::Tensor& g, const at::Tensor& rows, const at::Tensor& cols, const at::Tensor& workspace,
+                             const at::Tensor& perm) {
+    if (records(x, y, W, g)) {
+        const variable_list out = ConvBackward::apply(json, hash, x, y, W, g, rows, cols, workspace, perm);
+        return {out[0], out[1], out[2]};
+    }
+    at::AutoDispatchBelowADInplaceOrView below;
+    return conv_bwd_op().call(json, hash, x, y, W, g, rows, cols, workspace, perm);
+}
+
 }  // namespace
 
 TORCH_LIBRARY(libtorch_tp_jit, m) {
@@ -268,4 +440,11 @@ TORCH_LIBRARY_IMPL(libtorch_tp_jit, CUDA, m) {
     m.impl("jit_conv_forward", &jit_conv_forward);
     m.impl("jit_conv_backward", &jit_conv_backward);
     m.impl("jit_conv_double_backward", &jit_conv_double_backward);
+}
+
+TORCH_LIBRARY_IMPL(libtorch_tp_jit, Autograd, m) {
+    m.impl("jit_tp_forward", &autograd_tp_forward);
+    m.impl("jit_tp_backward", &autograd_tp_backward);
+    m.impl("jit_conv_forward", &autograd_conv_forward);
+    m.impl("jit_conv_backward", &autograd_conv_backward);
 }
