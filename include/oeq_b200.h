@@ -209,6 +209,22 @@ OEQB_API int oeqb_prepare_graph(int idx_dtype, int64_t n_nodes, int64_t n_edges,
 OEQB_API int oeqb_group_mm(int dtype, int ragged_inner, int64_t num_groups, int64_t num_features, int64_t M, int64_t K,
                            const int64_t* ragged_counts, const void* A, const void* B, void* C, void* stream);
 
+/* Symmetric contraction in one pass over the nodes (csrc/sym_contraction.cuh, csrc/kernels/sym_poly.cuh).
+ * meta (host): G, F, ell, n_out, n_sets, out_dim, terms, two words of a key that identifies `terms`, then per set
+ * {columns, rows} and per output component {column, stride} (more may follow).  terms (host): [terms, 4] = output component and
+ * ascending factors (ell = none) in the order of use; the kernels are specialised for them on first sight of the key.
+ * place (device): row of U -> its term.  U (device): the sets' rows, one after the other.  weights (host array of device
+ * pointers, one per set): [G, columns, F].  group (oeqb_symcon_group_ints values) and coef (oeqb_symcon_bytes, direction 0)
+ * are filled by the forward call and handed to the backward call; its workspace is oeqb_symcon_bytes, direction 1. */
+OEQB_API int64_t oeqb_symcon_group_ints(int64_t n_nodes, int64_t n_elements);
+OEQB_API int64_t oeqb_symcon_bytes(int dtype, const int32_t* meta, int n_meta, int direction, int64_t n_nodes);
+OEQB_API int oeqb_symcon_forward(int dtype, const int32_t* meta, int n_meta, const int32_t* terms, const int32_t* place, const void* U,
+                                 int64_t n_nodes, const int64_t* keys, const void* x, const void* const* weights, int32_t* group,
+                                 void* coef, void* out, void* stream);
+OEQB_API int oeqb_symcon_backward(int dtype, const int32_t* meta, int n_meta, const int32_t* terms, const int32_t* place, const void* U,
+                                  int64_t n_nodes, const int32_t* group, const void* coef, const void* x, const void* cot,
+                                  void* workspace, void* dx, void* const* dweights, void* stream);
+
 /* Kernels of this library report run-time failures (a bounded wait that ran out, an index out of range) through a
  * host-visible word per device that the next entry-point call inspects.  This call inspects it now: after the
  * caller has synchronised with the stream, it tells whether the work issued so far on the current device failed.

@@ -3,6 +3,10 @@ grouped product kernels.
 
 Counterpart of openequivariance/openequivariance/_torch/symmetric_contraction/symmetric_contraction.py:
 
+The work is done by ``oeq_b200::symmetric_contraction`` (csrc/sym_contraction.cuh): one pass over the nodes per direction,
+whose kernels are specialised for the monomials that the tensors ``U`` touch (``_Plan``).  Second and higher orders, tensors of
+order above three and installations without the C++ operators take the composed form below.
+
 * ``GroupMM`` (reference :7-108) -- the ragged grouped product as a torch custom op with autograd; the work is done by
   ``oeqb_group_mm`` (one kernel launch per call) instead of one cuBLAS strided-batched GEMM per chemical element.
 * ``Contraction`` / ``SymmetricContraction`` (reference :233-422) -- the contraction of node features with the
@@ -18,11 +22,14 @@ correlation order ``nu_max``:  ``out = sum_k U_numax[..., i, k] W_numax[e, k, f]
 from __future__ import annotations
 
 import ctypes
+import hashlib
+import struct
 from typing import Dict, List, Optional, Sequence
 
 import torch
 
 from .. import native
+from . import ops
 
 _DTYPE_ENUM = {torch.float32: 1, torch.float64: 2}
 
@@ -114,6 +121,181 @@ class GroupMM:
         return group_gemm(weights, vectors, bincounts, weights.shape[2], weights.shape[3], 0, self.num_elements)
 
 
+def _composed(Us, weights, x, bincount, sorted_indices, num_elements):
+    """The contraction of one output irrep from differentiable torch operations: ``Us`` and ``weights`` from the highest order
+    down to the first, nodes sorted by element."""
+    U = Us[0]
+    G, F = num_elements, x.shape[1]
+
+    def apply(U, W):     # [G, F] + U.shape[:-1]: the weights applied with one matrix product
+        flat = U.movedim(-1, 0).reshape(U.shape[-1], -1)
+        return (W.transpose(1, 2).reshape(-1, U.shape[-1]) @ flat).view([G, F] + list(U.shape[:-1]))
+
+    c = apply(U, weights[0])
+    out = group_gemm(c.reshape(G, F, -1, U.shape[-2]), x, bincount, c[0, 0].numel() // U.shape[-2], U.shape[-2], 0, G)
+    out = out.view([x.shape[0], F] + list(U.shape[:-2]))
+    for U, W in zip(Us[1:], weights[1:]):
+        c = apply(U, W)[sorted_indices] + out
+        s = c.shape
+        out = (c.reshape(s[0] * s[1], -1, s[-1]) * x.reshape(s[0] * s[1], 1, s[-1])).sum(dim=2).view(s[:-1])
+    return out.reshape(out.shape[0], -1)
+
+
+def _composed_unsorted(groups, weights, U, x, keys, num_elements):
+    """The composed form for nodes in any order: ``groups`` = number of orders of each output irrep, ``weights`` and ``U``
+    one tensor per (irrep, order)."""
+    bincount = torch.bincount(keys, minlength=num_elements).to("cpu")
+    permutation = torch.argsort(keys, stable=True)
+    inverse = torch.argsort(permutation)
+    xs, sorted_indices = x[permutation], keys[permutation]
+    outs, at = [], 0
+    for n in groups:
+        outs.append(_composed(U[at:at + n], weights[at:at + n], xs, bincount, sorted_indices, num_elements))
+        at += n
+    return torch.cat(outs, dim=-1)[inverse]
+
+
+_MONOMIALS = {}
+
+
+def _monomials(ell, device):
+    """Monomials of degree 0 ... 3 in ``ell`` features, numbered by degree: their exponent lists as ascending factors padded with
+    ``ell`` (``[count, 3]``), where each degree starts, and for every index tuple of degree 1 ... 3 its monomial's number."""
+    key = (ell, str(device))
+    if key not in _MONOMIALS:
+        r = torch.arange(ell, device=device)
+        factors, starts, number = [torch.full((1, 3), ell, device=device)], [0], [None]
+        for degree in (1, 2, 3):
+            tuples = torch.cartesian_prod(*([r] * degree)).reshape(-1, degree).sort(dim=1).values
+            code = (tuples * ell ** torch.arange(degree, device=device)).sum(1)
+            unique, inverse = torch.unique(code, return_inverse=True)
+            first = torch.empty_like(unique).scatter_(0, inverse, torch.arange(code.numel(), device=device))
+            starts.append(sum(f.shape[0] for f in factors))
+            factors.append(torch.nn.functional.pad(tuples[first], (0, 3 - degree), value=ell))
+            number.append(inverse + starts[-1])
+        _MONOMIALS[key] = (torch.cat(factors), starts, number)
+    return _MONOMIALS[key]
+
+
+class _Plan:
+    """What the operator needs to know about a set of tensors ``U``: the list of (output component, monomial) terms that they
+    touch and, for every term, the row of U (summed over the orders of the monomial's factors) that makes its coefficient."""
+
+    def __init__(self, U_groups, num_elements, num_features):
+        first = U_groups[0][0]
+        device, dtype, ell = first.device, first.dtype, first.shape[-2]
+        factors, starts, number = _monomials(ell, device)
+        self.groups = [len(g) for g in U_groups]
+        self.U = [U for g in U_groups for U in g]
+        self.versions = [_version(U) for U in self.U]
+        comp, mono, sets, rows, columns, out_col, out_stride, base = [], [], [], [], [], [], [], 0
+        for g in U_groups:
+            leading = g[0].dim() == len(g) + 2
+            lead = g[0].shape[0] if leading else 1
+            for w in range(lead):
+                out_col.append(base + w)
+                out_stride.append(lead)
+            for U in g:
+                degree, K = U.dim() - 1 - int(leading), U.shape[-1]
+                flat = U.detach().reshape(lead, ell ** degree, K).double()
+                count = factors.shape[0]
+                total = torch.zeros(lead, count, K, dtype=torch.float64, device=device).index_add_(1, number[degree], flat)
+                size = torch.zeros(lead, count, K, dtype=torch.float64, device=device).index_add_(1, number[degree], flat.abs())
+                # couplings that cancel between the orders of a monomial's factors leave rounding errors, not terms
+                total = torch.where(total.abs() <= 8 * torch.finfo(dtype).eps * size, 0.0, total)
+                w, m = (total != 0).any(dim=2).nonzero(as_tuple=True)
+                comp.append(w + len(out_col) - lead)
+                mono.append(m)
+                rows.append(total[w, m].to(dtype).reshape(-1))
+                sets.append(w.numel())
+                columns.append(K)
+            base += lead * num_features
+        self.out_dim, n_out = base, len(out_col)
+        w, m = torch.cat(comp), torch.cat(mono)
+        T = w.numel()
+        # (straight-line code: compiling it takes about a second per hundred terms, and more than a thousand are dense tensors)
+        self.fits = 0 < T <= 1024
+        if not self.fits:
+            return
+        # in the order of use: first order, then by the first two factors, by component, by the third factor (second order first)
+        i, j, k = factors[m].unbind(1)
+        third = (k + 1) % (ell + 1)
+        order = torch.argsort((((j != ell) * ell + i) * (ell + 1) + j) * n_out * (ell + 1) + w * (ell + 1) + third)
+        self.terms = torch.stack([w, i, j, k], dim=1)[order].to(device="cpu", dtype=torch.int32)
+        self.place = torch.empty(T, dtype=torch.int32, device=device)
+        self.place[order] = torch.arange(T, dtype=torch.int32, device=device)
+        self.U_rows = torch.cat(rows)
+        key = hashlib.blake2b(self.terms.numpy().tobytes() + bytes([ell, n_out]), digest_size=8).digest()
+        meta = [num_elements, num_features, ell, n_out, len(sets), self.out_dim, T, *struct.unpack("<ii", key)]
+        for pair in list(zip(columns, sets)) + list(zip(out_col, out_stride)):
+            meta += pair
+        # (the number of orders of every irrep comes last: only the composed second order reads it)
+        self.meta = torch.tensor(meta + self.groups + [len(self.groups)], dtype=torch.int32)
+
+    def holds_for(self, U_groups):
+        flat = [U for g in U_groups for U in g]
+        return len(flat) == len(self.U) and all(a is b and v == _version(b) for a, b, v in zip(self.U, flat, self.versions))
+
+
+def _version(t):
+    return 0 if t.is_inference() else t._version
+
+
+def _fused(owner, U_groups, weights, x, keys, num_elements):
+    """Runs the fused operator; None where it does not apply (the caller then composes)."""
+    first = U_groups[0][0]
+    if not ops.CPP_OPS or torch.compiler.is_compiling() or not x.is_cuda or x.dtype not in _DTYPE_ENUM or first.dtype != x.dtype:
+        return None
+    plan = owner.__dict__.get("_plan")
+    if plan is None or plan.F != x.shape[1] or not plan.holds_for(U_groups):
+        ell, n_out = first.shape[-2], sum(g[0].shape[0] if g[0].dim() == len(g) + 2 else 1 for g in U_groups)
+        fits = all(len(g) <= 3 and all(U.device == x.device and U.dtype == x.dtype and U.shape[-2] == ell for U in g) for g in U_groups)
+        if not fits or ell > 25 or n_out > 64 or sum(len(g) for g in U_groups) > 48 or num_elements > 256:
+            return None
+        with torch.no_grad(), torch.cuda.device(x.device):
+            plan = _Plan(U_groups, num_elements, x.shape[1])
+        plan.F = x.shape[1]
+        owner.__dict__["_plan"] = plan
+    if not plan.fits:
+        return None
+    return torch.ops.oeq_b200.symmetric_contraction(x, keys, weights, plan.U, plan.terms, plan.place, plan.U_rows, plan.meta, plan.out_dim)[0]
+
+
+if ops.CPP_OPS:
+    @torch.library.register_fake("oeq_b200::symmetric_contraction")
+    def _(x, keys, weights, U, terms, place, U_rows, meta, out_dim):
+        return x.new_empty(x.shape[0], out_dim), x.new_empty(x.shape[0], dtype=torch.int32), x.new_empty(1, dtype=torch.uint8)
+
+    @torch.library.register_fake("oeq_b200::symmetric_contraction_backward")
+    def _(grad, x, keys, group, coef, weights, U, terms, place, U_rows, meta):
+        return torch.empty_like(x), [torch.empty_like(w) for w in weights]
+
+    def _second_setup(ctx, inputs, output):
+        ctx.grad, ctx.x, ctx.keys, _, _, ctx.weights, ctx.U, _, _, _, ctx.meta = inputs
+
+    def _second_backward(ctx, t_dx, t_dw):
+        # the composed form's first-order gradients, differentiated again
+        keep = torch.is_grad_enabled()
+        groups = ctx.meta[-1 - int(ctx.meta[-1]):-1].tolist()
+        with torch.enable_grad():
+            leaves = [t.detach().requires_grad_(True) for t in (ctx.grad, ctx.x, *ctx.weights)]
+            g_, x_, w_ = leaves[0], leaves[1], leaves[2:]
+            out = _composed_unsorted(groups, w_, ctx.U, x_, ctx.keys, int(ctx.meta[0]))
+            first = torch.autograd.grad(out, [x_] + w_, g_, create_graph=True, allow_unused=True)
+            total = None
+            for f, t in zip(first, [t_dx] + list(t_dw if t_dw is not None else [None] * len(w_))):
+                if f is not None and t is not None:
+                    term = (f * t).sum()
+                    total = term if total is None else total + term
+            if total is None or not total.requires_grad:
+                grads = [None] * len(leaves)
+            else:
+                grads = torch.autograd.grad(total, leaves, create_graph=keep, allow_unused=True)
+        return grads[0], grads[1], None, None, None, list(grads[2:]), [None] * len(ctx.U), None, None, None, None
+
+    torch.library.register_autograd("oeq_b200::symmetric_contraction_backward", _second_backward, setup_context=_second_setup)
+
+
 class Contraction(torch.nn.Module):
     """Contraction for one output irrep.  ``U_matrices[nu]`` has shape ``[(2L+1,)] + [ell] * nu + [num_params_nu]``
     for ``nu = 1 ... correlation`` (the leading dimension only when the output irrep has ``L > 0``)."""
@@ -125,10 +307,11 @@ class Contraction(torch.nn.Module):
         self.correlation = max(U_matrices)
         assert sorted(U_matrices) == list(range(1, self.correlation + 1)), "U_matrices needs every order 1 ... correlation"
         self.num_features, self.num_elements = num_features, num_elements
+        self._names = [f"U_matrix_{nu}" for nu in range(self.correlation, 0, -1)]
         for nu, U in U_matrices.items():
             U = U.to(dtype)
             self.register_buffer(f"U_matrix_{nu}", U)
-            # [params, everything else]: the weights are applied with one matrix product per order
+            # [params, everything else]; part of the state dict, computed afresh where it is needed
             self.register_buffer(f"U_permuted_{nu}", U.movedim(-1, 0).reshape(U.shape[-1], -1).contiguous())
         self.groupMM = GroupMM(dtype, num_elements, num_features)
         if internal_weights:
@@ -147,22 +330,23 @@ class Contraction(torch.nn.Module):
     def U(self, nu):
         return getattr(self, f"U_matrix_{nu}")
 
+    def _tensors(self):
+        """``U`` from the highest order down, without ``nn.Module``'s attribute look-up."""
+        buffers = self._buffers
+        return [buffers[name] for name in self._names]
+
+    def _weights(self):
+        weights = self._modules.get("weights")     # (iterating a ParameterList costs several microseconds)
+        if weights is None:
+            return [self.weights_max, *self.weights]
+        return [self._parameters["weights_max"], *weights._parameters.values()]
+
     def forward(self, x: torch.Tensor, bincount: torch.Tensor, sorted_indices: torch.Tensor) -> torch.Tensor:
         """``x [N, F, ell]`` with the nodes sorted by element, ``bincount`` (CPU) nodes per element, ``sorted_indices [N]``
         the element of each (sorted) node."""
-        U = self.U(self.correlation)
-        n_par, ell = U.shape[-1], U.shape[-2]
-        UW = self.weights_max.transpose(1, 2).reshape(-1, n_par) @ getattr(self, f"U_permuted_{self.correlation}")
-        out = self.groupMM.forward(UW.view(self.num_elements, self.num_features, -1, ell), x, bincount)
-        out = out.view([x.shape[0], self.num_features] + list(U.shape[:-2]))
-        for i, W in enumerate(self.weights):
-            nu = self.correlation - i - 1
-            U = self.U(nu)
-            c = W.transpose(1, 2).reshape(-1, W.shape[1]) @ getattr(self, f"U_permuted_{nu}")
-            c = c.view([W.shape[0], W.shape[2]] + list(U.shape[:-1]))[sorted_indices] + out
-            s = c.shape
-            out = (c.reshape(s[0] * s[1], -1, s[-1]) * x.reshape(s[0] * s[1], 1, s[-1])).sum(dim=2).view(s[:-1])
-        return out.reshape(out.shape[0], -1)
+        Us, weights = self._tensors(), self._weights()
+        out = _fused(self, [Us], weights, x, sorted_indices, self.num_elements)
+        return _composed(Us, weights, x, bincount, sorted_indices, self.num_elements) if out is None else out
 
 
 class SymmetricContraction(torch.nn.Module):
@@ -179,9 +363,11 @@ class SymmetricContraction(torch.nn.Module):
 
     def forward(self, x: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
         indices = torch.argmax(y, dim=1)
-        bincount = torch.bincount(indices, minlength=self.num_elements).to("cpu")
-        permutation = torch.argsort(indices, stable=True)
-        inverse = torch.argsort(permutation)
-        xs, sorted_indices = x[permutation], indices[permutation]
-        outs = [c(xs, bincount, sorted_indices) for c in self.contractions]
-        return torch.cat(outs, dim=-1)[inverse]
+        contractions = list(self._modules["contractions"]._modules.values())
+        U_groups = [c._tensors() for c in contractions]
+        weights = [w for c in contractions for w in c._weights()]
+        if y.shape[1] <= self.num_elements:
+            out = _fused(self, U_groups, weights, x, indices, self.num_elements)
+            if out is not None:
+                return out
+        return _composed_unsorted([len(g) for g in U_groups], weights, [U for g in U_groups for U in g], x, indices, self.num_elements)

@@ -17,12 +17,12 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(CSRC, "liboeq_b200.so")
 STAMP = LIB + ".srchash"
 EMBED = {"K_COMMON": "common.cuh", "K_GENERIC": "generic_tp.cuh", "K_FAST_UVU": "fast_uvu.cuh",
-         "K_UVW_TC": "uvw_tc.cuh"}
+         "K_UVW_TC": "uvw_tc.cuh", "K_SYM_POLY": "sym_poly.cuh"}
 
 
 def _sources():
     out = [os.path.join(CSRC, "oeq_b200.cu"), os.path.join(CSRC, "graph_prep.cuh"), os.path.join(CSRC, "group_mm.cuh"),
-           os.path.join(CSRC, "partition_plan.cuh"),
+           os.path.join(CSRC, "sym_contraction.cuh"), os.path.join(CSRC, "partition_plan.cuh"),
            os.path.join(HERE, "..", "include", "oeq_b200.h")]
     out += [os.path.join(CSRC, "kernels", f) for f in EMBED.values()]
     return [p for p in out if os.path.exists(p)]

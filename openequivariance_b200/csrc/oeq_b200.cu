@@ -32,10 +32,11 @@
 #include <vector>
 
 #include "../../include/oeq_b200.h"
-#include "kernels_embed.inc"  // generated at build time: K_COMMON, K_GENERIC, K_FAST_UVU as raw strings
+#include "kernels_embed.inc"  // generated at build time: K_COMMON, K_GENERIC, ... as raw strings
 #include "graph_prep.cuh"         // problem-independent kernels: grouping / sorting of edge lists
 #include "partition_plan.cuh"     // ... and the plans of the partitioned / streamed drivers
 #include "group_mm.cuh"       // problem-independent kernels: ragged grouped products of the symmetric contraction
+#include "sym_contraction.cuh"    // ... and the whole contraction in one pass
 
 namespace {
 
@@ -957,26 +958,31 @@ int get_entry(const void* desc, size_t len, int64_t key, Entry** out) {
     return OEQB_OK;
 }
 
-// Caller holds g_mutex.
-int get_program(Entry* e, int fam, Program** out, bool allow_streams = true) {
-    std::unique_ptr<Program>& slot = allow_streams ? e->prog[fam] : e->prog_single[fam];
-    if (slot) { *out = slot.get(); return OEQB_OK; }
-    auto p = std::make_unique<Program>();
-    const std::string src = family_source(e->d, e->header, fam, allow_streams);
+// Compiles (or takes from the cubin cache) and loads one program.
+int load_program(const std::string& src, const char* label, Program* p) {
     std::string cache_path;
-    int rc = compile_cubin(src, family_name(fam), p->cubin, &cache_path);
+    int rc = compile_cubin(src, label, p->cubin, &cache_path);
     if (rc) return rc;
     cudaError_t ce = cudaLibraryLoadData(&p->lib, p->cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0);
     if (ce != cudaSuccess && !cache_path.empty()) {
         // a truncated or foreign file in the cache: drop it and compile afresh, once
         cudaGetLastError();
         remove(cache_path.c_str());
-        if (g_log) fprintf(stderr, "[oeq_b200] %s: cached cubin %s did not load (%s); recompiling\n", family_name(fam),
-                           cache_path.c_str(), cudaGetErrorString(ce));
-        if ((rc = compile_cubin(src, family_name(fam), p->cubin, nullptr))) return rc;
+        if (g_log) fprintf(stderr, "[oeq_b200] %s: cached cubin %s did not load (%s); recompiling\n", label, cache_path.c_str(),
+                           cudaGetErrorString(ce));
+        if ((rc = compile_cubin(src, label, p->cubin, nullptr))) return rc;
         ce = cudaLibraryLoadData(&p->lib, p->cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0);
     }
-    if (ce != cudaSuccess) return fail(OEQB_ECOMPILE, "cudaLibraryLoadData(%s): %s", family_name(fam), cudaGetErrorString(ce));
+    if (ce != cudaSuccess) return fail(OEQB_ECOMPILE, "cudaLibraryLoadData(%s): %s", label, cudaGetErrorString(ce));
+    return OEQB_OK;
+}
+
+// Caller holds g_mutex.
+int get_program(Entry* e, int fam, Program** out, bool allow_streams = true) {
+    std::unique_ptr<Program>& slot = allow_streams ? e->prog[fam] : e->prog_single[fam];
+    if (slot) { *out = slot.get(); return OEQB_OK; }
+    auto p = std::make_unique<Program>();
+    if (int rc = load_program(family_source(e->d, e->header, fam, allow_streams), family_name(fam), p.get())) return rc;
     *out = p.get();
     slot = std::move(p);
     return OEQB_OK;
@@ -2151,6 +2157,235 @@ int oeqb_group_mm(int dtype, int ragged_inner, int64_t num_groups, int64_t num_f
     cudaError_t ce = dtype == 2 ? gmm::dispatch<double>(ragged_inner, offs, n_nodes, num_features, (int)M, (int)K, A, B, C, st)
                                 : gmm::dispatch<float>(ragged_inner, offs, n_nodes, num_features, (int)M, (int)K, A, B, C, st);
     if (ce != cudaSuccess) return fail(OEQB_ECUDA, "oeqb_group_mm: kernel launch failed: %s", cudaGetErrorString(ce));
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    return OEQB_OK;
+}
+
+extern "C++" {
+namespace {
+struct SymTerm { int w, i, j, k; };
+struct SymPlan {
+    int G, F, ell, n_out, out_dim;
+    uint64_t key;
+    symc::Sets sets;
+    int out_col[symc::MAX_OUT], out_stride[symc::MAX_OUT];
+    // chunks of the weight gradient's terms: at most 56 (28 doubles) running sums per thread
+    int chunks(int dtype) const { return (sets.terms + (dtype == 2 ? 28 : 56) - 1) / (dtype == 2 ? 28 : 56); }
+    int chunk(int dtype) const { return (sets.terms + chunks(dtype) - 1) / chunks(dtype); }
+    // slices of an element's nodes in the weight gradient: sixteen warps per SM, eight nodes or more each
+    int slices(int dtype, long long n) const {
+        const long long warps = (long long)G * ((F + 31) / 32) * chunks(dtype);
+        const long long want = (16 * 148 + warps - 1) / warps, most = n / (8LL * G) + 1;
+        return (int)std::min<long long>(std::min(want, most), 64);
+    }
+    size_t coef_bytes(size_t elt) const { return round_up((size_t)G * ((sets.terms + 3) / 4) * F * 4 * elt); }
+    size_t part_bytes(int dtype, long long n) const { return round_up((size_t)slices(dtype, n) * G * sets.terms * F * (dtype == 2 ? 8 : 4)); }
+};
+
+int symcon_plan(const int32_t* meta, int n_meta, SymPlan* p) {
+    if (!meta || n_meta < 9) return fail(OEQB_EINVAL, "oeqb_symcon: bad meta");
+    memset(p, 0, sizeof *p);
+    p->G = meta[0]; p->F = meta[1]; p->ell = meta[2]; p->n_out = meta[3]; p->sets.n_sets = meta[4];
+    p->out_dim = meta[5]; p->sets.terms = meta[6]; p->sets.F = p->F;
+    p->key = (uint64_t)(uint32_t)meta[7] | (uint64_t)(uint32_t)meta[8] << 32;
+    if (p->G < 1 || p->G > gmm::MAX_GROUPS || p->F < 1 || p->F > 65535 || p->ell < 1 || p->ell > symc::MAX_ELL || p->n_out < 1 || p->n_out > symc::MAX_OUT ||
+        p->sets.n_sets < 1 || p->sets.n_sets > symc::MAX_SETS || p->sets.terms < 1 || p->sets.terms > symc::MAX_TERMS ||
+        n_meta < 9 + 2 * p->sets.n_sets + 2 * p->n_out)
+        return fail(OEQB_EINVAL, "oeqb_symcon: bad meta");
+    const int32_t* m = meta + 9;
+    int rows = 0, u = 0;
+    for (int s = 0; s < p->sets.n_sets; ++s) {
+        p->sets.k[s] = *m++;
+        p->sets.t0[s] = rows;
+        rows += *m++;
+        p->sets.t1[s] = rows;
+        p->sets.u[s] = u;
+        if (p->sets.k[s] < 0 || rows < p->sets.t0[s]) return fail(OEQB_EINVAL, "oeqb_symcon: bad meta");
+        u += p->sets.k[s] * (rows - p->sets.t0[s]);
+    }
+    if (rows != p->sets.terms) return fail(OEQB_EINVAL, "oeqb_symcon: bad meta");
+    for (int w = 0; w < p->n_out; ++w) { p->out_col[w] = *m++; p->out_stride[w] = *m++; }
+    return OEQB_OK;
+}
+
+// The straight-line code of kernels/sym_poly.cuh for one list of terms (sorted: first order, then by the first two factors, by
+// component, by the third factor).
+std::string emit_sym(const SymPlan& p, int dtype, const SymTerm* t) {
+    std::ostringstream s;
+    const int n = p.sets.terms, ell = p.ell, chunk = p.chunk(dtype), chunks = p.chunks(dtype);
+    s << "typedef " << (dtype == 2 ? "double" : "float") << " T;\n#define OEQ_DEV __device__ __forceinline__\n"
+      << "constexpr int ELL = " << ell << ", NOUT = " << p.n_out << ", TERMS = " << n << ", QUADS = " << (n + 3) / 4 << ", CHUNK = " << chunk
+      << ", CHUNKS = " << chunks << ";\nstruct __align__(16) T4 { T x, y, z, w; };\n";
+    const char comp[4] = {'x', 'y', 'z', 'w'};
+    auto coef = [&](int q) { return "c" + std::to_string(q / 4) + "." + comp[q % 4]; };
+    auto load = [&](int q) { if (q % 4 == 0) s << "  const T4 c" << q / 4 << " = c[" << q / 4 << "];\n"; };
+    for (int grad = 0; grad < 2; ++grad) {
+        if (!grad) s << "OEQ_DEV void sym_eval(const T (&x)[ELL], const T4* c, T (&P)[NOUT]) {\n  for (int w = 0; w < NOUT; ++w) P[w] = T(0);\n";
+        else s << "OEQ_DEV void sym_grad(const T (&x)[ELL], const T (&cot)[NOUT], const T4* c, T (&dx)[ELL]) {\n";
+        for (int q = 0; q < n;) {
+            if (t[q].j == ell) {
+                load(q);
+                if (!grad) s << "  P[" << t[q].w << "] = fma(" << coef(q) << ", x[" << t[q].i << "], P[" << t[q].w << "]);\n";
+                else s << "  dx[" << t[q].i << "] = fma(cot[" << t[q].w << "], " << coef(q) << ", dx[" << t[q].i << "]);\n";
+                ++q;
+                continue;
+            }
+            const int i = t[q].i, j = t[q].j, pair = q;
+            s << "  const T xx" << pair << " = x[" << i << "] * x[" << j << "];\n";
+            if (grad) s << "  T s" << pair << " = T(0);\n";
+            while (q < n && t[q].i == i && t[q].j == j) {
+                const int w = t[q].w, at = q;
+                s << "  T r" << at << " = T(0);\n";
+                if (grad) s << "  const T g" << at << " = cot[" << w << "] * xx" << pair << ";\n";
+                for (; q < n && t[q].i == i && t[q].j == j && t[q].w == w; ++q) {
+                    load(q);
+                    if (t[q].k == ell) { s << "  r" << at << " += " << coef(q) << ";\n"; continue; }
+                    s << "  r" << at << " = fma(" << coef(q) << ", x[" << t[q].k << "], r" << at << ");";
+                    if (grad) s << " dx[" << t[q].k << "] = fma(" << coef(q) << ", g" << at << ", dx[" << t[q].k << "]);";
+                    s << "\n";
+                }
+                if (!grad) s << "  P[" << w << "] = fma(xx" << pair << ", r" << at << ", P[" << w << "]);\n";
+                else s << "  s" << pair << " = fma(cot[" << w << "], r" << at << ", s" << pair << ");\n";
+            }
+            if (grad)
+                s << "  dx[" << i << "] = fma(s" << pair << ", x[" << j << "], dx[" << i << "]); dx[" << j << "] = fma(s" << pair << ", x[" << i
+                  << "], dx[" << j << "]);\n";
+        }
+        s << "}\n";
+    }
+    s << "template <int N> struct SymChunk;\n";
+    for (int c = 0; c < chunks; ++c) {
+        s << "template <> struct SymChunk<" << c << "> { static OEQ_DEV void add(const T (&x)[ELL], const T (&cot)[NOUT], T (&m)[CHUNK]) {\n";
+        for (int q = c * chunk; q < n && q < (c + 1) * chunk; ++q) {
+            const int at = q - c * chunk;
+            const bool fresh = at == 0 || t[q].i != t[q - 1].i || t[q].j != t[q - 1].j || t[q].w != t[q - 1].w;
+            if (t[q].j == ell) { s << "  m[" << at << "] = fma(cot[" << t[q].w << "], x[" << t[q].i << "], m[" << at << "]);\n"; continue; }
+            if (at == 0 || t[q].i != t[q - 1].i || t[q].j != t[q - 1].j)
+                s << "  const T xx" << t[q].i << "_" << t[q].j << " = x[" << t[q].i << "] * x[" << t[q].j << "];\n";
+            if (fresh) s << "  const T g" << t[q].i << "_" << t[q].j << "_" << t[q].w << " = cot[" << t[q].w << "] * xx" << t[q].i << "_" << t[q].j << ";\n";
+            s << "  m[" << at << "] ";
+            if (t[q].k == ell) s << "+= g" << t[q].i << "_" << t[q].j << "_" << t[q].w << ";\n";
+            else s << "= fma(g" << t[q].i << "_" << t[q].j << "_" << t[q].w << ", x[" << t[q].k << "], m[" << at << "]);\n";
+        }
+        s << "} };\n";
+    }
+    return s.str();
+}
+
+std::map<std::pair<uint64_t, int>, std::unique_ptr<Program>> g_sym_programs;   // by (key of the terms, dtype)
+
+// Caller holds g_mutex.
+int symcon_program(const SymPlan& p, int dtype, const int32_t* terms, Program** out) {
+    std::unique_ptr<Program>& slot = g_sym_programs[{p.key, dtype}];
+    if (!slot) {
+        if (int rc = check_ptrs({terms}, "oeqb_symcon")) return rc;
+        const SymTerm* t = (const SymTerm*)terms;
+        for (int q = 0; q < p.sets.terms; ++q)
+            if (t[q].w < 0 || t[q].w >= p.n_out || t[q].i < 0 || t[q].i >= p.ell || t[q].j < t[q].i || t[q].j > p.ell || t[q].k < t[q].j || t[q].k > p.ell)
+                return fail(OEQB_EINVAL, "oeqb_symcon: bad term");
+        auto fresh = std::make_unique<Program>();
+        if (int rc = load_program(emit_sym(p, dtype, t) + K_COMMON + K_SYM_POLY, "symmetric_contraction", fresh.get())) return rc;
+        slot = std::move(fresh);
+    }
+    *out = slot.get();
+    return OEQB_OK;
+}
+
+struct SymParams {
+    const int* group; long long n;
+    int G, F, out_dim, slices;
+    const void* x; const void* cot; const void* coef;
+    void* out; void* dx; void* part;
+    int out_cols[2 * symc::MAX_OUT];   // n_out columns, then n_out strides (the kernel's arrays have exactly n_out entries)
+};
+SymParams symcon_params(const SymPlan& p, const int32_t* group, long long n) {
+    SymParams a{};
+    a.group = group; a.n = n; a.G = p.G; a.F = p.F; a.out_dim = p.out_dim;
+    for (int w = 0; w < p.n_out; ++w) { a.out_cols[w] = p.out_col[w]; a.out_cols[p.n_out + w] = p.out_stride[w]; }
+    return a;
+}
+int symcon_launch(Program* prog, const char* name, dim3 grid, unsigned block, SymParams& a, cudaStream_t st) {
+    cudaKernel_t k;
+    if (int rc = get_kernel(prog, name, 0, &k)) return rc;
+    void* args[] = {&a};
+    cudaError_t ce = cudaLaunchKernel((const void*)k, grid, dim3(block), args, 0, st);
+    if (ce != cudaSuccess) return fail(OEQB_ECUDA, "%s: %s", name, cudaGetErrorString(ce));
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    return OEQB_OK;
+}
+// as SYM_WPB in kernels/sym_poly.cuh
+unsigned symcon_wpb(const SymPlan& p, size_t elt) { return 8 * (size_t)((p.sets.terms + 3) / 4) * 4 * elt <= 48000 ? 8 : 1; }
+}  // namespace
+}
+
+int64_t oeqb_symcon_group_ints(int64_t n_nodes, int64_t n_elements) {
+    if (n_nodes < 0 || n_elements < 1 || n_elements > gmm::MAX_GROUPS) return -(int64_t)fail(OEQB_EINVAL, "oeqb_symcon_group_ints: bad size");
+    return symc::group_ints(n_nodes, (int)n_elements);
+}
+
+int64_t oeqb_symcon_bytes(int dtype, const int32_t* meta, int n_meta, int direction, int64_t n_nodes) {
+    if ((dtype != 1 && dtype != 2) || n_nodes < 0) return -(int64_t)fail(OEQB_EINVAL, "oeqb_symcon_bytes: bad argument");
+    SymPlan p;
+    if (int rc = symcon_plan(meta, n_meta, &p)) return -(int64_t)rc;
+    return (int64_t)(direction == 0 ? p.coef_bytes(dtype == 2 ? 8 : 4) : p.part_bytes(dtype, n_nodes));
+}
+
+int oeqb_symcon_forward(int dtype, const int32_t* meta, int n_meta, const int32_t* terms, const int32_t* place, const void* U, int64_t n_nodes,
+                        const int64_t* keys, const void* x, const void* const* weights, int32_t* group, void* coef, void* out, void* stream) {
+    if (dtype != 1 && dtype != 2) return fail(OEQB_EINVAL, "oeqb_symcon_forward: dtype must be 1 (float32) or 2 (float64)");
+    SymPlan p;
+    if (int rc = symcon_plan(meta, n_meta, &p)) return rc;
+    if (n_nodes == 0) return OEQB_OK;
+    if (n_nodes < 0 || n_nodes > (1LL << 30)) return fail(OEQB_EINVAL, "oeqb_symcon_forward: bad size");
+    if (int rc = check_ptrs({place, U, keys, x, weights, group, coef, out}, "oeqb_symcon_forward")) return rc;
+    if (!aligned16({x, coef})) return fail(OEQB_EINVAL, "oeqb_symcon_forward: x is not 16-byte aligned");
+    std::lock_guard<std::mutex> lock(g_mutex);
+    Program* prog;
+    if (int rc = symcon_program(p, dtype, terms, &prog)) return rc;
+    p.sets.place = place;
+    symc::Pointers w{};
+    for (int s = 0; s < p.sets.n_sets; ++s) w.p[s] = (void*)weights[s];
+    cudaStream_t st = (cudaStream_t)stream;
+    CUDA_TRY(symc::run_group((const long long*)keys, n_nodes, p.G, group, st));
+    CUDA_TRY(dtype == 2 ? symc::run_coefficients<double>(p.sets, p.G, (const double*)U, w, (double*)coef, st)
+                        : symc::run_coefficients<float>(p.sets, p.G, (const float*)U, w, (float*)coef, st));
+    g_launches.fetch_add(2, std::memory_order_relaxed);
+    SymParams a = symcon_params(p, group, n_nodes);
+    a.x = x; a.coef = coef; a.out = out;
+    const unsigned wpb = symcon_wpb(p, dtype == 2 ? 8 : 4);
+    return symcon_launch(prog, "oeq_sym_forward", dim3((unsigned)symc::max_tiles(n_nodes, p.G), (p.F + wpb - 1) / wpb), 32 * wpb, a, st);
+}
+
+int oeqb_symcon_backward(int dtype, const int32_t* meta, int n_meta, const int32_t* terms, const int32_t* place, const void* U, int64_t n_nodes,
+                         const int32_t* group, const void* coef, const void* x, const void* cot, void* workspace, void* dx,
+                         void* const* dweights, void* stream) {
+    if (dtype != 1 && dtype != 2) return fail(OEQB_EINVAL, "oeqb_symcon_backward: dtype must be 1 (float32) or 2 (float64)");
+    SymPlan p;
+    if (int rc = symcon_plan(meta, n_meta, &p)) return rc;
+    if (n_nodes < 0 || n_nodes > (1LL << 30)) return fail(OEQB_EINVAL, "oeqb_symcon_backward: bad size");
+    const size_t elt = dtype == 2 ? 8 : 4;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (int rc = check_ptrs({dweights}, "oeqb_symcon_backward")) return rc;
+    if (n_nodes == 0) {
+        for (int s = 0; s < p.sets.n_sets; ++s) if (p.sets.k[s] > 0) CUDA_TRY(cudaMemsetAsync(dweights[s], 0, (size_t)p.G * p.sets.k[s] * p.F * elt, st));
+        return OEQB_OK;
+    }
+    if (int rc = check_ptrs({place, U, group, coef, x, cot, workspace, dx}, "oeqb_symcon_backward")) return rc;
+    if (!aligned16({x, coef, dx})) return fail(OEQB_EINVAL, "oeqb_symcon_backward: an operand is not 16-byte aligned");
+    std::lock_guard<std::mutex> lock(g_mutex);
+    Program* prog;
+    if (int rc = symcon_program(p, dtype, terms, &prog)) return rc;
+    p.sets.place = place;
+    symc::Pointers dw{};
+    for (int s = 0; s < p.sets.n_sets; ++s) dw.p[s] = dweights[s];
+    SymParams a = symcon_params(p, group, n_nodes);
+    a.x = x; a.cot = cot; a.coef = coef; a.dx = dx; a.part = workspace;
+    a.slices = p.slices(dtype, n_nodes);
+    const unsigned wpb = symcon_wpb(p, elt);
+    if (int rc = symcon_launch(prog, "oeq_sym_backward_x", dim3((unsigned)symc::max_tiles(n_nodes, p.G), (p.F + wpb - 1) / wpb), 32 * wpb, a, st)) return rc;
+    if (int rc = symcon_launch(prog, "oeq_sym_backward_c", dim3((unsigned)(((long long)p.G * ((p.F + 31) / 32) * a.slices + 3) / 4), (unsigned)p.chunks(dtype)), 128, a, st)) return rc;
+    CUDA_TRY(dtype == 2 ? symc::run_gradient_w<double>(p.sets, p.G, (const double*)U, (const double*)workspace, a.slices, dw, st)
+                        : symc::run_gradient_w<float>(p.sets, p.G, (const float*)U, (const float*)workspace, a.slices, dw, st));
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return OEQB_OK;
 }

@@ -422,7 +422,143 @@ Three autograd_conv_backward(const at::Tensor& json, int64_t hash, const at::Ten
     return conv_bwd_op().call(json, hash, x, y, W, g, rows, cols, workspace, perm);
 }
 
+// ---- symmetric contraction ---------------------------------------------------------------------------------------
+// `terms`, `meta` (CPU), `place` and `U_rows` describe the contraction's tensors U (made by _torch/symmetric_contraction.py);
+// `keys` holds the element of each node; `weights` one tensor [elements, columns, channels] per (irrep, order).  The dense
+// tensors `U` are only used by the second order, which Python composes.  Besides the result the forward returns what the
+// backward takes again: the nodes by element and the polynomials' coefficients.
+int symcon_dtype(const at::Tensor& x) {
+    if (x.scalar_type() == at::kFloat) return 1;
+    if (x.scalar_type() == at::kDouble) return 2;
+    refuse("symmetric_contraction: x must be float32 or float64");
+}
+at::Tensor aligned(const at::Tensor& t) {   // rows are read 16 bytes at a time
+    at::Tensor c = t.contiguous();
+    return ((uintptr_t)c.data_ptr() & 15u) ? c.clone() : c;
+}
+
+Three symcon_forward(const at::Tensor& x_in, const at::Tensor& keys_in, at::TensorList weights, at::TensorList U, const at::Tensor& terms,
+                     const at::Tensor& place, const at::Tensor& U_rows, const at::Tensor& meta_in, int64_t out_dim) {
+    (void)U;
+    const int32_t* meta = meta_in.data_ptr<int32_t>();
+    const int n_meta = (int)meta_in.numel(), dt = symcon_dtype(x_in);
+    const int64_t N = first_dim(x_in, "x");
+    check(x_in, {N, meta[1], meta[2]}, x_in.scalar_type(), "x");
+    check(keys_in, {N}, at::kLong, "keys");
+    check(U_rows, {-1}, x_in.scalar_type(), "U");
+    if (out_dim != meta[5] || (int64_t)weights.size() != meta[4]) refuse("symmetric_contraction: the plan does not fit the operands");
+    c10::cuda::CUDAGuard guard(x_in.device());
+    at::Tensor x = aligned(x_in), keys = keys_in.contiguous();
+    std::vector<at::Tensor> held;
+    std::vector<const void*> w;
+    for (size_t s = 0; s < weights.size(); ++s) {
+        check(weights[s], {meta[0], meta[9 + 2 * s], meta[1]}, x.scalar_type(), "weights");
+        held.push_back(weights[s].contiguous());
+        w.push_back(held.back().data_ptr());
+    }
+    const int64_t bytes = oeqb_symcon_bytes(dt, meta, n_meta, 0, N);
+    if (bytes < 0) done((int)-bytes, "symmetric_contraction");
+    at::Tensor group = at::empty({oeqb_symcon_group_ints(N, meta[0])}, x.options().dtype(at::kInt));
+    at::Tensor out = at::empty({N, out_dim}, x.options()), coef = at::empty({bytes}, x.options().dtype(at::kByte));
+    done(oeqb_symcon_forward(dt, meta, n_meta, terms.data_ptr<int32_t>(), place.data_ptr<int32_t>(), U_rows.data_ptr(), N,
+                             keys.data_ptr<int64_t>(), ptr(x), w.data(), group.data_ptr<int32_t>(), coef.data_ptr(), mptr(out),
+                             current_stream(x)),
+         "symmetric_contraction");
+    return {out, group, coef};
+}
+
+std::tuple<at::Tensor, std::vector<at::Tensor>> symcon_backward(const at::Tensor& cot_in, const at::Tensor& x_in, const at::Tensor& keys,
+                                                               const at::Tensor& group, const at::Tensor& coef, at::TensorList weights,
+                                                               at::TensorList U, const at::Tensor& terms, const at::Tensor& place,
+                                                               const at::Tensor& U_rows, const at::Tensor& meta_in) {
+    (void)U; (void)keys;
+    const int32_t* meta = meta_in.data_ptr<int32_t>();
+    const int n_meta = (int)meta_in.numel(), dt = symcon_dtype(x_in);
+    const int64_t N = x_in.size(0);
+    check(cot_in, {N, meta[5]}, x_in.scalar_type(), "grad");
+    c10::cuda::CUDAGuard guard(x_in.device());
+    at::Tensor x = aligned(x_in), cot = cot_in.contiguous(), dx = at::empty_like(x);
+    // one allocation for the weight gradients and the scratch
+    const int64_t elt = (int64_t)x.element_size(), part = oeqb_symcon_bytes(dt, meta, n_meta, 1, N);
+    if (part < 0) done((int)-part, "symmetric_contraction_backward");
+    std::vector<at::Tensor> dw;
+    std::vector<void*> dwp;
+    for (const at::Tensor& t : weights) {
+        dw.push_back(at::empty(t.sizes(), x.options()));
+        dwp.push_back(dw.back().data_ptr());
+    }
+    at::Tensor ws = at::empty({part / elt + 1}, x.options());
+    done(oeqb_symcon_backward(dt, meta, n_meta, terms.data_ptr<int32_t>(), place.data_ptr<int32_t>(), U_rows.data_ptr(), N,
+                              group.data_ptr<int32_t>(), coef.data_ptr(), ptr(x), ptr(cot), ws.data_ptr(), mptr(dx), dwp.data(),
+                              current_stream(x)),
+         "symmetric_contraction_backward");
+    return {dx, dw};
+}
+
+typedef Three SymFwdSig(const at::Tensor&, const at::Tensor&, at::TensorList, at::TensorList, const at::Tensor&, const at::Tensor&,
+                        const at::Tensor&, const at::Tensor&, int64_t);
+typedef std::tuple<at::Tensor, std::vector<at::Tensor>> SymBwdSig(const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
+                                                                  const at::Tensor&, at::TensorList, at::TensorList, const at::Tensor&,
+                                                                  const at::Tensor&, const at::Tensor&, const at::Tensor&);
+const c10::TypedOperatorHandle<SymFwdSig>& sym_fwd_op() {
+    static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("oeq_b200::symmetric_contraction", "").typed<SymFwdSig>();
+    return op;
+}
+const c10::TypedOperatorHandle<SymBwdSig>& sym_bwd_op() {
+    static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("oeq_b200::symmetric_contraction_backward", "").typed<SymBwdSig>();
+    return op;
+}
+
+struct SymForward : torch::autograd::Function<SymForward> {
+    static variable_list forward(AutogradContext* ctx, const at::Tensor& x, const at::Tensor& keys, at::TensorList weights, at::TensorList U,
+                                 const at::Tensor& terms, const at::Tensor& place, const at::Tensor& U_rows, const at::Tensor& meta,
+                                 int64_t out_dim) {
+        at::AutoDispatchBelowADInplaceOrView below;
+        auto [out, group, coef] = sym_fwd_op().call(x, keys, weights, U, terms, place, U_rows, meta, out_dim);
+        ctx->mark_non_differentiable({group, coef});
+        ctx->set_materialize_grads(false);
+        variable_list saved{x};
+        saved.insert(saved.end(), weights.begin(), weights.end());
+        ctx->save_for_backward(saved);
+        ctx->saved_data["fixed"] = std::vector<at::Tensor>{keys, group, coef, terms, place, U_rows, meta};
+        ctx->saved_data["U"] = U.vec();
+        return {out, group, coef};
+    }
+    static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
+        const variable_list v = ctx->get_saved_variables();
+        const std::vector<at::Tensor> weights(v.begin() + 1, v.end()), U = ctx->saved_data["U"].toTensorVector();
+        const std::vector<at::Tensor> fixed = ctx->saved_data["fixed"].toTensorVector();
+        auto [dx, dw] = sym_bwd_op().call(grads[0], v[0], fixed[0], fixed[1], fixed[2], weights, U, fixed[3], fixed[4], fixed[5], fixed[6]);
+        variable_list out{dx, at::Tensor()};
+        out.insert(out.end(), dw.begin(), dw.end());
+        out.resize(out.size() + U.size() + 5);   // U, terms, place, U_rows, meta, out_dim
+        return out;
+    }
+};
+
+Three autograd_symcon(const at::Tensor& x, const at::Tensor& keys, at::TensorList weights, at::TensorList U, const at::Tensor& terms,
+                      const at::Tensor& place, const at::Tensor& U_rows, const at::Tensor& meta, int64_t out_dim) {
+    bool any = records(x);
+    for (const at::Tensor& w : weights) any = any || records(w);
+    if (any) {
+        const variable_list out = SymForward::apply(x, keys, weights, U, terms, place, U_rows, meta, out_dim);
+        return {out[0], out[1], out[2]};
+    }
+    at::AutoDispatchBelowADInplaceOrView below;
+    return sym_fwd_op().call(x, keys, weights, U, terms, place, U_rows, meta, out_dim);
+}
+
 }  // namespace
+
+TORCH_LIBRARY_FRAGMENT(oeq_b200, m) {
+    m.def("symmetric_contraction(Tensor x, Tensor keys, Tensor[] weights, Tensor[] U, Tensor terms, Tensor place, Tensor U_rows, Tensor meta, int out_dim) -> (Tensor, Tensor, Tensor)");
+    m.def("symmetric_contraction_backward(Tensor grad, Tensor x, Tensor keys, Tensor group, Tensor coef, Tensor[] weights, Tensor[] U, Tensor terms, Tensor place, Tensor U_rows, Tensor meta) -> (Tensor, Tensor[])");
+}
+TORCH_LIBRARY_IMPL(oeq_b200, CUDA, m) {
+    m.impl("symmetric_contraction", &symcon_forward);
+    m.impl("symmetric_contraction_backward", &symcon_backward);
+}
+TORCH_LIBRARY_IMPL(oeq_b200, Autograd, m) { m.impl("symmetric_contraction", &autograd_symcon); }
 
 TORCH_LIBRARY(libtorch_tp_jit, m) {
     m.def("jit_tp_forward(Tensor json_bytes, int hash, Tensor L1_in, Tensor L2_in, Tensor W, int L3_dim) -> Tensor");
