@@ -119,6 +119,7 @@ struct Desc {
     int fast_V = 1;          // edge streams per CTA of the first-order kernels (see kernels/fast_uvu.cuh); 1 = none
     int fast_SV = 0;         // stages per stream when fast_V > 1
     size_t fast_smemV = 0;
+    bool item = false;       // 'uvw' with a weight row per item: one block per item (kernels/uvw_item.cuh)
     size_t elt() const { return dtype == 2 ? 8 : 4; }
 };
 
@@ -306,6 +307,23 @@ bool parse_desc(const char* text, size_t len, Desc& d, std::string& why) {
         d.tc = d.tc && d.tc_smem[0] <= 232448;
         d.tc_bwd = d.tc_bwd && d.tc && d.tc_smem[1] <= 232448 && d.tc_smem[2] <= 232448;
         if (d.tc_bwd) { d.tc_ngrp = (int)tc_dw_groups(d, nullptr).size(); d.tc_dw_smem = tc_dw_smem_bytes(d); }
+    }
+    // 'uvw' with per-item weights: a block per item with all intermediates in (static) shared memory, in2 multiplicity 1.
+    d.item = false;
+    if (d.uvw && !d.shared && !d.conv && d.layout == 0) {
+        bool ok = d.dim[1] > 0 && d.dim[1] <= 32;
+        for (auto& b : d.L[0]) ok = ok && b.mul > 0;
+        for (auto& b : d.L[1]) ok = ok && b.mul == 1;
+        for (auto& b : d.L[2]) ok = ok && b.mul > 0;
+        size_t t = 0, g = 0;
+        for (auto& I : d.ins) {
+            const size_t n = (size_t)d.L[0][I.a].mul * d.L[2][I.o].d();
+            t += n;
+            g += n * ((d.L[2][I.o].mul + 31) / 32);
+        }
+        const size_t fwd = (size_t)d.dim[0] + d.dim[1] + t + 4 * (size_t)d.dim[2];
+        const size_t bwd = (size_t)d.dim[0] + 6 * (size_t)d.dim[1] + d.dim[2] + t + g;
+        d.item = ok && std::max(fwd, bwd) * d.elt() <= 48 * 1024 - 256;
     }
     return true;
 }
@@ -771,12 +789,13 @@ enum Family {
     FAM_UVW_TC,                                                  // tcgen05 'uvw' forward
     FAM_FAST_FWD3_TP, FAM_FAST_FWD3_DET,                         // fused second-order forward (three terms in one pass)
     FAM_UVW_TC_DX, FAM_UVW_TC_DY, FAM_UVW_TC_DW,                 // tcgen05 'uvw' backward: gradients of x, y and the weights
+    FAM_UVW_ITEM,                                                // 'uvw' with a weight row per item
     FAM_COUNT
 };
 const char* const kFamilyNames[FAM_COUNT] = {"generic", "fast_fwd_tp", "fast_fwd_det", "fast_fwd_atomic", "fast_bwd_tp",
                                              "fast_bwd_det", "fast_bwd_atomic", "fast_scatter", "fast_bwd2_tp",
                                              "fast_bwd2_det", "fast_bwd2_atomic", "uvw_tc", "fast_fwd3_tp", "fast_fwd3_det",
-                                             "uvw_tc_dx", "uvw_tc_dy", "uvw_tc_dw"};
+                                             "uvw_tc_dx", "uvw_tc_dy", "uvw_tc_dw", "uvw_item"};
 const char* family_name(int f) { return (f >= 0 && f < FAM_COUNT) ? kFamilyNames[f] : "?"; }
 int family_from_name(const std::string& n) {
     for (int f = 0; f < FAM_COUNT; ++f)
@@ -793,11 +812,26 @@ int family_streams(const Desc& d, int fam, bool allow) {
     return (allow && eligible && d.fast && d.fast_V > 1) ? d.fast_V : 1;
 }
 
+// Elements per access to a weight row: the largest power of two up to 16 bytes that divides the row and every offset in it.
+int item_vec(const Desc& d) {
+    int v = (int)(16 / d.elt());
+    auto divides = [&](int v) {
+        for (auto& I : d.ins) if (I.woff % v) return false;
+        return d.wn % v == 0;
+    };
+    while (v > 1 && !divides(v)) v /= 2;
+    return v;
+}
+
 std::string family_source(const Desc& d, const std::string& header, int fam, bool allow_streams = true) {
     std::string src = header;
     if (fam == FAM_GENERIC) {
         src += K_COMMON;
         src += K_GENERIC;
+    } else if (fam == FAM_UVW_ITEM) {
+        src += "constexpr int ITEM_VEC = " + std::to_string(item_vec(d)) + ";\n";
+        src += K_COMMON;
+        src += K_UVW_ITEM;
     } else if (fam == FAM_UVW_TC || (fam >= FAM_UVW_TC_DX && fam <= FAM_UVW_TC_DW)) {
         src += emit_tc(d, fam == FAM_UVW_TC ? 0 : fam - FAM_UVW_TC_DX + 1);
         src += K_COMMON;
@@ -1103,6 +1137,36 @@ int generic_backward(Entry* e, BwdParams p, cudaStream_t st) {
     if ((rc = get_kernel(prog, "oeq_generic_backward", 0, &k))) return rc;
     void* args[] = {&p};
     return launch(k, generic_grid(p.n_units), 128, 0, args, st);
+}
+
+// ------------------------------------------------------------------------------- 'uvw' with a weight row per item
+struct ItemFwdParams {
+    const void* x; const void* y; const void* W; void* z;
+    long long items;
+    int add;
+};
+struct ItemBwdParams {
+    const void* x; const void* y_dx; const void* y_dw; const void* W; const void* g;
+    void* dx; void* dy; void* dW;
+    long long items;
+    int add;
+};
+int item_launch(Entry* e, const char* name, void* params, long long items, cudaStream_t st) {
+    Program* prog;
+    if (int rc = get_program(e, FAM_UVW_ITEM, &prog)) return rc;
+    cudaKernel_t k;
+    if (int rc = get_kernel(prog, name, 0, &k)) return rc;
+    void* args[] = {params};
+    return launch(k, (unsigned)std::min<long long>(items, 1 << 30), 128, 0, args, st);
+}
+int item_forward(Entry* e, const void* x, const void* y, const void* W, void* z, long long items, int add, cudaStream_t st) {
+    ItemFwdParams p{x, y, W, z, items, add};
+    return item_launch(e, "oeq_uvw_item_forward", &p, items, st);
+}
+int item_backward(Entry* e, const void* x, const void* y_dx, const void* y_dw, const void* W, const void* g, void* dx, void* dy,
+                  void* dW, long long items, int add, cudaStream_t st) {
+    ItemBwdParams p{x, y_dx, y_dw, W, g, dx, dy, dW, items, add};
+    return item_launch(e, "oeq_uvw_item_backward", &p, items, st);
 }
 
 // ------------------------------------------------------------------------------- channel-parallel path
@@ -1551,6 +1615,7 @@ int oeqb_precompile(const void* desc, size_t desc_len, int64_t key) {
     for (int fam = 0; fam < FAM_COUNT; ++fam) {
         if (fam == FAM_UVW_TC) { if (!d.tc) continue; }
         else if (fam >= FAM_UVW_TC_DX && fam <= FAM_UVW_TC_DW) { if (!d.tc_bwd) continue; }
+        else if (fam == FAM_UVW_ITEM) { if (!d.item) continue; }
         else if (fam != FAM_GENERIC && !d.fast) continue;
         if (fam >= FAM_FAST_BWD2_TP && fam <= FAM_FAST_BWD2_ATOMIC && d.fast_S4 < 3) continue;
         if (fam == FAM_FAST_FWD_ATOMIC && d.fast_S3 < 2) continue;
@@ -1584,6 +1649,7 @@ int oeqb_tp_forward(const void* desc, size_t desc_len, int64_t key, int64_t batc
         TcParams t{x, y, W, z, nullptr, batch, 0, nullptr};
         return tc_forward(e, t, (cudaStream_t)stream);
     }
+    if (e->d.item && !g_force_generic && aligned16({W})) return item_forward(e, x, y, W, z, batch, 0, (cudaStream_t)stream);
     FwdParams p{x, y, W, z, nullptr, nullptr, batch, batch, UNIT_ITEM, OUT_STORE};
     return generic_forward(e, p, (cudaStream_t)stream);
 }
@@ -1603,6 +1669,7 @@ int oeqb_tp_backward(const void* desc, size_t desc_len, int64_t key, int64_t bat
         FastParams f{x, y, W, g, nullptr, dx, dy, dW, nullptr, nullptr, nullptr, batch, batch, nullptr};
         return fast_launch(e, 3, f, st);
     }
+    if (d.item && !g_force_generic && aligned16({W, dW})) return item_backward(e, x, y, y, W, g, dx, dy, dW, batch, 0, st);
     const int tcb = (d.tc_bwd && !g_force_generic && !g_no_tc && aligned16({x, dx, g})) ? g_tc_backward : 0;
     if (tcb != 7) {
         CUDA_TRY(cudaMemsetAsync(dy, 0, batch * d.dim[1] * d.elt(), st));
@@ -1654,6 +1721,13 @@ int oeqb_tp_double_backward(const void* desc, size_t desc_len, int64_t key, int6
         if ((rc = tc_forward(e, t, st, 0))) return rc;
         if ((rc = tc_backward(e, 7, x2, y2, y, W, g, dx, dy, dW, batch, 0, st))) return rc;
         return tc_backward(e, 7, x, y, y2, W2, g, dx, dy, dW, batch, 1, st);
+    }
+    if (d.item && !g_force_generic && aligned16({W, W2, dW})) {   // the five passes of the general path below
+        if ((rc = item_forward(e, x2, y, W, dg, batch, 0, st))) return rc;
+        if ((rc = item_forward(e, x, y2, W, dg, batch, 1, st))) return rc;
+        if ((rc = item_forward(e, x, y, W2, dg, batch, 1, st))) return rc;
+        if ((rc = item_backward(e, x2, y2, y, W, g, dx, dy, dW, batch, 0, st))) return rc;
+        return item_backward(e, x, y, y2, W2, g, dx, dy, dW, batch, 1, st);
     }
     CUDA_TRY(cudaMemsetAsync(dy, 0, batch * d.dim[1] * d.elt(), st));
     // dg = F(x2, y, W) + F(x, y2, W) + F(x, y, W2): the product is linear in each argument
