@@ -12,8 +12,9 @@
 // the cotangent (or the sum) of those columns stays in registers and the sum over w is log2(PP) shuffles per row of VEC * P.
 // All sums run in an order fixed by the problem: bitwise reproducible.
 //
-// DiffDock L = 2 (multiplicities 10 and 48, 7,128 weights), 8,191 items: forward 65 us (3.8 TB/s of rows), backward 195 us (2.6 TB/s);
-// the general kernels (a warp per item, strided stores of dW, a shuffle per product) took 733 us for both.
+// DiffDock L = 2 (multiplicities 10 and 48, 7,128 weights), 8,191 items: forward 65 us (3.8 TB/s of rows), backward 147 us (3.4 TB/s;
+// 195 us with five blocks of 127 registers to an SM instead of eight of 64); the general kernels (a warp per item, strided stores of
+// dW, a shuffle per product) took 733 us for both.
 #pragma once
 
 // ITEM_VEC (emitted): the largest power of two up to 16 bytes that divides the row length and every weight offset.
@@ -160,7 +161,7 @@ struct ItemBwdParams {
     int add;
 };
 
-extern "C" __global__ void __launch_bounds__(ITEM_WARPS * 32) oeq_uvw_item_backward(const ItemBwdParams p) {
+extern "C" __global__ void __launch_bounds__(ITEM_WARPS * 32, sizeof(T) == 4 ? 8 : 4) oeq_uvw_item_backward(const ItemBwdParams p) {
     __shared__ T xs[L1_DIM], y1[L2_DIM], y2[L2_DIM], gs[L3_DIM], ts[ItemOff<NINS>::T0], gp[ItemOff<NINS>::G0], dys[ITEM_WARPS][L2_DIM];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (long long b = blockIdx.x; b < p.items; b += gridDim.x) {
