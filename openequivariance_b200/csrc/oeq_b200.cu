@@ -120,6 +120,7 @@ struct Desc {
     int fast_SV = 0;         // stages per stream when fast_V > 1
     size_t fast_smemV = 0;
     bool item = false;       // 'uvw' with a weight row per item: one block per item (kernels/uvw_item.cuh)
+    int f64mm = 0;           // 'uvw' in doubles on the FP64 matrix instruction: number of 32 x 32 weight tiles (0: not applicable)
     size_t elt() const { return dtype == 2 ? 8 : 4; }
 };
 
@@ -307,6 +308,18 @@ bool parse_desc(const char* text, size_t len, Desc& d, std::string& why) {
         d.tc = d.tc && d.tc_smem[0] <= 232448;
         d.tc_bwd = d.tc_bwd && d.tc && d.tc_smem[1] <= 232448 && d.tc_smem[2] <= 232448;
         if (d.tc_bwd) { d.tc_ngrp = (int)tc_dw_groups(d, nullptr).size(); d.tc_dw_smem = tc_dw_smem_bytes(d); }
+    }
+    // 'uvw' in doubles, shared weights: multiplicities that are multiples of 32 and in2 multiplicity 1, as on the tensor-core
+    // path; l <= 3 for the accumulators' registers, and no more weight tiles than compile to a few hundred KB of code.
+    d.f64mm = 0;
+    if (d.dtype == 2 && d.layout == 0 && d.uvw && d.shared && !d.conv) {
+        bool ok = d.dim[1] > 0 && d.dim[1] <= 16;
+        for (auto& b : d.L[0]) ok = ok && b.mul > 0 && b.mul % 32 == 0 && b.l <= 3;
+        for (auto& b : d.L[1]) ok = ok && b.mul == 1 && b.l <= 3;
+        for (auto& b : d.L[2]) ok = ok && b.mul > 0 && b.mul % 32 == 0 && b.l <= 3;
+        long long tiles = 0;
+        if (ok) for (auto& I : d.ins) tiles += (long long)(d.L[0][I.a].mul / 32) * (d.L[2][I.o].mul / 32);
+        if (ok && tiles <= 128) d.f64mm = (int)tiles;
     }
     // 'uvw' with per-item weights: a block per item with all intermediates in (static) shared memory, in2 multiplicity 1.
     d.item = false;
@@ -790,12 +803,13 @@ enum Family {
     FAM_FAST_FWD3_TP, FAM_FAST_FWD3_DET,                         // fused second-order forward (three terms in one pass)
     FAM_UVW_TC_DX, FAM_UVW_TC_DY, FAM_UVW_TC_DW,                 // tcgen05 'uvw' backward: gradients of x, y and the weights
     FAM_UVW_ITEM,                                                // 'uvw' with a weight row per item
+    FAM_UVW_F64,                                                 // 'uvw' in doubles on the FP64 matrix instruction
     FAM_COUNT
 };
 const char* const kFamilyNames[FAM_COUNT] = {"generic", "fast_fwd_tp", "fast_fwd_det", "fast_fwd_atomic", "fast_bwd_tp",
                                              "fast_bwd_det", "fast_bwd_atomic", "fast_scatter", "fast_bwd2_tp",
                                              "fast_bwd2_det", "fast_bwd2_atomic", "uvw_tc", "fast_fwd3_tp", "fast_fwd3_det",
-                                             "uvw_tc_dx", "uvw_tc_dy", "uvw_tc_dw", "uvw_item"};
+                                             "uvw_tc_dx", "uvw_tc_dy", "uvw_tc_dw", "uvw_item", "uvw_f64"};
 const char* family_name(int f) { return (f >= 0 && f < FAM_COUNT) ? kFamilyNames[f] : "?"; }
 int family_from_name(const std::string& n) {
     for (int f = 0; f < FAM_COUNT; ++f)
@@ -832,6 +846,9 @@ std::string family_source(const Desc& d, const std::string& header, int fam, boo
         src += "constexpr int ITEM_VEC = " + std::to_string(item_vec(d)) + ";\n";
         src += K_COMMON;
         src += K_UVW_ITEM;
+    } else if (fam == FAM_UVW_F64) {
+        src += K_COMMON;
+        src += K_UVW_F64;
     } else if (fam == FAM_UVW_TC || (fam >= FAM_UVW_TC_DX && fam <= FAM_UVW_TC_DW)) {
         src += emit_tc(d, fam == FAM_UVW_TC ? 0 : fam - FAM_UVW_TC_DX + 1);
         src += K_COMMON;
@@ -1167,6 +1184,57 @@ int item_backward(Entry* e, const void* x, const void* y_dx, const void* y_dw, c
                   void* dW, long long items, int add, cudaStream_t st) {
     ItemBwdParams p{x, y_dx, y_dw, W, g, dx, dy, dW, items, add};
     return item_launch(e, "oeq_uvw_item_backward", &p, items, st);
+}
+
+// ------------------------------------------------------------------------------- 'uvw' in doubles, shared weights
+struct F64FwdParams { const void* x; const void* y; const void* W; void* z; long long batch; int accum; };
+struct F64BwdParams { const void* x; const void* y; const void* W; const void* g; void* dx; void* dy; long long batch; int accum; };
+struct F64DwParams { const void* x; const void* y; const void* g; void* part; long long batch; int chunk; };
+int f64_launch(Entry* e, const char* name, dim3 grid, void* params, cudaStream_t st) {
+    Program* prog;
+    if (int rc = get_program(e, FAM_UVW_F64, &prog)) return rc;
+    cudaKernel_t k;
+    if (int rc = get_kernel(prog, name, 0, &k)) return rc;
+    void* args[] = {params};
+    cudaError_t ce = cudaLaunchKernel((const void*)k, grid, dim3(128), args, 0, st);
+    if (ce != cudaSuccess) return fail(OEQB_ECUDA, "%s: %s", name, cudaGetErrorString(ce));
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    return OEQB_OK;
+}
+int f64_forward(Entry* e, const void* x, const void* y, const void* W, void* z, long long batch, int accum, cudaStream_t st) {
+    int tiles = 0;
+    for (auto& b : e->d.L[2]) tiles += b.mul / 32;
+    F64FwdParams p{x, y, W, z, batch, accum};
+    return f64_launch(e, "oeq_uvw_f64_forward", dim3((unsigned)((batch + 31) / 32), (unsigned)tiles), &p, st);
+}
+// dW is added to (the caller zeroes it); dx and dy are stored, or added to with accum
+int f64_backward(Entry* e, const void* x, const void* y_dx, const void* y_dw, const void* W, const void* g, void* dx, void* dy,
+                 void* dW, long long batch, int accum, cudaStream_t st) {
+    const Desc& d = e->d;
+    F64BwdParams p{x, y_dx, W, g, dx, dy, batch, accum};
+    int rc = f64_launch(e, "oeq_uvw_f64_backward", dim3((unsigned)((batch + 7) / 8)), &p, st);
+    if (rc) return rc;
+    Program* gen;
+    if ((rc = get_program(e, FAM_GENERIC, &gen))) return rc;
+    cudaKernel_t kr;
+    if ((rc = get_kernel(gen, "oeq_generic_dw_reduce", 0, &kr))) return rc;
+    // Items per row of partial sums, by the batch alone (so results do not depend on the device): about 80 rows keep the chip
+    // busy with few paths, and a row costs wn doubles written and read once.
+    int chunk = (int)std::min<long long>(std::max<long long>((batch + 79) / 80, 16), 4096);
+    chunk = (chunk + 3) & ~3;
+    long long chunks = (batch + chunk - 1) / chunk;
+    if ((rc = keep_pool_memory())) return rc;
+    void* part = nullptr;
+    CUDA_TRY(cudaMallocAsync(&part, (size_t)chunks * d.wn * sizeof(double), st));
+    F64DwParams q{x, y_dw, g, part, batch, chunk};
+    rc = f64_launch(e, "oeq_uvw_f64_backward_dw", dim3((unsigned)chunks, (unsigned)((d.f64mm + 3) / 4)), &q, st);
+    if (!rc) {
+        int add = 1;
+        void* rargs[] = {&part, &chunks, &dW, &add};
+        rc = launch(kr, (unsigned)((d.wn + 31) / 32), 256, 0, rargs, st);
+    }
+    cudaFreeAsync(part, st);
+    return rc;
 }
 
 // ------------------------------------------------------------------------------- channel-parallel path
@@ -1616,6 +1684,7 @@ int oeqb_precompile(const void* desc, size_t desc_len, int64_t key) {
         if (fam == FAM_UVW_TC) { if (!d.tc) continue; }
         else if (fam >= FAM_UVW_TC_DX && fam <= FAM_UVW_TC_DW) { if (!d.tc_bwd) continue; }
         else if (fam == FAM_UVW_ITEM) { if (!d.item) continue; }
+        else if (fam == FAM_UVW_F64) { if (!d.f64mm) continue; }
         else if (fam != FAM_GENERIC && !d.fast) continue;
         if (fam >= FAM_FAST_BWD2_TP && fam <= FAM_FAST_BWD2_ATOMIC && d.fast_S4 < 3) continue;
         if (fam == FAM_FAST_FWD_ATOMIC && d.fast_S3 < 2) continue;
@@ -1633,6 +1702,9 @@ int oeqb_precompile(const void* desc, size_t desc_len, int64_t key) {
     return done;
 }
 
+// (the launches cover 8 items per block: the x extent of a grid ends at 2^31 - 1)
+static bool f64_route(const Desc& d, int64_t batch) { return d.f64mm > 0 && !g_force_generic && batch <= (1LL << 33); }
+
 int oeqb_tp_forward(const void* desc, size_t desc_len, int64_t key, int64_t batch, const void* x, const void* y,
                     const void* W, void* z, void* stream) {
     if (batch < 0) return fail(OEQB_EINVAL, "oeqb_tp_forward: negative batch");
@@ -1649,6 +1721,7 @@ int oeqb_tp_forward(const void* desc, size_t desc_len, int64_t key, int64_t batc
         TcParams t{x, y, W, z, nullptr, batch, 0, nullptr};
         return tc_forward(e, t, (cudaStream_t)stream);
     }
+    if (f64_route(e->d, batch)) return f64_forward(e, x, y, W, z, batch, 0, (cudaStream_t)stream);
     if (e->d.item && !g_force_generic && aligned16({W})) return item_forward(e, x, y, W, z, batch, 0, (cudaStream_t)stream);
     FwdParams p{x, y, W, z, nullptr, nullptr, batch, batch, UNIT_ITEM, OUT_STORE};
     return generic_forward(e, p, (cudaStream_t)stream);
@@ -1669,6 +1742,7 @@ int oeqb_tp_backward(const void* desc, size_t desc_len, int64_t key, int64_t bat
         FastParams f{x, y, W, g, nullptr, dx, dy, dW, nullptr, nullptr, nullptr, batch, batch, nullptr};
         return fast_launch(e, 3, f, st);
     }
+    if (f64_route(d, batch)) return f64_backward(e, x, y, y, W, g, dx, dy, dW, batch, 0, st);
     if (d.item && !g_force_generic && aligned16({W, dW})) return item_backward(e, x, y, y, W, g, dx, dy, dW, batch, 0, st);
     const int tcb = (d.tc_bwd && !g_force_generic && !g_no_tc && aligned16({x, dx, g})) ? g_tc_backward : 0;
     if (tcb != 7) {
@@ -1721,6 +1795,13 @@ int oeqb_tp_double_backward(const void* desc, size_t desc_len, int64_t key, int6
         if ((rc = tc_forward(e, t, st, 0))) return rc;
         if ((rc = tc_backward(e, 7, x2, y2, y, W, g, dx, dy, dW, batch, 0, st))) return rc;
         return tc_backward(e, 7, x, y, y2, W2, g, dx, dy, dW, batch, 1, st);
+    }
+    if (f64_route(d, batch)) {   // the five passes of the general path below
+        if ((rc = f64_forward(e, x2, y, W, dg, batch, 0, st))) return rc;
+        if ((rc = f64_forward(e, x, y2, W, dg, batch, 1, st))) return rc;
+        if ((rc = f64_forward(e, x, y, W2, dg, batch, 1, st))) return rc;
+        if ((rc = f64_backward(e, x2, y2, y, W, g, dx, dy, dW, batch, 0, st))) return rc;
+        return f64_backward(e, x, y, y2, W2, g, dx, dy, dW, batch, 1, st);
     }
     if (d.item && !g_force_generic && aligned16({W, W2, dW})) {   // the five passes of the general path below
         if ((rc = item_forward(e, x2, y, W, dg, batch, 0, st))) return rc;
