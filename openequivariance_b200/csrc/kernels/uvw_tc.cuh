@@ -27,6 +27,9 @@ struct TcParams {
     long long batch;
     int accum;          // add to what z holds instead of overwriting it
     int* status;
+    int splits;         // a tile's schedule of paths is shared by this many CTAs: part s takes paths cut[s] .. cut[s + 1]
+    int cut[9];
+    float* parts; int* count;   // mode 2 with splits > 1: [splits][batch][L2] partial sums of dy, and the finished parts of every tile
 };
 
 OEQ_DEV unsigned tc_smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -134,6 +137,7 @@ struct __align__(128) TcShared {
     unsigned long long xs_full[2];    // a staged input block has arrived (bytes of the bulk copies), per staging buffer
     unsigned tmem_base;
     int abort_flag;
+    int last_part;
 };
 // One CTA per SM is assumed (it owns all of TMEM): the host asks for more than half of the shared memory even when the
 // buffers need less.
@@ -205,7 +209,7 @@ OEQ_DEV void tc_cg(const float* xrow, const float* yrow, int t0, int t1, float (
 // stores), buffers come back through mma_done, finished accumulators through acc_done (tcgen05.commit).  The compute
 // warps meet among themselves (named barrier) only where the staged input block changes hands.  A thread that gave up
 // keeps walking the loops and joining those barriers without doing work, so nobody waits for it.
-extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const TcParams p) {
+extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const __grid_constant__ TcParams p) {
     extern __shared__ __align__(128) unsigned char tc_smem_raw[];
     TcShared& sh = *reinterpret_cast<TcShared*>(tc_smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -226,7 +230,9 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const
     __syncthreads();
     tc_fence_after();
     const unsigned tmem = sh.tmem_base;
-    const long long ntiles = (p.batch + 127) / 128;
+    // A unit of work is a tile and a part of the schedule, cut where a destination block ends.  One part needs the least staging;
+    // more parts fill the chip when there are few tiles, or a last wave that would be nearly empty (the host counts).
+    const long long nunits = (p.batch + 127) / 128 * p.splits;
     unsigned step = 0;     // chunk steps so far: operand buffer = step & 1
     unsigned npath = 0;    // paths started so far: weight buffer = npath & 1
     unsigned nblock = 0;   // output blocks finished so far: accumulator half = nblock & 1
@@ -239,8 +245,9 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const
         const unsigned long long da1h = tc_desc(&sh.a[1][0][0], TC_LBO, TC_SBO), da1l = tc_desc(&sh.a[1][1][0], TC_LBO, TC_SBO);
         const unsigned long long db0h = tc_desc(&sh.b[0][0][0], TC_LBO, TC_SBO), db0l = tc_desc(&sh.b[0][1][0], TC_LBO, TC_SBO);
         const unsigned long long db1h = tc_desc(&sh.b[1][0][0], TC_LBO, TC_SBO), db1l = tc_desc(&sh.b[1][1][0], TC_LBO, TC_SBO);
-        for (long long tile = blockIdx.x; tile < ntiles && !dead; tile += gridDim.x) {
-            for (int q = 0; q < TC_NPATH && !dead; ++q) {
+        for (long long unit = blockIdx.x; unit < nunits && !dead; unit += gridDim.x) {
+            const int part = (int)(unit % p.splits), q1 = p.cut[part + 1];
+            for (int q = p.cut[part]; q < q1 && !dead; ++q) {
                 const int d3 = TC_D3[q], first = TC_FIRST[q], last = TC_LAST[q];
                 for (int k = 0; k < d3 && !dead; ++k) {
                     const unsigned buf = step & 1u;
@@ -278,9 +285,11 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const
         float gnext[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // mode 2: the next step's cotangent values
         float wnext[1024 / TC_CT];                                    // this thread's entries of the next path's weight block
 #pragma unroll
-        for (int r = 0; r < 1024 / TC_CT; ++r) wnext[r] = __ldg(p.W + TC_WOFF[0] + tid + TC_CT * r);
-        for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-            const long long item0 = tile * 128;
+        for (int r = 0; r < 1024 / TC_CT; ++r) wnext[r] = __ldg(p.W + TC_WOFF[p.cut[blockIdx.x % p.splits]] + tid + TC_CT * r);
+        for (long long unit = blockIdx.x; unit < nunits; unit += gridDim.x) {
+            const int part_s = (int)(unit % p.splits), q0 = p.cut[part_s], q1 = p.cut[part_s + 1];
+            const int qnext = p.cut[(unit + gridDim.x) % p.splits];   // first path of this CTA's next unit
+            const long long item0 = unit / p.splits * 128;
             int pre_q = -1;      // path whose block has been requested ahead (none across tiles)
             tc_compute_sync();   // previous tile's readers of xs / ys / dys are done
             if (TC_MODE != 2) {
@@ -290,13 +299,13 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const
             } else {
                 for (int j = 0; j < TC_DYS; ++j) sh.dys[tid * TC_DYS + j] = 0.f;   // read and written by this thread only
             }
-            for (int q = 0; q < TC_NPATH; ++q) {
+            for (int q = q0; q < q1; ++q) {
                 const int d1 = TC_D1[q], d3 = TC_D3[q], xoff = TC_XOFF[q], zoff = TC_ZOFF[q], woff = TC_WOFF[q];
                 const int tq = TC_INS[q] * 8;   // this path's instruction: start of its term ranges
                 const int last = TC_LAST[q];
                 // stage the path's input block by asynchronous row copies; the block stays when the previous path of this
                 // tile read the same one
-                const bool restage = q == 0 || TC_XOFF[q - 1] != xoff;
+                const bool restage = q == q0 || TC_XOFF[q - 1] != xoff;
                 tc_compute_sync();   // readers of the previous path's block are done
                 if (TC_MODE != 2) {
                     // One bulk copy per row, issued by the first 128 threads; everybody waits for the bytes to arrive.  Rows past
@@ -318,7 +327,7 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const
                         if (!tc_mbar_wait(&sh.xs_full[cur], nfill[cur] & 1u, abortf, p.status, 37)) dead = true;
                         ++nfill[cur];
                         const int qn = TC_NEXTX[q];   // first later path of the schedule that stages another block, or -1
-                        if (!dead && qn >= 0 && TC_D1[qn] <= (cur ? TC_MAXD1 : TC_XS2_D1)) { request(cur ^ 1, qn); pre_q = qn; }
+                        if (!dead && qn >= 0 && qn < q1 && TC_D1[qn] <= (cur ? TC_MAXD1 : TC_XS2_D1)) { request(cur ^ 1, qn); pre_q = qn; }
                     }
                 } else {
                     if (restage && !dead) {   // warp w copies rows w, w + 16, ... (odd row stride: 4-byte pieces)
@@ -355,14 +364,14 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const
                         const long long b0 = item0 + brow;
                         const bool live = b0 < p.batch;
                         const float* grow = p.g + (live ? b0 : 0) * L3_DIM;
-                        if (q == 0 && k == 0) {
+                        if (q == q0 && k == 0) {
 #pragma unroll
                             for (int uu = 0; uu < 8; ++uu) gnext[uu] = live ? __ldg(grow + zoff + (ucol + 4 * uu) * d3) : 0.f;
                         }
 #pragma unroll
                         for (int uu = 0; uu < 8; ++uu) acc[uu] = gnext[uu];
                         const bool more = k + 1 < d3;
-                        if (more || q + 1 < TC_NPATH) {
+                        if (more || q + 1 < q1) {
                             const int nd3 = more ? d3 : TC_D3[q + 1];
                             const float* gn = grow + (more ? zoff + k + 1 : TC_ZOFF[q + 1]) + ucol * nd3;
 #pragma unroll
@@ -385,7 +394,7 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const
                                 sh.b[npath & 1u][0][off] = hi;
                                 sh.b[npath & 1u][1][off] = tc_tf32(v - hi);
                             }
-                            const int wq = (q + 1 < TC_NPATH) ? TC_WOFF[q + 1] : TC_WOFF[0];   // the next path's (or next tile's first)
+                            const int wq = TC_WOFF[q + 1 < q1 ? q + 1 : qnext];   // the next path's (or the next unit's first)
 #pragma unroll
                             for (int r = 0; r < 1024 / TC_CT; ++r) wnext[r] = __ldg(p.W + wq + tid + TC_CT * r);
                         }
@@ -446,13 +455,32 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const
                 // dy of the tile: threads t, t + 128, ... hold the channel parts of item t
                 tc_compute_sync();
                 const long long b = item0 + tid;
-                if (tid < 128 && b < p.batch && !sh.abort_flag)
+                const bool live = tid < 128 && b < p.batch && !sh.abort_flag;
+                if (live) {
+                    float* out = p.splits > 1 ? p.parts + (part_s * p.batch + b) * L2_DIM : p.z + b * L2_DIM;
+                    const bool add = p.splits == 1 && p.accum;
                     for (int j = 0; j < L2_DIM; ++j) {
                         float v = 0.f;
 #pragma unroll
                         for (int part = 0; part < TC_CW / 4; ++part) v += sh.dys[(tid + 128 * part) * TC_DYS + j];
-                        p.z[b * L2_DIM + j] = p.accum ? p.z[b * L2_DIM + j] + v : v;
+                        out[j] = add ? out[j] + v : v;
                     }
+                }
+                if (p.splits > 1) {
+                    // the part that finishes a tile last adds the parts' rows in the order of the schedule
+                    __threadfence();
+                    tc_compute_sync();
+                    if (tid == 0) sh.last_part = atomicAdd(p.count + unit / p.splits, 1) == p.splits - 1;
+                    tc_compute_sync();
+                    if (live && sh.last_part) {
+                        __threadfence();
+                        for (int j = 0; j < L2_DIM; ++j) {
+                            float v = p.accum ? p.z[b * L2_DIM + j] : 0.f;
+                            for (int s = 0; s < p.splits; ++s) v += __ldcg(p.parts + (s * p.batch + b) * L2_DIM + j);
+                            p.z[b * L2_DIM + j] = v;
+                        }
+                    }
+                }
             }
         }
     }
@@ -481,8 +509,9 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const
 struct TcDwParams {
     const float* x; const float* y; const float* g; float* part;
     long long batch;
-    int grp_begin, grp_end;   // this launch's groups (at most 16: one 32-column accumulator each)
     int* status;
+    int splits;               // a unit of work is a tile and a part of the groups, as in TcParams
+    int cut[9];               // part s: groups cut[s] .. cut[s + 1] (at most 16: one 32-column accumulator each)
 };
 constexpr int TCW_TILE = 64;
 constexpr int TCW_YS = L2_DIM | 1;
@@ -516,7 +545,7 @@ OEQ_DEV void tcw_cg(const float* xt, const float* yb, int t0, int t1, float (&ac
 }
 static_assert(sizeof(TcDwShared) <= 232448, "the buffers exceed shared memory");   // (one CTA per SM: see TcShared)
 
-extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) oeq_uvw_tc_backward_dw(const TcDwParams p) {
+extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) oeq_uvw_tc_backward_dw(const __grid_constant__ TcDwParams p) {
     extern __shared__ __align__(128) unsigned char tc_smem_raw[];
     TcDwShared& sh = *reinterpret_cast<TcDwShared*>(tc_smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -536,7 +565,7 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) oeq_uvw_tc_backward_
     __syncthreads();
     tc_fence_after();
     const unsigned tmem = sh.tmem_base;
-    const long long ntiles = (p.batch + TCW_TILE - 1) / TCW_TILE;
+    const long long nunits = (p.batch + TCW_TILE - 1) / TCW_TILE * p.splits;
     unsigned step = 0;     // steps so far: operand buffer = step & 1
     bool dead = false;
 
@@ -546,15 +575,16 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) oeq_uvw_tc_backward_
         const unsigned long long da1h = tc_desc(&sh.a[1][0][0], TC_LBO, TC_SBO), da1l = tc_desc(&sh.a[1][1][0], TC_LBO, TC_SBO);
         const unsigned long long db0h = tc_desc(&sh.b[0][0][0], TC_LBO, TC_SBO), db0l = tc_desc(&sh.b[0][1][0], TC_LBO, TC_SBO);
         const unsigned long long db1h = tc_desc(&sh.b[1][0][0], TC_LBO, TC_SBO), db1l = tc_desc(&sh.b[1][1][0], TC_LBO, TC_SBO);
-        for (long long tile = blockIdx.x; tile < ntiles && !dead; tile += gridDim.x) {
-            for (int grp = p.grp_begin; grp < p.grp_end && !dead; ++grp) {
+        for (long long unit = blockIdx.x; unit < nunits && !dead; unit += gridDim.x) {
+            const int g0 = p.cut[unit % p.splits], g1 = p.cut[unit % p.splits + 1];
+            for (int grp = g0; grp < g1 && !dead; ++grp) {
                 const int d3 = TCW_D3[grp];
                 for (int kh = 0; kh < 2 * d3 && !dead; ++kh) {   // (component k, half of the tile)
                     const unsigned buf = step & 1u;
                     if (!tc_mbar_wait(&sh.a_full[buf], (step >> 1) & 1u, abortf, p.status, 36)) { dead = true; break; }
                     tc_fence_after();
                     if (lane == 0) {
-                        const unsigned dcol = tmem + 32u * (unsigned)(grp - p.grp_begin);
+                        const unsigned dcol = tmem + 32u * (unsigned)(grp - g0);
                         const unsigned long long ah0 = buf ? da1h : da0h, al0 = buf ? da1l : da0l;
                         const unsigned long long bh0 = buf ? db1h : db0h, bl0 = buf ? db1l : db0l;
 #pragma unroll
@@ -575,14 +605,15 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) oeq_uvw_tc_backward_
     } else {
         const int slot = warp & 3, sub = warp >> 2, r8 = lane >> 2, b4 = lane & 3;
         unsigned nstage = 0;   // staged groups so far (phase of xs_full)
-        for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-            const long long item0 = tile * TCW_TILE;
+        for (long long unit = blockIdx.x; unit < nunits; unit += gridDim.x) {
+            const long long tile = unit / p.splits, item0 = tile * TCW_TILE;
+            const int g0 = p.cut[unit % p.splits], g1 = p.cut[unit % p.splits + 1];
             const long long nlive = p.batch - item0;         // items of the tile that exist
             tc_compute_sync();   // the previous tile's readers of ys are done
             for (int r = warp; r < TCW_TILE; r += TC_CW)
                 for (int j = lane; j < L2_DIM; j += 32)
                     sh.ys[r * TCW_YS + j] = (r < nlive) ? __ldg(p.y + (item0 + r) * L2_DIM + j) : 0.f;
-            for (int grp = p.grp_begin; grp < p.grp_end; ++grp) {
+            for (int grp = g0; grp < g1; ++grp) {
                 const int d3 = TCW_D3[grp], zoff = TCW_ZOFF[grp], ns = TCW_NS[grp];
                 // stage the slots' input blocks: one bulk copy per (slot, row), issued by the first 64 * ns threads; everybody
                 // waits for the bytes.  Rows past the end of the batch read row 0 and meet y = 0.
@@ -663,10 +694,10 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) oeq_uvw_tc_backward_
             if (!dead && step >= 1) {
                 tc_fence_after();
                 float* prow = p.part + tile * WN;
-                for (int grp = p.grp_begin; grp < p.grp_end; ++grp) {
+                for (int grp = g0; grp < g1; ++grp) {
                     if (slot >= TCW_NS[grp]) continue;   // uniform in the warp
                     unsigned r[8];
-                    tc_ld8(tmem + ((unsigned)(slot * 32) << 16) + 32u * (unsigned)(grp - p.grp_begin) + (unsigned)(TC_EC * sub), r);
+                    tc_ld8(tmem + ((unsigned)(slot * 32) << 16) + 32u * (unsigned)(grp - g0) + (unsigned)(TC_EC * sub), r);
                     float4* dst = reinterpret_cast<float4*>(prow + TCW_WOFF[grp * 4 + slot] + lane * 32 + TC_EC * sub);
                     dst[0] = make_float4(__uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2]), __uint_as_float(r[3]));
                     dst[1] = make_float4(__uint_as_float(r[4]), __uint_as_float(r[5]), __uint_as_float(r[6]), __uint_as_float(r[7]));

@@ -649,16 +649,9 @@ void emit_tc_terms(std::ostringstream& s, const Desc& d, bool by_i, const char* 
 }
 
 std::string emit_tc_dw(const Desc& d);
-std::string emit_tc(const Desc& d, int mode = 0) {
-    std::ostringstream s;
-    if (!d.tc) { s << "#define OEQ_TC 0\n"; return s.str(); }
-    if (mode == 3) return emit_tc_dw(d);
-    s << "#define OEQ_TC 1\n";
+// Order of the paths (indices of tc_subpaths) in a kernel of mode 0 to 2, and which of them begin and end a destination tile.
+std::vector<int> tc_schedule(const Desc& d, int mode, std::vector<int>* first_out, std::vector<int>* last_out) {
     const bool dx = mode == 1, dy = mode == 2;
-    s << "#define TC_MODE " << mode << "\n";
-    s << "#define TC_WT " << (mode != 0 ? 1 : 0) << "\n";
-    s << "#define TC_KERNEL_NAME " << (dx ? "oeq_uvw_tc_backward_dx" : dy ? "oeq_uvw_tc_backward_dy" : "oeq_uvw_tc_forward") << "\n";
-    s << "constexpr int TC_IN_DIM = " << (dx ? d.dim[2] : d.dim[0]) << ", TC_OUT_DIM = " << (dx ? d.dim[0] : d.dim[2]) << ";\n";
     const std::vector<TcSub> subs = tc_subpaths(d);
     // mode 2 (dy) accumulates nowhere across paths: every path is its own group; the paths are ordered by the input
     // tile they stage
@@ -682,11 +675,30 @@ std::string emit_tc(const Desc& d, int mode = 0) {
         }
         g0 = g1;
     }
-    std::vector<int> first(subs.size(), 0), last(subs.size(), 0);
+    std::vector<int>& first = *first_out;
+    std::vector<int>& last = *last_out;
+    first.assign(subs.size(), 0);
+    last.assign(subs.size(), 0);
     for (size_t q = 0; q < order.size(); ++q) {
         if (q == 0 || dst(order[q - 1]) != dst(order[q])) first[order[q]] = 1;
         if (q + 1 == order.size() || dst(order[q + 1]) != dst(order[q])) last[order[q]] = 1;
     }
+    return order;
+}
+
+std::string emit_tc(const Desc& d, int mode = 0) {
+    std::ostringstream s;
+    if (!d.tc) { s << "#define OEQ_TC 0\n"; return s.str(); }
+    if (mode == 3) return emit_tc_dw(d);
+    s << "#define OEQ_TC 1\n";
+    const bool dx = mode == 1, dy = mode == 2;
+    s << "#define TC_MODE " << mode << "\n";
+    s << "#define TC_WT " << (mode != 0 ? 1 : 0) << "\n";
+    s << "#define TC_KERNEL_NAME " << (dx ? "oeq_uvw_tc_backward_dx" : dy ? "oeq_uvw_tc_backward_dy" : "oeq_uvw_tc_forward") << "\n";
+    s << "constexpr int TC_IN_DIM = " << (dx ? d.dim[2] : d.dim[0]) << ", TC_OUT_DIM = " << (dx ? d.dim[0] : d.dim[2]) << ";\n";
+    std::vector<int> first, last;
+    const std::vector<TcSub> subs = tc_subpaths(d);
+    const std::vector<int> order = tc_schedule(d, mode, &first, &last);
     // run-time tables, one entry per path in schedule order
     auto ilist = [&](const char* name, const std::vector<long long>& v) {
         s << "__constant__ int " << name << "[" << (v.empty() ? 1 : v.size()) << "] = {";
@@ -969,6 +981,18 @@ struct Program {
     bool regs_checked = false;            // multi-stream kernels: register count verified against the hand-over scheme
 };
 
+// How the schedule of a tensor-core kernel is cut into parts (see TcParams::splits): for S parts the boundaries that make the
+// costliest part cheapest, a group (destination tile, or stack of paths for dW) never being cut.  Unit of cost: one step.
+struct TcCuts {
+    std::vector<int> begin;                   // first path (mode 3: first group) of every group, and the end
+    std::vector<double> cost;
+    int n[9] = {0};                           // parts that S asks for (fewer when there are fewer groups)
+    int cut[9][9] = {{0}};
+    double part[9][8] = {{0}};
+    long long seen_tiles = -1;                // the last choice
+    int seen_splits = 0;
+};
+
 struct Entry {
     Desc d;
     uint64_t desc_hash = 0;     // of the descriptor text this entry was built from: a key reused for another problem is refused
@@ -976,6 +1000,7 @@ struct Entry {
     const void* seen_ptr = nullptr;   // last caller buffer whose contents were compared (callers pass the same buffer again)
     std::string header;
     std::unique_ptr<Program> prog[FAM_COUNT];
+    std::unique_ptr<TcCuts> tc_cuts[4];                 // how the tensor-core kernels' schedules are cut, by mode (3: dW)
     std::unique_ptr<Program> prog_single[FAM_COUNT];   // the same families built with one edge stream per CTA
     bool streams_off = false;                           // a multi-stream kernel came out with the wrong register count
 };
@@ -1430,12 +1455,16 @@ struct TcParams {
     long long batch;
     int accum;
     int* status;
+    int splits;
+    int cut[9];
+    void* parts; int* count;
 };
 struct TcDwParams {
     const void* x; const void* y; const void* g; void* part;
     long long batch;
-    int grp_begin, grp_end;
     int* status;
+    int splits;
+    int cut[9];
 };
 // sizeof(TcShared) in kernels/uvw_tc.cuh, rounded up: operand buffers + staged block + harmonics (+ the dy partials);
 // mode as in emit_tc
@@ -1466,6 +1495,87 @@ size_t tc_smem_base_bytes(const Desc& d, int mode) {   // without the second sta
     return 4 * (2 * 2 * 4096 + 2 * 2 * 1024 + xs + ys + dys) + 256;
 }
 
+void tc_cut(TcCuts& c) {
+    const int G = (int)c.cost.size();
+    double total = 0, big = 0;
+    for (double v : c.cost) { total += v; big = std::max(big, v); }
+    for (int S = 1; S <= 8; ++S) {
+        double lo = big, hi = total + 1;
+        auto fill = [&](double cap, bool keep) {
+            int parts = 0;
+            for (int g = 0; g < G;) {
+                if (parts == S) return false;
+                double sum = 0;
+                if (keep) c.cut[S][parts] = c.begin[g];
+                do sum += c.cost[g++]; while (g < G && sum + c.cost[g] <= cap);
+                if (keep) { c.part[S][parts] = sum; c.cut[S][parts + 1] = c.begin[g]; }
+                ++parts;
+            }
+            if (keep) c.n[S] = parts;
+            return true;
+        };
+        for (int it = 0; it < 24; ++it) (fill((lo + hi) / 2, false) ? hi : lo) = (lo + hi) / 2;
+        fill(hi, true);
+    }
+}
+TcCuts& tc_cuts(Entry* e, int mode) {
+    std::unique_ptr<TcCuts>& slot = e->tc_cuts[mode];
+    if (slot) return *slot;
+    slot = std::make_unique<TcCuts>();
+    const Desc& d = e->d;
+    const std::vector<TcSub> subs = tc_subpaths(d);
+    if (mode == 3) {
+        const auto groups = tc_dw_groups(d, nullptr);
+        for (size_t g = 0; g < groups.size(); ++g) {
+            slot->begin.push_back((int)g);
+            slot->cost.push_back(2.0 * d.L[2][d.ins[subs[groups[g][0]].ins].o].d() + 1);   // + 1: staging
+        }
+        slot->begin.push_back((int)groups.size());
+    } else {
+        std::vector<int> first, last;
+        const std::vector<int> order = tc_schedule(d, mode, &first, &last);
+        for (size_t q = 0; q < order.size(); ++q) {
+            const Instr& I = d.ins[subs[order[q]].ins];
+            if (first[order[q]]) { slot->begin.push_back((int)q); slot->cost.push_back(1.0); }   // the epilogue
+            slot->cost.back() += d.L[mode == 1 ? 0 : 2][mode == 1 ? I.a : I.o].d() + 0.5;
+        }
+        slot->begin.push_back((int)order.size());
+    }
+    tc_cut(*slot);
+    return *slot;
+}
+// Parts for `tiles` tiles: the number whose busiest CTA has least to do when units are dealt out in turn.  Beside its paths a unit costs
+// harmonics, a first block that nobody requested ahead and a drained pipeline: about eight steps (four parts of 391 tiles measured
+// 470 us against 451 us in one), two for dW, which drains after every tile anyway; mode 2 clears counters and sums the parts.  30 paths
+// of 32 x 32, second order of 2,500 items (20 tiles on 148 SMs): 619 / 455 / 585 / 314 us (forward, dx, dy, dW) in one part, 222 / 164 /
+// 151 / 127 us in parts.
+int tc_splits(Entry* e, int mode, long long tiles) {
+    TcCuts& c = tc_cuts(e, mode);
+    if (c.seen_tiles == tiles) return c.seen_splits;
+    const int sms = sm_count();
+    int best = 1;
+    double best_time = 0;
+    std::vector<double> load;
+    for (int S = 1; S <= 8; ++S) {
+        const int n = c.n[S];
+        if (S > 1 && (n < S || tiles >= 16LL * sms)) break;   // too few groups, or so many tiles that the last wave hardly counts
+        load.assign(sms, 0.0);
+        for (long long u = 0; u < std::min<long long>(tiles, 16LL * sms) * n; ++u) load[u % sms] += c.part[S][u % n] + (mode == 3 ? 2.0 : 8.0);
+        const double t = *std::max_element(load.begin(), load.end()) + (mode == 2 && n > 1 ? 4.0 : 0.0);
+        if (S == 1 || t < 0.95 * best_time) { best = S; best_time = t; }
+    }
+    c.seen_tiles = tiles;
+    c.seen_splits = best;
+    return best;
+}
+unsigned tc_set_cut(Entry* e, int mode, long long tiles, int* splits, int* cut) {   // returns the grid
+    const int S = tc_splits(e, mode, tiles);
+    const TcCuts& c = tc_cuts(e, mode);
+    *splits = c.n[S];
+    for (int i = 0; i <= c.n[S]; ++i) cut[i] = c.cut[S][i];
+    return (unsigned)std::min<long long>(sm_count(), tiles * c.n[S]);
+}
+
 // mode 0: z from (x, y, W); mode 1: the gradient of x from (g, y, W), passed in the places of x and z; mode 2: the
 // gradient of y (in the place of z) from (x, W, g)
 int tc_forward(Entry* e, TcParams p, cudaStream_t st, int mode = 0) {
@@ -1479,10 +1589,21 @@ int tc_forward(Entry* e, TcParams p, cudaStream_t st, int mode = 0) {
     cudaKernel_t k;
     const size_t smem = e->d.tc_smem[mode];
     if ((rc = get_kernel(prog, names[mode], smem, &k))) return rc;
-    long long tiles = (p.batch + 127) / 128, grid = sm_count();
-    if (grid > tiles) grid = tiles;
+    const unsigned grid = tc_set_cut(e, mode, (p.batch + 127) / 128, &p.splits, p.cut);
+    void* scratch = nullptr;
+    if (mode == 2 && p.splits > 1) {   // the parts' sums of dy: rows of scratch, added in order by a tile's last part (counters)
+        const size_t rows = round_up((size_t)p.splits * p.batch * e->d.dim[1] * sizeof(float)), counts = (size_t)(p.batch + 127) / 128 * 4;
+        if ((rc = keep_pool_memory())) return rc;
+        CUDA_TRY(cudaMallocAsync(&scratch, rows + counts, st));
+        p.parts = scratch;
+        p.count = (int*)((char*)scratch + rows);
+        cudaError_t ce = cudaMemsetAsync(p.count, 0, counts, st);
+        if (ce != cudaSuccess) { cudaFreeAsync(scratch, st); return fail(OEQB_ECUDA, "cudaMemsetAsync: %s", cudaGetErrorString(ce)); }
+    }
     void* args[] = {&p};
-    return launch(k, (unsigned)grid, 16 * 32 + 32, smem, args, st);   // TC_THREADS: sixteen compute warps + the issuing warp
+    rc = launch(k, grid, 16 * 32 + 32, smem, args, st);   // TC_THREADS: sixteen compute warps + the issuing warp
+    if (scratch) cudaFreeAsync(scratch, st);
+    return rc;
 }
 
 // Keep freed stream-ordered scratch in the device's pool: by default the pool gives memory back to the driver at every
@@ -1506,7 +1627,7 @@ int keep_pool_memory() {
 int tc_backward_dw(Entry* e, const void* x, const void* y, const void* g, void* dW, long long batch, int accum, cudaStream_t st) {
     int rc;
     const Desc& d = e->d;
-    TcDwParams p{x, y, g, nullptr, batch, 0, 0, nullptr};
+    TcDwParams p{x, y, g, nullptr, batch, nullptr};
     if ((rc = status_word(&p.status))) return rc;
     Program *prog, *gen;
     if ((rc = get_program(e, FAM_UVW_TC_DW, &prog))) return rc;
@@ -1515,20 +1636,20 @@ int tc_backward_dw(Entry* e, const void* x, const void* y, const void* g, void* 
     const size_t smem = d.tc_dw_smem;
     if ((rc = get_kernel(prog, "oeq_uvw_tc_backward_dw", smem, &k))) return rc;
     if ((rc = get_kernel(gen, "oeq_generic_dw_reduce", 0, &kr))) return rc;
-    long long tiles = (batch + 63) / 64, grid = sm_count();
-    if (grid > tiles) grid = tiles;
+    long long tiles = (batch + 63) / 64;
     if ((rc = keep_pool_memory())) return rc;
     void* part = nullptr;
     CUDA_TRY(cudaMallocAsync(&part, (size_t)tiles * d.wn * sizeof(float), st));   // one row per tile of 64 items
     p.part = part;
-    // the accumulators of 16 groups fill the tensor memory: more groups take more launches (each writes its groups' part
-    // of every tile's row)
-    const int ngrp = d.tc_ngrp;
-    for (int g0 = 0; g0 < ngrp && !rc; g0 += 16) {
-        p.grp_begin = g0;
-        p.grp_end = std::min(ngrp, g0 + 16);
-        void* args[] = {&p};
-        rc = launch(k, (unsigned)grid, 16 * 32 + 32, smem, args, st);   // TC_THREADS
+    void* args[] = {&p};
+    // the accumulators of 16 groups fill the tensor memory: more groups take more launches (each writes its groups' part of every
+    // tile's row)
+    unsigned grid = (unsigned)std::min<long long>(sm_count(), tiles);
+    p.splits = 1;
+    if (d.tc_ngrp <= 16) grid = tc_set_cut(e, 3, tiles, &p.splits, p.cut);
+    for (int g0 = 0; g0 < d.tc_ngrp && !rc; g0 += 16) {
+        if (d.tc_ngrp > 16) { p.cut[0] = g0; p.cut[1] = std::min(d.tc_ngrp, g0 + 16); }
+        rc = launch(k, grid, 16 * 32 + 32, smem, args, st);   // TC_THREADS
     }
     if (!rc) {
         void* rargs[] = {&part, &tiles, &dW, &accum};

@@ -1,0 +1,13 @@
+"""Tensor-core 'uvw' kernels where a tile's schedule is dealt to several CTAs: batches around one tile (64 / 128 items), few
+tiles (every cut of the schedule), one tile more than there are SMs (a ragged last wave), against the fp64 oracle."""
+import pytest
+
+from test_uvw_f64_gpu import orders_0_to_2, shared_problem
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("batch", [1, 64, 65, 129, 1000, 2500, 128 * 148 + 1])
+def test_cut_schedules(batch, wide):
+    orders_0_to_2(shared_problem(wide), batch)
