@@ -202,14 +202,17 @@ OEQ_DEV void tc_cg(const float* xrow, const float* yrow, int t0, int t1, float (
 // problem header (not unrolled): the whole kernel is a few KB of code and stays in the instruction cache.
 // The same kernel computes the gradient of the first input when it is compiled with the transposed tables (TC_WT = 1:
 // x is then the output cotangent, z the gradient, and the weight block is applied transposed), and the gradient of the
-// second input (mode 2); TC_KERNEL_NAME, TC_IN_DIM and TC_OUT_DIM (row lengths of x and z) come with the tables.
+// second input (mode 2); TC_KERNEL_NAME, TC_PARTS_NAME, TC_IN_DIM and TC_OUT_DIM (row lengths of x and z) come with the tables.
 //
 // Sixteen compute warps and one warp that issues the MMAs.  The compute warps never meet the issuing warp at a CTA-wide
 // barrier: a step's operands are handed over through the a_full mbarrier (every compute thread arrives after its
 // stores), buffers come back through mma_done, finished accumulators through acc_done (tcgen05.commit).  The compute
 // warps meet among themselves (named barrier) only where the staged input block changes hands.  A thread that gave up
 // keeps walking the loops and joining those barriers without doing work, so nobody waits for it.
-extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const __grid_constant__ TcParams p) {
+//
+// PARTS: the schedule is cut (p.splits > 1).  The uncut kernel is compiled by itself: with the cuts in registers its spills cost 8 %.
+template <bool PARTS>
+OEQ_DEV void tc_kernel(const TcParams& p) {
     extern __shared__ __align__(128) unsigned char tc_smem_raw[];
     TcShared& sh = *reinterpret_cast<TcShared*>(tc_smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -232,7 +235,8 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const
     const unsigned tmem = sh.tmem_base;
     // A unit of work is a tile and a part of the schedule, cut where a destination block ends.  One part needs the least staging;
     // more parts fill the chip when there are few tiles, or a last wave that would be nearly empty (the host counts).
-    const long long nunits = (p.batch + 127) / 128 * p.splits;
+    const int splits = PARTS ? p.splits : 1;
+    const long long nunits = (p.batch + 127) / 128 * splits;
     unsigned step = 0;     // chunk steps so far: operand buffer = step & 1
     unsigned npath = 0;    // paths started so far: weight buffer = npath & 1
     unsigned nblock = 0;   // output blocks finished so far: accumulator half = nblock & 1
@@ -246,8 +250,8 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const
         const unsigned long long db0h = tc_desc(&sh.b[0][0][0], TC_LBO, TC_SBO), db0l = tc_desc(&sh.b[0][1][0], TC_LBO, TC_SBO);
         const unsigned long long db1h = tc_desc(&sh.b[1][0][0], TC_LBO, TC_SBO), db1l = tc_desc(&sh.b[1][1][0], TC_LBO, TC_SBO);
         for (long long unit = blockIdx.x; unit < nunits && !dead; unit += gridDim.x) {
-            const int part = (int)(unit % p.splits), q1 = p.cut[part + 1];
-            for (int q = p.cut[part]; q < q1 && !dead; ++q) {
+            const int part = PARTS ? (int)(unit % splits) : 0, q1 = PARTS ? p.cut[part + 1] : TC_NPATH;
+            for (int q = PARTS ? p.cut[part] : 0; q < q1 && !dead; ++q) {
                 const int d3 = TC_D3[q], first = TC_FIRST[q], last = TC_LAST[q];
                 for (int k = 0; k < d3 && !dead; ++k) {
                     const unsigned buf = step & 1u;
@@ -285,11 +289,11 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const
         float gnext[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // mode 2: the next step's cotangent values
         float wnext[1024 / TC_CT];                                    // this thread's entries of the next path's weight block
 #pragma unroll
-        for (int r = 0; r < 1024 / TC_CT; ++r) wnext[r] = __ldg(p.W + TC_WOFF[p.cut[blockIdx.x % p.splits]] + tid + TC_CT * r);
+        for (int r = 0; r < 1024 / TC_CT; ++r) wnext[r] = __ldg(p.W + TC_WOFF[PARTS ? p.cut[blockIdx.x % splits] : 0] + tid + TC_CT * r);
         for (long long unit = blockIdx.x; unit < nunits; unit += gridDim.x) {
-            const int part_s = (int)(unit % p.splits), q0 = p.cut[part_s], q1 = p.cut[part_s + 1];
-            const int qnext = p.cut[(unit + gridDim.x) % p.splits];   // first path of this CTA's next unit
-            const long long item0 = unit / p.splits * 128;
+            const int part_s = PARTS ? (int)(unit % splits) : 0, q0 = PARTS ? p.cut[part_s] : 0, q1 = PARTS ? p.cut[part_s + 1] : TC_NPATH;
+            const int qnext = PARTS ? p.cut[(unit + gridDim.x) % splits] : 0;   // first path of this CTA's next unit
+            const long long item0 = unit / splits * 128;
             int pre_q = -1;      // path whose block has been requested ahead (none across tiles)
             tc_compute_sync();   // previous tile's readers of xs / ys / dys are done
             if (TC_MODE != 2) {
@@ -327,7 +331,7 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const
                         if (!tc_mbar_wait(&sh.xs_full[cur], nfill[cur] & 1u, abortf, p.status, 37)) dead = true;
                         ++nfill[cur];
                         const int qn = TC_NEXTX[q];   // first later path of the schedule that stages another block, or -1
-                        if (!dead && qn >= 0 && qn < q1 && TC_D1[qn] <= (cur ? TC_MAXD1 : TC_XS2_D1)) { request(cur ^ 1, qn); pre_q = qn; }
+                        if (!dead && qn >= 0 && (!PARTS || qn < q1) && TC_D1[qn] <= (cur ? TC_MAXD1 : TC_XS2_D1)) { request(cur ^ 1, qn); pre_q = qn; }
                     }
                 } else {
                     if (restage && !dead) {   // warp w copies rows w, w + 16, ... (odd row stride: 4-byte pieces)
@@ -457,8 +461,8 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const
                 const long long b = item0 + tid;
                 const bool live = tid < 128 && b < p.batch && !sh.abort_flag;
                 if (live) {
-                    float* out = p.splits > 1 ? p.parts + (part_s * p.batch + b) * L2_DIM : p.z + b * L2_DIM;
-                    const bool add = p.splits == 1 && p.accum;
+                    float* out = PARTS ? p.parts + (part_s * p.batch + b) * L2_DIM : p.z + b * L2_DIM;
+                    const bool add = !PARTS && p.accum;
                     for (int j = 0; j < L2_DIM; ++j) {
                         float v = 0.f;
 #pragma unroll
@@ -466,17 +470,17 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const
                         out[j] = add ? out[j] + v : v;
                     }
                 }
-                if (p.splits > 1) {
+                if (PARTS) {
                     // the part that finishes a tile last adds the parts' rows in the order of the schedule
                     __threadfence();
                     tc_compute_sync();
-                    if (tid == 0) sh.last_part = atomicAdd(p.count + unit / p.splits, 1) == p.splits - 1;
+                    if (tid == 0) sh.last_part = atomicAdd(p.count + unit / splits, 1) == splits - 1;
                     tc_compute_sync();
                     if (live && sh.last_part) {
                         __threadfence();
                         for (int j = 0; j < L2_DIM; ++j) {
                             float v = p.accum ? p.z[b * L2_DIM + j] : 0.f;
-                            for (int s = 0; s < p.splits; ++s) v += __ldcg(p.parts + (s * p.batch + b) * L2_DIM + j);
+                            for (int s = 0; s < splits; ++s) v += __ldcg(p.parts + (s * p.batch + b) * L2_DIM + j);
                             p.z[b * L2_DIM + j] = v;
                         }
                     }
@@ -488,6 +492,8 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
+extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const TcParams p) { tc_kernel<false>(p); }
+extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_PARTS_NAME(const __grid_constant__ TcParams p) { tc_kernel<true>(p); }
 #endif  // TC_MODE != 3
 
 #if TC_MODE == 3

@@ -694,7 +694,8 @@ std::string emit_tc(const Desc& d, int mode = 0) {
     const bool dx = mode == 1, dy = mode == 2;
     s << "#define TC_MODE " << mode << "\n";
     s << "#define TC_WT " << (mode != 0 ? 1 : 0) << "\n";
-    s << "#define TC_KERNEL_NAME " << (dx ? "oeq_uvw_tc_backward_dx" : dy ? "oeq_uvw_tc_backward_dy" : "oeq_uvw_tc_forward") << "\n";
+    const std::string name = dx ? "oeq_uvw_tc_backward_dx" : dy ? "oeq_uvw_tc_backward_dy" : "oeq_uvw_tc_forward";
+    s << "#define TC_KERNEL_NAME " << name << "\n#define TC_PARTS_NAME " << name << "_parts\n";
     s << "constexpr int TC_IN_DIM = " << (dx ? d.dim[2] : d.dim[0]) << ", TC_OUT_DIM = " << (dx ? d.dim[0] : d.dim[2]) << ";\n";
     std::vector<int> first, last;
     const std::vector<TcSub> subs = tc_subpaths(d);
@@ -1579,7 +1580,9 @@ unsigned tc_set_cut(Entry* e, int mode, long long tiles, int* splits, int* cut) 
 // mode 0: z from (x, y, W); mode 1: the gradient of x from (g, y, W), passed in the places of x and z; mode 2: the
 // gradient of y (in the place of z) from (x, W, g)
 int tc_forward(Entry* e, TcParams p, cudaStream_t st, int mode = 0) {
-    static const char* names[3] = {"oeq_uvw_tc_forward", "oeq_uvw_tc_backward_dx", "oeq_uvw_tc_backward_dy"};
+    static const char* names[3][2] = {{"oeq_uvw_tc_forward", "oeq_uvw_tc_forward_parts"},
+                                      {"oeq_uvw_tc_backward_dx", "oeq_uvw_tc_backward_dx_parts"},
+                                      {"oeq_uvw_tc_backward_dy", "oeq_uvw_tc_backward_dy_parts"}};
     int rc;
     if (!p.accum && ((mode == 0 && e->d.tc_zero_z) || (mode == 1 && e->d.tc_zero_dx)))
         CUDA_TRY(cudaMemsetAsync(p.z, 0, (size_t)p.batch * e->d.dim[mode == 0 ? 2 : 0] * sizeof(float), st));
@@ -1588,8 +1591,8 @@ int tc_forward(Entry* e, TcParams p, cudaStream_t st, int mode = 0) {
     if ((rc = get_program(e, mode == 0 ? FAM_UVW_TC : FAM_UVW_TC_DX + (mode - 1), &prog))) return rc;
     cudaKernel_t k;
     const size_t smem = e->d.tc_smem[mode];
-    if ((rc = get_kernel(prog, names[mode], smem, &k))) return rc;
     const unsigned grid = tc_set_cut(e, mode, (p.batch + 127) / 128, &p.splits, p.cut);
+    if ((rc = get_kernel(prog, names[mode][p.splits > 1], smem, &k))) return rc;
     void* scratch = nullptr;
     if (mode == 2 && p.splits > 1) {   // the parts' sums of dy: rows of scratch, added in order by a tile's last part (counters)
         const size_t rows = round_up((size_t)p.splits * p.batch * e->d.dim[1] * sizeof(float)), counts = (size_t)(p.batch + 127) / 128 * 4;
