@@ -12,8 +12,8 @@
 // the cotangent (or the sum) of those columns stays in registers and the sum over w is log2(PP) shuffles per row of VEC * P.
 // All sums run in an order fixed by the problem: bitwise reproducible.
 //
-// DiffDock L = 2 (multiplicities 10 and 48, 7,128 weights), 8,191 items: forward 65 us (3.8 TB/s of rows), backward 147 us (3.4 TB/s;
-// 195 us with five blocks of 127 registers to an SM instead of eight of 64); the general kernels (a warp per item, strided stores of
+// DiffDock L = 2 (multiplicities 10 and 48, 7,128 weights), 8,191 items: forward 65 us (3.8 TB/s of rows), backward 122 us (4.1 TB/s;
+// 195 us with five blocks of 127 registers to an SM instead of eight of 64 and no staged row); the general kernels (a warp per item, strided stores of
 // dW, a shuffle per product) took 733 us for both.
 #pragma once
 
@@ -64,6 +64,24 @@ OEQ_DEV void item_rows(int warp, int lane, F&& f) {
             f(on ? 32 * UC + ul : -1, on ? BASE + ul * C::WLEN + c * C::VEC : 0);
         }
     });
+}
+
+// The item's weight row, requested whole by asynchronous copies before anything else is read (ITEM_STAGE_W, emitted: rows that
+// leave room for several blocks in an SM's shared memory); longer rows are read from global memory where they are used.  The backward
+// gained (147 -> 122 us, DiffDock L = 2, 8,191 items); the forward, whose loads are already far ahead of their use, lost (65 -> 72 us) and
+// reads global memory.
+OEQ_DEV void item_request(const T* src, T* dst) {
+#if ITEM_STAGE_W
+    constexpr int BYTES = ITEM_VEC * (int)sizeof(T);
+    const unsigned to = (unsigned)__cvta_generic_to_shared(dst);
+    for (int i = threadIdx.x; i < WN / ITEM_VEC; i += ITEM_WARPS * 32)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(to + i * BYTES), "l"(src + (long long)i * ITEM_VEC), "n"(BYTES) : "memory");
+#endif
+}
+OEQ_DEV void item_arrived() {
+#if ITEM_STAGE_W
+    asm volatile("cp.async.wait_all;" ::: "memory");
+#endif
 }
 
 OEQ_DEV void item_stage(const T* __restrict__ src, T* dst, int n) {
@@ -163,16 +181,19 @@ struct ItemBwdParams {
 
 extern "C" __global__ void __launch_bounds__(ITEM_WARPS * 32, sizeof(T) == 4 ? 8 : 4) oeq_uvw_item_backward(const ItemBwdParams p) {
     __shared__ T xs[L1_DIM], y1[L2_DIM], y2[L2_DIM], gs[L3_DIM], ts[ItemOff<NINS>::T0], gp[ItemOff<NINS>::G0], dys[ITEM_WARPS][L2_DIM];
+    extern __shared__ __align__(16) unsigned char item_row[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (long long b = blockIdx.x; b < p.items; b += gridDim.x) {
+        item_request(p.W + b * WN, (T*)item_row);
         item_stage(p.x + b * L1_DIM, xs, L1_DIM);
         item_stage(p.y_dx + b * L2_DIM, y1, L2_DIM);
         item_stage(p.y_dw + b * L2_DIM, y2, L2_DIM);
         item_stage(p.g + b * L3_DIM, gs, L3_DIM);
         __syncthreads();
         item_cg(xs, y2, ts, warp, lane);
+        item_arrived();
         __syncthreads();
-        const T* __restrict__ wrow = p.W + b * WN;
+        const T* __restrict__ wrow = ITEM_STAGE_W ? (const T*)item_row : p.W + b * WN;
         T* __restrict__ dwrow = p.dW + b * WN;
         static_for<0, NB3>([&](auto oc) {
             constexpr int O = decltype(oc)::value;
@@ -275,6 +296,6 @@ extern "C" __global__ void __launch_bounds__(ITEM_WARPS * 32, sizeof(T) == 4 ? 8
             T* out = p.dy + b * L2_DIM + j;
             *out = p.add ? *out + s : s;
         }
-        // the next item overwrites the operands, last read before the barrier above; dys only after three more barriers
+        // the next item overwrites the row and the operands, last read before the barrier above; dys only after three more barriers
     }
 }

@@ -850,13 +850,19 @@ int item_vec(const Desc& d) {
     return v;
 }
 
+// Shared memory for an item's weight row: rows up to 40 KB leave room for four blocks or more in an SM; 0: not staged.
+size_t item_row_bytes(const Desc& d) {
+    const size_t b = (size_t)d.wn * d.elt();
+    return b <= 40 * 1024 ? b : 0;
+}
+
 std::string family_source(const Desc& d, const std::string& header, int fam, bool allow_streams = true) {
     std::string src = header;
     if (fam == FAM_GENERIC) {
         src += K_COMMON;
         src += K_GENERIC;
     } else if (fam == FAM_UVW_ITEM) {
-        src += "constexpr int ITEM_VEC = " + std::to_string(item_vec(d)) + ";\n";
+        src += "constexpr int ITEM_VEC = " + std::to_string(item_vec(d)) + ";\n#define ITEM_STAGE_W " + (item_row_bytes(d) ? "1\n" : "0\n");
         src += K_COMMON;
         src += K_UVW_ITEM;
     } else if (fam == FAM_UVW_F64) {
@@ -1194,22 +1200,23 @@ struct ItemBwdParams {
     long long items;
     int add;
 };
-int item_launch(Entry* e, const char* name, void* params, long long items, cudaStream_t st) {
+int item_launch(Entry* e, const char* name, size_t row, void* params, long long items, cudaStream_t st) {
     Program* prog;
     if (int rc = get_program(e, FAM_UVW_ITEM, &prog)) return rc;
     cudaKernel_t k;
-    if (int rc = get_kernel(prog, name, 0, &k)) return rc;
+    // (the kernels' static arrays and the row together may exceed 48 KB: the attribute is then needed whatever the row alone takes)
+    if (int rc = get_kernel(prog, name, row ? std::max<size_t>(row, 48 * 1024 + 16) : 0, &k)) return rc;
     void* args[] = {params};
-    return launch(k, (unsigned)std::min<long long>(items, 1 << 30), 128, 0, args, st);
+    return launch(k, (unsigned)std::min<long long>(items, 1 << 30), 128, row, args, st);
 }
 int item_forward(Entry* e, const void* x, const void* y, const void* W, void* z, long long items, int add, cudaStream_t st) {
     ItemFwdParams p{x, y, W, z, items, add};
-    return item_launch(e, "oeq_uvw_item_forward", &p, items, st);
+    return item_launch(e, "oeq_uvw_item_forward", 0, &p, items, st);
 }
 int item_backward(Entry* e, const void* x, const void* y_dx, const void* y_dw, const void* W, const void* g, void* dx, void* dy,
                   void* dW, long long items, int add, cudaStream_t st) {
     ItemBwdParams p{x, y_dx, y_dw, W, g, dx, dy, dW, items, add};
-    return item_launch(e, "oeq_uvw_item_backward", &p, items, st);
+    return item_launch(e, "oeq_uvw_item_backward", item_row_bytes(e->d), &p, items, st);
 }
 
 // ------------------------------------------------------------------------------- 'uvw' in doubles, shared weights
