@@ -139,7 +139,7 @@ __global__ void rank_segments(const long long* __restrict__ ptr, const long long
 }
 
 // The same grouping as one block, for lists that fit its shared memory: keys counted, scanned, scattered and ranked there.
-// Small lists are nothing but launches: 1,680 edges over 105 nodes took 24 us of device time in six kernels and a clear, and
+// Small lists are nothing but launches: 1,680 edges over 105 nodes took 12 us of device time in six kernels and a clear, and
 // their launches as much again on the host; one block needs 4.8 us.  Up to the limits of its shared memory one SM is faster.
 constexpr int SMALL_EDGES = 8192, SMALL_KEYS = 4096;
 template <typename IDX>
