@@ -4,8 +4,8 @@ grouped product kernels.
 Counterpart of openequivariance/openequivariance/_torch/symmetric_contraction/symmetric_contraction.py:
 
 The work is done by ``oeq_b200::symmetric_contraction`` (csrc/sym_contraction.cuh): one pass over the nodes per direction,
-whose kernels are specialised for the monomials that the tensors ``U`` touch (``_Plan``).  Second and higher orders, tensors of
-order above three and installations without the C++ operators take the composed form below.
+whose kernels are specialised for the monomials that the tensors ``U`` touch (``_Plan``).  Gradients that are differentiated
+again, tensors of order above three and installations without the C++ operators take the composed form below.
 
 * ``GroupMM`` (reference :7-108) -- the ragged grouped product as a torch custom op with autograd; the work is done by
   ``oeqb_group_mm`` (one kernel launch per call) instead of one cuBLAS strided-batched GEMM per chemical element.
@@ -229,7 +229,7 @@ class _Plan:
         meta = [num_elements, num_features, ell, n_out, len(sets), self.out_dim, T, *struct.unpack("<ii", key)]
         for pair in list(zip(columns, sets)) + list(zip(out_col, out_stride)):
             meta += pair
-        # (the number of orders of every irrep comes last: only the composed second order reads it)
+        # (the number of orders of every irrep comes last: only the gradients that are differentiated again read it)
         self.meta = torch.tensor(meta + self.groups + [len(self.groups)], dtype=torch.int32)
 
     def holds_for(self, U_groups):
@@ -270,30 +270,12 @@ if ops.CPP_OPS:
     def _(grad, x, keys, group, coef, weights, U, terms, place, U_rows, meta):
         return torch.empty_like(x), [torch.empty_like(w) for w in weights]
 
-    def _second_setup(ctx, inputs, output):
-        ctx.grad, ctx.x, ctx.keys, _, _, ctx.weights, ctx.U, _, _, _, ctx.meta = inputs
-
-    def _second_backward(ctx, t_dx, t_dw):
-        # the composed form's first-order gradients, differentiated again
-        keep = torch.is_grad_enabled()
-        groups = ctx.meta[-1 - int(ctx.meta[-1]):-1].tolist()
-        with torch.enable_grad():
-            leaves = [t.detach().requires_grad_(True) for t in (ctx.grad, ctx.x, *ctx.weights)]
-            g_, x_, w_ = leaves[0], leaves[1], leaves[2:]
-            out = _composed_unsorted(groups, w_, ctx.U, x_, ctx.keys, int(ctx.meta[0]))
-            first = torch.autograd.grad(out, [x_] + w_, g_, create_graph=True, allow_unused=True)
-            total = None
-            for f, t in zip(first, [t_dx] + list(t_dw if t_dw is not None else [None] * len(w_))):
-                if f is not None and t is not None:
-                    term = (f * t).sum()
-                    total = term if total is None else total + term
-            if total is None or not total.requires_grad:
-                grads = [None] * len(leaves)
-            else:
-                grads = torch.autograd.grad(total, leaves, create_graph=keep, allow_unused=True)
-        return grads[0], grads[1], None, None, None, list(grads[2:]), [None] * len(ctx.U), None, None, None, None
-
-    torch.library.register_autograd("oeq_b200::symmetric_contraction_backward", _second_backward, setup_context=_second_setup)
+    # what the C++ autograd node differentiates where its gradients are differentiated again
+    _lib = torch.library.Library("oeq_b200", "FRAGMENT")
+    _lib.define("symmetric_contraction_composed(Tensor x, Tensor keys, Tensor[] weights, Tensor[] U, int[] orders, int num_elements) -> Tensor")
+    _lib.impl("symmetric_contraction_composed",
+              lambda x, keys, weights, U, orders, num_elements: _composed_unsorted(orders, weights, U, x, keys, num_elements),
+              "CompositeImplicitAutograd")
 
 
 class Contraction(torch.nn.Module):

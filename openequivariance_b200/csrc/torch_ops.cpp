@@ -15,6 +15,7 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/autograd.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/library.h>
 
@@ -425,7 +426,7 @@ Three autograd_conv_backward(const at::Tensor& json, int64_t hash, const at::Ten
 // ---- symmetric contraction ---------------------------------------------------------------------------------------
 // `terms`, `meta` (CPU), `place` and `U_rows` describe the contraction's tensors U (made by _torch/symmetric_contraction.py);
 // `keys` holds the element of each node; `weights` one tensor [elements, columns, channels] per (irrep, order).  The dense
-// tensors `U` are only used by the second order, which Python composes.  Besides the result the forward returns what the
+// tensors `U` are only used by gradients that are differentiated again, which Python composes.  Besides the result the forward returns what the
 // backward takes again: the nodes by element and the polynomials' coefficients.
 int symcon_dtype(const at::Tensor& x) {
     if (x.scalar_type() == at::kFloat) return 1;
@@ -509,6 +510,32 @@ const c10::TypedOperatorHandle<SymBwdSig>& sym_bwd_op() {
     return op;
 }
 
+typedef at::Tensor SymComposedSig(const at::Tensor&, const at::Tensor&, at::TensorList, at::TensorList, c10::IntArrayRef, int64_t);
+const c10::TypedOperatorHandle<SymComposedSig>& sym_composed_op() {
+    static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("oeq_b200::symmetric_contraction_composed", "").typed<SymComposedSig>();
+    return op;
+}
+
+// Gradients (of x, then of the weights; undefined where none is needed) that may be differentiated again: those of the composed
+// form, whose recorded graph the next order continues.  It is formed on aliases of the operands: the graph stays connected to
+// them, so every order is right, and a gradient ends at the operand it is for even where one operand was made from another.
+variable_list symcon_composed_gradients(const at::Tensor& cot, const variable_list& operands, const at::Tensor& keys, at::TensorList U,
+                                        const at::Tensor& meta) {
+    variable_list alias, wanted, found(operands.size());
+    for (const at::Tensor& t : operands) {
+        alias.push_back(t.view_as(t));
+        if (t.requires_grad()) wanted.push_back(alias.back());
+    }
+    const int32_t* end = meta.data_ptr<int32_t>() + meta.numel() - 1;   // orders of every irrep, then their number
+    const std::vector<int64_t> orders(end - *end, end);
+    const std::vector<at::Tensor> weights(alias.begin() + 1, alias.end());
+    const at::Tensor out = sym_composed_op().call(alias[0], keys, weights, U, orders, meta.data_ptr<int32_t>()[0]);
+    const variable_list got = torch::autograd::grad({out}, wanted, {cot}, c10::nullopt, true, true);
+    for (size_t i = 0, j = 0; i < alias.size(); ++i)
+        if (alias[i].requires_grad()) found[i] = got[j++];
+    return found;
+}
+
 struct SymForward : torch::autograd::Function<SymForward> {
     static variable_list forward(AutogradContext* ctx, const at::Tensor& x, const at::Tensor& keys, at::TensorList weights, at::TensorList U,
                                  const at::Tensor& terms, const at::Tensor& place, const at::Tensor& U_rows, const at::Tensor& meta,
@@ -526,11 +553,18 @@ struct SymForward : torch::autograd::Function<SymForward> {
     }
     static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
         const variable_list v = ctx->get_saved_variables();
-        const std::vector<at::Tensor> weights(v.begin() + 1, v.end()), U = ctx->saved_data["U"].toTensorVector();
-        const std::vector<at::Tensor> fixed = ctx->saved_data["fixed"].toTensorVector();
-        auto [dx, dw] = sym_bwd_op().call(grads[0], v[0], fixed[0], fixed[1], fixed[2], weights, U, fixed[3], fixed[4], fixed[5], fixed[6]);
-        variable_list out{dx, at::Tensor()};
-        out.insert(out.end(), dw.begin(), dw.end());
+        const std::vector<at::Tensor> U = ctx->saved_data["U"].toTensorVector(), fixed = ctx->saved_data["fixed"].toTensorVector();
+        variable_list out(v.size() + 1);
+        if (grads[0].defined() && at::GradMode::is_enabled()) {
+            const variable_list d = symcon_composed_gradients(grads[0], v, fixed[0], U, fixed[6]);
+            out[0] = d[0];
+            std::copy(d.begin() + 1, d.end(), out.begin() + 2);
+        } else if (grads[0].defined()) {
+            const std::vector<at::Tensor> weights(v.begin() + 1, v.end());
+            auto [dx, dw] = sym_bwd_op().call(grads[0], v[0], fixed[0], fixed[1], fixed[2], weights, U, fixed[3], fixed[4], fixed[5], fixed[6]);
+            out[0] = dx;
+            std::copy(dw.begin(), dw.end(), out.begin() + 2);
+        }
         out.resize(out.size() + U.size() + 5);   // U, terms, place, U_rows, meta, out_dim
         return out;
     }
