@@ -186,8 +186,10 @@ class _Plan:
         device, dtype, ell = first.device, first.dtype, first.shape[-2]
         factors, starts, number = _monomials(ell, device)
         self.groups = [len(g) for g in U_groups]
+        self.shapes = _shapes(U_groups)
+        # what the terms are made from: every call compares its tensors with this copy (csrc/sym_contraction.cuh, compare)
+        U_groups = [[U.detach().clone(memory_format=torch.contiguous_format) for U in g] for g in U_groups]
         self.U = [U for g in U_groups for U in g]
-        self.versions = [_version(U) for U in self.U]
         comp, mono, sets, rows, columns, out_col, out_stride, base = [], [], [], [], [], [], [], 0
         for g in U_groups:
             leading = g[0].dim() == len(g) + 2
@@ -232,13 +234,9 @@ class _Plan:
         # (the number of orders of every irrep comes last: only the gradients that are differentiated again read it)
         self.meta = torch.tensor(meta + self.groups + [len(self.groups)], dtype=torch.int32)
 
-    def holds_for(self, U_groups):
-        flat = [U for g in U_groups for U in g]
-        return len(flat) == len(self.U) and all(a is b and v == _version(b) for a, b, v in zip(self.U, flat, self.versions))
 
-
-def _version(t):
-    return 0 if t.is_inference() else t._version
+def _shapes(U_groups):
+    return [[U.shape for U in g] for g in U_groups]
 
 
 def _fused(owner, U_groups, weights, x, keys, num_elements):
@@ -247,24 +245,32 @@ def _fused(owner, U_groups, weights, x, keys, num_elements):
     if not ops.CPP_OPS or torch.compiler.is_compiling() or not x.is_cuda or x.dtype not in _DTYPE_ENUM or first.dtype != x.dtype:
         return None
     plan = owner.__dict__.get("_plan")
-    if plan is None or plan.F != x.shape[1] or not plan.holds_for(U_groups):
-        ell, n_out = first.shape[-2], sum(g[0].shape[0] if g[0].dim() == len(g) + 2 else 1 for g in U_groups)
-        fits = all(len(g) <= 3 and all(U.device == x.device and U.dtype == x.dtype and U.shape[-2] == ell for U in g) for g in U_groups)
-        if not fits or ell > 25 or n_out > 64 or sum(len(g) for g in U_groups) > 48 or num_elements > 256:
+    for _ in range(2):
+        if plan is None or plan.F != x.shape[1] or plan.shapes != _shapes(U_groups) or plan.U[0].dtype != x.dtype:
+            ell, n_out = first.shape[-2], sum(g[0].shape[0] if g[0].dim() == len(g) + 2 else 1 for g in U_groups)
+            fits = all(len(g) <= 3 and all(U.device == x.device and U.dtype == x.dtype and U.shape[-2] == ell for U in g) for g in U_groups)
+            if not fits or ell > 25 or n_out > 64 or sum(len(g) for g in U_groups) > 48 or num_elements > 256:
+                return None
+            with torch.no_grad(), torch.cuda.device(x.device):
+                plan = _Plan(U_groups, num_elements, x.shape[1])
+            plan.F = x.shape[1]
+            owner.__dict__["_plan"] = plan
+        if not plan.fits:
             return None
-        with torch.no_grad(), torch.cuda.device(x.device):
-            plan = _Plan(U_groups, num_elements, x.shape[1])
-        plan.F = x.shape[1]
-        owner.__dict__["_plan"] = plan
-    if not plan.fits:
-        return None
-    return torch.ops.oeq_b200.symmetric_contraction(x, keys, weights, plan.U, plan.terms, plan.place, plan.U_rows, plan.meta, plan.out_dim)[0]
+        U = [U for g in U_groups for U in g]
+        out, _, _, changed = torch.ops.oeq_b200.symmetric_contraction(x, keys, weights, U, plan.U, plan.terms, plan.place, plan.U_rows,
+                                                                      plan.meta, plan.out_dim)
+        if not changed.item():
+            return out
+        plan = None
+    return None
 
 
 if ops.CPP_OPS:
     @torch.library.register_fake("oeq_b200::symmetric_contraction")
-    def _(x, keys, weights, U, terms, place, U_rows, meta, out_dim):
-        return x.new_empty(x.shape[0], out_dim), x.new_empty(x.shape[0], dtype=torch.int32), x.new_empty(1, dtype=torch.uint8)
+    def _(x, keys, weights, U, U_made, terms, place, U_rows, meta, out_dim):
+        return (x.new_empty(x.shape[0], out_dim), x.new_empty(x.shape[0], dtype=torch.int32), x.new_empty(1, dtype=torch.uint8),
+                torch.empty(1, dtype=torch.int32, device="cpu"))
 
     @torch.library.register_fake("oeq_b200::symmetric_contraction_backward")
     def _(grad, x, keys, group, coef, weights, U, terms, place, U_rows, meta):

@@ -1309,6 +1309,9 @@ int status_word(int** dev_ptr) {
         if (code == gprep::STATUS_BAD_INDEX)
             return fail(OEQB_EINVAL, "an earlier call was given an index array (rows / cols / transpose_perm) with a value "
                                      "out of range, or a receiver list that is not sorted; its outputs are invalid");
+        if (code == symc::STATUS_CHANGED)
+            return fail(OEQB_EINVAL, "a captured symmetric contraction was replayed with other coupling tensors than it was captured "
+                                     "with; its outputs are invalid: capture it again");
         return fail(OEQB_EKERNEL, "an earlier kernel gave up a bounded wait (code %d); its outputs are invalid", code);
     }
     if (dev_ptr) *dev_ptr = g_status_dev[dev];
@@ -2297,6 +2300,12 @@ int oeqb_selftest_bounded_wait(const void* desc, size_t desc_len, int64_t key, v
     return OEQB_OK;
 }
 
+int oeqb_stream_is_capturing(void* stream) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing((cudaStream_t)stream, &cap) != cudaSuccess) return -fail(OEQB_ECUDA, "cudaStreamIsCapturing failed");
+    return cap != cudaStreamCaptureStatusNone;
+}
+
 int oeqb_check_status(void) {
     std::lock_guard<std::mutex> lock(g_mutex);
     return status_word(nullptr);
@@ -2614,6 +2623,28 @@ int64_t oeqb_symcon_bytes(int dtype, const int32_t* meta, int n_meta, int direct
     SymPlan p;
     if (int rc = symcon_plan(meta, n_meta, &p)) return -(int64_t)rc;
     return (int64_t)(direction == 0 ? p.coef_bytes(dtype == 2 ? 8 : 4) : p.part_bytes(dtype, n_nodes));
+}
+
+int oeqb_symcon_compare(int n, const void* const* a, const void* const* b, const int64_t* bytes, int32_t* changed, void* stream) {
+    if (n < 0 || n > symc::MAX_SETS) return fail(OEQB_EINVAL, "oeqb_symcon_compare: bad size");
+    if (int rc = check_ptrs({a, b, bytes}, "oeqb_symcon_compare")) return rc;
+    symc::Pairs p{};
+    for (int i = 0; i < n; ++i) {
+        if (bytes[i] < 0 || bytes[i] % 4) return fail(OEQB_EINVAL, "oeqb_symcon_compare: bad size");
+        if (bytes[i] == 0) continue;
+        if (int rc = check_ptrs({a[i], b[i]}, "oeqb_symcon_compare")) return rc;
+        p.a[p.n] = (const unsigned*)a[i];
+        p.b[p.n] = (const unsigned*)b[i];
+        p.words[p.n++] = bytes[i] / 4;
+    }
+    std::lock_guard<std::mutex> lock(g_mutex);
+    int* status = nullptr;
+    if (int rc = status_word(&status)) return rc;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (p.n == 0) return OEQB_OK;
+    CUDA_TRY(changed ? symc::run_compare(p, changed, 1, st) : symc::run_compare(p, status, symc::STATUS_CHANGED, st));
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    return OEQB_OK;
 }
 
 int oeqb_symcon_forward(int dtype, const int32_t* meta, int n_meta, const int32_t* terms, const int32_t* place, const void* U, int64_t n_nodes,

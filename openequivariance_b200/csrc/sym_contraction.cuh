@@ -5,6 +5,7 @@
 // ell features x[n, f, :].  Its coefficients c[e, f, t] are the generalised Clebsch-Gordan tensors U applied to the
 // element's weights; only the (component, monomial) terms that U touches are kept (410 for 0e + 1o at ell = 16 out of 4 x 968).
 //
+//   compare     : whether the tensors U are still the ones that the list of terms was made from
 //   group_nodes : nodes by element, in node order (the order of every sum over nodes), and the list of 32-node tiles
 //   coefficients: c[e, t, f] = sum_k U[t, k] W[e, k, f]
 //   (kernels/sym_poly.cuh, specialised for the list of terms: the polynomials, their gradient, and for every term the sum over
@@ -25,6 +26,7 @@ constexpr int MAX_OUT = 64;        // output components over all irreps
 constexpr int MAX_ELL = 25;
 constexpr int MAX_TERMS = 1024;
 constexpr int TILE = 32;           // nodes per warp
+constexpr int STATUS_CHANGED = 42; // code stored in the status word when a captured call meets other tensors U than it was made for
 
 struct Sets {
     int n_sets, F, terms;
@@ -40,6 +42,27 @@ __device__ __forceinline__ int set_of(const Sets& s, int z) {
     int i = 0;
     while (i + 1 < s.n_sets && z >= s.z0[i + 1]) ++i;
     return i;
+}
+
+// ---- comparison -----------------------------------------------------------------------------------------------
+// The kernels are specialised for the terms that the tensors U touch, and U can change in ways that leave no trace on the host (a write
+// through .data, through another view of the memory, to a tensor without a version).  So every call compares the contents with the
+// copy that the terms were made from.  Both are read from the L2: 3 MB for 0e + 1o at ell = 16.
+struct Pairs { int n; const unsigned *a[MAX_SETS], *b[MAX_SETS]; long long words[MAX_SETS]; };
+constexpr int CMP_BLOCKS = 64, CMP_THREADS = 256;
+
+__global__ void __launch_bounds__(CMP_THREADS) compare(const __grid_constant__ Pairs p, int* changed, int code) {
+    const unsigned *a = p.a[blockIdx.y], *b = p.b[blockIdx.y];
+    const long long words = p.words[blockIdx.y], step = (long long)CMP_BLOCKS * CMP_THREADS;
+    const long long at = blockIdx.x * (long long)CMP_THREADS + threadIdx.x;
+    const long long quads = ((uintptr_t)a | (uintptr_t)b) % 16 == 0 ? words / 4 : 0;   // (a buffer may start anywhere in its storage)
+    unsigned differ = 0;
+    for (long long i = at; i < quads; i += step) {
+        const uint4 v = reinterpret_cast<const uint4*>(a)[i], w = reinterpret_cast<const uint4*>(b)[i];
+        differ |= (v.x ^ w.x) | (v.y ^ w.y) | (v.z ^ w.z) | (v.w ^ w.w);
+    }
+    for (long long i = 4 * quads + at; i < words; i += step) differ |= a[i] ^ b[i];
+    if (differ) *(volatile int*)changed = code;   // host memory
 }
 
 // ---- grouping -------------------------------------------------------------------------------------------------
@@ -191,6 +214,11 @@ __global__ void __launch_bounds__(GW_THREADS) gradient_w(const __grid_constant__
 }
 
 // ---- launches -------------------------------------------------------------------------------------------------
+inline cudaError_t run_compare(const Pairs& p, int* changed, int code, cudaStream_t st) {
+    compare<<<dim3(CMP_BLOCKS, (unsigned)p.n), CMP_THREADS, 0, st>>>(p, changed, code);
+    return cudaGetLastError();
+}
+
 inline cudaError_t run_group(const long long* keys, long long n, int G, int* group, cudaStream_t st) {
     group_nodes<<<1, 32 * GROUP_WARPS, sizeof(int) * (size_t)G * GROUP_WARPS, st>>>(keys, n, G, group);
     return cudaGetLastError();

@@ -13,6 +13,7 @@
 // Built by openequivariance_b200/build_native.py (g++ against the installed torch; links liboeq_b200.so).
 
 #include <ATen/ATen.h>
+#include <c10/core/Event.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/autograd.h>
@@ -426,8 +427,9 @@ Three autograd_conv_backward(const at::Tensor& json, int64_t hash, const at::Ten
 // ---- symmetric contraction ---------------------------------------------------------------------------------------
 // `terms`, `meta` (CPU), `place` and `U_rows` describe the contraction's tensors U (made by _torch/symmetric_contraction.py);
 // `keys` holds the element of each node; `weights` one tensor [elements, columns, channels] per (irrep, order).  The dense
-// tensors `U` are only used by gradients that are differentiated again, which Python composes.  Besides the result the forward returns what the
-// backward takes again: the nodes by element and the polynomials' coefficients.
+// tensors `U` are used by gradients that are differentiated again, which Python composes, and to see that they still are what
+// the description was made from (`U_made`).  Besides the result the forward returns what the backward takes again, the nodes by
+// element and the polynomials' coefficients, and on the host whether U has changed: the result is then to be thrown away.
 int symcon_dtype(const at::Tensor& x) {
     if (x.scalar_type() == at::kFloat) return 1;
     if (x.scalar_type() == at::kDouble) return 2;
@@ -438,9 +440,8 @@ at::Tensor aligned(const at::Tensor& t) {   // rows are read 16 bytes at a time
     return ((uintptr_t)c.data_ptr() & 15u) ? c.clone() : c;
 }
 
-Three symcon_forward(const at::Tensor& x_in, const at::Tensor& keys_in, at::TensorList weights, at::TensorList U, const at::Tensor& terms,
-                     const at::Tensor& place, const at::Tensor& U_rows, const at::Tensor& meta_in, int64_t out_dim) {
-    (void)U;
+Four symcon_forward(const at::Tensor& x_in, const at::Tensor& keys_in, at::TensorList weights, at::TensorList U, at::TensorList U_made,
+                    const at::Tensor& terms, const at::Tensor& place, const at::Tensor& U_rows, const at::Tensor& meta_in, int64_t out_dim) {
     const int32_t* meta = meta_in.data_ptr<int32_t>();
     const int n_meta = (int)meta_in.numel(), dt = symcon_dtype(x_in);
     const int64_t N = first_dim(x_in, "x");
@@ -451,21 +452,49 @@ Three symcon_forward(const at::Tensor& x_in, const at::Tensor& keys_in, at::Tens
     c10::cuda::CUDAGuard guard(x_in.device());
     at::Tensor x = aligned(x_in), keys = keys_in.contiguous();
     std::vector<at::Tensor> held;
-    std::vector<const void*> w;
+    std::vector<const void*> w, now, made;
+    std::vector<int64_t> size;
     for (size_t s = 0; s < weights.size(); ++s) {
         check(weights[s], {meta[0], meta[9 + 2 * s], meta[1]}, x.scalar_type(), "weights");
         held.push_back(weights[s].contiguous());
         w.push_back(held.back().data_ptr());
     }
+    if (U.size() != U_made.size()) refuse("symmetric_contraction: the plan does not fit the operands");
+    for (size_t s = 0; s < U.size(); ++s) {
+        check(U[s], U_made[s].sizes().vec(), U_made[s].scalar_type(), "U");
+        held.push_back(U[s].contiguous());
+        now.push_back(ptr(held.back()));
+        made.push_back(ptr(U_made[s]));
+        size.push_back((int64_t)U_made[s].nbytes());
+    }
     const int64_t bytes = oeqb_symcon_bytes(dt, meta, n_meta, 0, N);
     if (bytes < 0) done((int)-bytes, "symmetric_contraction");
     at::Tensor group = at::empty({oeqb_symcon_group_ints(N, meta[0])}, x.options().dtype(at::kInt));
     at::Tensor out = at::empty({N, out_dim}, x.options()), coef = at::empty({bytes}, x.options().dtype(at::kByte));
+    // the comparison goes first and is waited for last: the work proper is under way meanwhile.  A captured call does not wait, and
+    // has its replays report a difference.
+    const bool captured = oeqb_stream_is_capturing(current_stream(x)) == 1;
+    at::Tensor changed = at::empty({1}, at::TensorOptions().dtype(at::kInt).pinned_memory(!captured));
+    *changed.data_ptr<int32_t>() = 0;
+    done(oeqb_symcon_compare((int)U.size(), now.data(), made.data(), size.data(), captured ? nullptr : changed.data_ptr<int32_t>(),
+                             current_stream(x)),
+         "symmetric_contraction");
+    struct Compared {   // `changed` is the device's until then, whatever happens below
+        c10::Event event{c10::DeviceType::CUDA};
+        bool waits = false;
+        void wait() { if (waits) event.synchronize(); waits = false; }
+        ~Compared() { try { wait(); } catch (...) {} }
+    } compared;
+    if (!captured) {
+        compared.event.record(c10::cuda::getCurrentCUDAStream(x.device().index()));
+        compared.waits = true;
+    }
     done(oeqb_symcon_forward(dt, meta, n_meta, terms.data_ptr<int32_t>(), place.data_ptr<int32_t>(), U_rows.data_ptr(), N,
                              keys.data_ptr<int64_t>(), ptr(x), w.data(), group.data_ptr<int32_t>(), coef.data_ptr(), mptr(out),
                              current_stream(x)),
          "symmetric_contraction");
-    return {out, group, coef};
+    compared.wait();
+    return {out, group, coef, changed};
 }
 
 std::tuple<at::Tensor, std::vector<at::Tensor>> symcon_backward(const at::Tensor& cot_in, const at::Tensor& x_in, const at::Tensor& keys,
@@ -496,8 +525,8 @@ std::tuple<at::Tensor, std::vector<at::Tensor>> symcon_backward(const at::Tensor
     return {dx, dw};
 }
 
-typedef Three SymFwdSig(const at::Tensor&, const at::Tensor&, at::TensorList, at::TensorList, const at::Tensor&, const at::Tensor&,
-                        const at::Tensor&, const at::Tensor&, int64_t);
+typedef Four SymFwdSig(const at::Tensor&, const at::Tensor&, at::TensorList, at::TensorList, at::TensorList, const at::Tensor&,
+                       const at::Tensor&, const at::Tensor&, const at::Tensor&, int64_t);
 typedef std::tuple<at::Tensor, std::vector<at::Tensor>> SymBwdSig(const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
                                                                   const at::Tensor&, at::TensorList, at::TensorList, const at::Tensor&,
                                                                   const at::Tensor&, const at::Tensor&, const at::Tensor&);
@@ -538,24 +567,31 @@ variable_list symcon_composed_gradients(const at::Tensor& cot, const variable_li
 
 struct SymForward : torch::autograd::Function<SymForward> {
     static variable_list forward(AutogradContext* ctx, const at::Tensor& x, const at::Tensor& keys, at::TensorList weights, at::TensorList U,
-                                 const at::Tensor& terms, const at::Tensor& place, const at::Tensor& U_rows, const at::Tensor& meta,
-                                 int64_t out_dim) {
+                                 at::TensorList U_made, const at::Tensor& terms, const at::Tensor& place, const at::Tensor& U_rows,
+                                 const at::Tensor& meta, int64_t out_dim) {
         at::AutoDispatchBelowADInplaceOrView below;
-        auto [out, group, coef] = sym_fwd_op().call(x, keys, weights, U, terms, place, U_rows, meta, out_dim);
-        ctx->mark_non_differentiable({group, coef});
+        auto [out, group, coef, changed] = sym_fwd_op().call(x, keys, weights, U, U_made, terms, place, U_rows, meta, out_dim);
+        ctx->mark_non_differentiable({group, coef, changed});
         ctx->set_materialize_grads(false);
         variable_list saved{x};
         saved.insert(saved.end(), weights.begin(), weights.end());
         ctx->save_for_backward(saved);
         ctx->saved_data["fixed"] = std::vector<at::Tensor>{keys, group, coef, terms, place, U_rows, meta};
         ctx->saved_data["U"] = U.vec();
-        return {out, group, coef};
+        std::vector<int64_t> versions;
+        for (const at::Tensor& u : U) versions.push_back(u.is_inference() ? 0 : (int64_t)u._version());
+        ctx->saved_data["versions"] = versions;
+        return {out, group, coef, changed};
     }
     static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
         const variable_list v = ctx->get_saved_variables();
         const std::vector<at::Tensor> U = ctx->saved_data["U"].toTensorVector(), fixed = ctx->saved_data["fixed"].toTensorVector();
         variable_list out(v.size() + 1);
         if (grads[0].defined() && at::GradMode::is_enabled()) {
+            const std::vector<int64_t> versions = ctx->saved_data["versions"].toIntVector();
+            for (size_t s = 0; s < U.size(); ++s)
+                if (!U[s].is_inference() && (int64_t)U[s]._version() != versions[s])
+                    refuse("one of the variables needed for gradient computation has been modified by an inplace operation: U");
             const variable_list d = symcon_composed_gradients(grads[0], v, fixed[0], U, fixed[6]);
             out[0] = d[0];
             std::copy(d.begin() + 1, d.end(), out.begin() + 2);
@@ -565,27 +601,27 @@ struct SymForward : torch::autograd::Function<SymForward> {
             out[0] = dx;
             std::copy(dw.begin(), dw.end(), out.begin() + 2);
         }
-        out.resize(out.size() + U.size() + 5);   // U, terms, place, U_rows, meta, out_dim
+        out.resize(out.size() + 2 * U.size() + 5);   // U, U_made, terms, place, U_rows, meta, out_dim
         return out;
     }
 };
 
-Three autograd_symcon(const at::Tensor& x, const at::Tensor& keys, at::TensorList weights, at::TensorList U, const at::Tensor& terms,
-                      const at::Tensor& place, const at::Tensor& U_rows, const at::Tensor& meta, int64_t out_dim) {
+Four autograd_symcon(const at::Tensor& x, const at::Tensor& keys, at::TensorList weights, at::TensorList U, at::TensorList U_made,
+                     const at::Tensor& terms, const at::Tensor& place, const at::Tensor& U_rows, const at::Tensor& meta, int64_t out_dim) {
     bool any = records(x);
     for (const at::Tensor& w : weights) any = any || records(w);
     if (any) {
-        const variable_list out = SymForward::apply(x, keys, weights, U, terms, place, U_rows, meta, out_dim);
-        return {out[0], out[1], out[2]};
+        const variable_list out = SymForward::apply(x, keys, weights, U, U_made, terms, place, U_rows, meta, out_dim);
+        return {out[0], out[1], out[2], out[3]};
     }
     at::AutoDispatchBelowADInplaceOrView below;
-    return sym_fwd_op().call(x, keys, weights, U, terms, place, U_rows, meta, out_dim);
+    return sym_fwd_op().call(x, keys, weights, U, U_made, terms, place, U_rows, meta, out_dim);
 }
 
 }  // namespace
 
 TORCH_LIBRARY_FRAGMENT(oeq_b200, m) {
-    m.def("symmetric_contraction(Tensor x, Tensor keys, Tensor[] weights, Tensor[] U, Tensor terms, Tensor place, Tensor U_rows, Tensor meta, int out_dim) -> (Tensor, Tensor, Tensor)");
+    m.def("symmetric_contraction(Tensor x, Tensor keys, Tensor[] weights, Tensor[] U, Tensor[] U_made, Tensor terms, Tensor place, Tensor U_rows, Tensor meta, int out_dim) -> (Tensor, Tensor, Tensor, Tensor)");
     m.def("symmetric_contraction_backward(Tensor grad, Tensor x, Tensor keys, Tensor group, Tensor coef, Tensor[] weights, Tensor[] U, Tensor terms, Tensor place, Tensor U_rows, Tensor meta) -> (Tensor, Tensor[])");
 }
 TORCH_LIBRARY_IMPL(oeq_b200, CUDA, m) {

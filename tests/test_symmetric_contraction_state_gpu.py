@@ -1,0 +1,95 @@
+"""What the symmetric contraction keeps between calls: it has to answer for the tensors, weights and devices that a module has
+now, on whatever stream and thread it is called."""
+import pytest
+import torch
+
+from helpers import rel_l2
+from test_symmetric_contraction_fused_gpu import TOL, _oracle, _setup
+
+pytestmark = pytest.mark.gpu
+
+
+def _right(sc, Us, elem, x, out):
+    want, _, _ = _oracle(sc, Us, elem, x)
+    return rel_l2(out.detach().cpu().numpy(), want.detach().cpu().numpy()) <= TOL[x.dtype]
+
+
+def _data(c, nu, new):
+    c._buffers[f"U_matrix_{nu}"].data.copy_(new)
+
+
+def _in_place(c, nu, new):
+    with torch.no_grad():
+        c._buffers[f"U_matrix_{nu}"].copy_(new)
+
+
+def _replaced(c, nu, new):
+    setattr(c, f"U_matrix_{nu}", new.to(c._buffers[f"U_matrix_{nu}"].dtype))
+
+
+def _transposed(c, nu, new):
+    # the same numbers in another order of memory, and off a 16-byte boundary
+    old = c._buffers[f"U_matrix_{nu}"]
+    store = torch.empty(old.numel() + 1, device=old.device, dtype=old.dtype)[1:]
+    setattr(c, f"U_matrix_{nu}", store.view(old.shape[::-1]).permute(*reversed(range(old.dim()))).copy_(new))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("change", [_data, _in_place, _replaced, _transposed])
+def test_changed_tensors_are_seen(change, dtype):
+    sc, Us, elem, y, x, _, _ = _setup(5, 6, 37, 3, dtype, keep=0.4)
+    assert _right(sc, Us, elem, x, sc(x, y))
+    new = [{nu: U.flip(0) for nu, U in U_set.items()} for U_set in Us]
+    new[1] = dict(Us[1])
+    new[1][3] = Us[1][3].clone()
+    new[1][3].view(-1)[-1] += 1.0                                   # one number, the last of the last tensor
+    for c, U_set, old in zip(sc.contractions, new, Us):
+        for nu in U_set:
+            if not torch.equal(U_set[nu], old[nu]):
+                change(c, nu, U_set[nu])
+    assert _right(sc, new, elem, x, sc(x, y))
+    assert _right(sc, new, elem, x, sc(x, y))
+
+
+def test_changed_tensors_of_a_module_made_in_inference_mode():
+    with torch.inference_mode():
+        sc, Us, elem, y, x, _, _ = _setup(5, 6, 37, 3, torch.float64, keep=0.4)
+        other = _setup(5, 6, 37, 3, torch.float64, seed=1, keep=0.4)
+        assert _right(sc, Us, elem, x, sc(x, y))
+        sc.load_state_dict(other[0].state_dict())
+        assert _right(sc, other[1], elem, x, sc(x, y))
+
+
+def test_captured_call_reports_changed_tensors():
+    from openequivariance_b200 import native
+    sc, Us, elem, y, x, _, _ = _setup(5, 6, 37, 3, torch.float32, keep=0.4)
+    x = x.detach()
+    for p in sc.parameters():
+        p.requires_grad_(False)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        want = sc(x, y)
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = sc(x, y)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want) and native.load().oeqb_check_status() == 0
+    sc.contractions[0].U_matrix_2.data.mul_(2)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert native.load().oeqb_check_status() != 0
+    assert native.load().oeqb_check_status() == 0                  # reported once
+    Us[0][2] = Us[0][2] * 2
+    assert _right(sc, Us, elem, x, sc(x, y))
+
+
+def test_tensors_changed_before_a_gradient_that_is_differentiated_again():
+    sc, Us, elem, y, x, cot, _ = _setup(5, 6, 37, 3, torch.float64, keep=0.4)
+    out = sc(x, y)
+    with torch.no_grad():
+        sc.contractions[0].U_matrix_2.mul_(2)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        torch.autograd.grad(out, x, cot, create_graph=True)
