@@ -215,12 +215,15 @@ OEQB_API int oeqb_group_mm(int dtype, int ragged_inner, int64_t num_groups, int6
  * ascending factors (ell = none) in the order of use; the kernels are specialised for them on first sight of the key.
  * place (device): row of U -> its term.  U (device): the sets' rows, one after the other.  weights (host array of device
  * pointers, one per set): [G, columns, F].  group (oeqb_symcon_group_ints values) and coef (oeqb_symcon_bytes, direction 0)
- * are filled by the forward call and handed to the backward call; its workspace is oeqb_symcon_bytes, direction 1. */
+ * are filled by the forward call (group beforehand, by oeqb_symcon_group, where keys is NULL) and handed to the backward call; its workspace is oeqb_symcon_bytes, direction 1. */
 /* oeqb_symcon_compare: are the n arrays a[i] (device, bytes[i]: a multiple of 4) still equal to b[i]?  If not, the stream's work sets
  * *changed (pinned host memory that the caller has set to zero) to 1.  NULL, for a stream that is being captured: a replay that meets
  * a difference reports it through the status word. */
 OEQB_API int oeqb_symcon_compare(int n, const void* const* a, const void* const* b, const int64_t* bytes, int32_t* changed, void* stream);
 OEQB_API int oeqb_stream_is_capturing(void* stream);   /* 1, 0 or a negative error */
+/* Nodes by element (0 ... n_elements - 1, or counted from the end if negative).  Nodes of no element are reported through the status
+ * word; their rows of the results are zero. */
+OEQB_API int oeqb_symcon_group(int64_t n_nodes, int64_t n_elements, const int64_t* keys, int32_t* group, void* stream);
 OEQB_API int64_t oeqb_symcon_group_ints(int64_t n_nodes, int64_t n_elements);
 OEQB_API int64_t oeqb_symcon_bytes(int dtype, const int32_t* meta, int n_meta, int direction, int64_t n_nodes);
 OEQB_API int oeqb_symcon_forward(int dtype, const int32_t* meta, int n_meta, const int32_t* terms, const int32_t* place, const void* U,

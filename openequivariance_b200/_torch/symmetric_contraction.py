@@ -144,6 +144,7 @@ def _composed(Us, weights, x, bincount, sorted_indices, num_elements):
 def _composed_unsorted(groups, weights, U, x, keys, num_elements):
     """The composed form for nodes in any order: ``groups`` = number of orders of each output irrep, ``weights`` and ``U``
     one tensor per (irrep, order)."""
+    keys = torch.where(keys < 0, keys + num_elements, keys)
     bincount = torch.bincount(keys, minlength=num_elements).to("cpu")
     permutation = torch.argsort(keys, stable=True)
     inverse = torch.argsort(permutation)
@@ -239,7 +240,7 @@ def _shapes(U_groups):
     return [[U.shape for U in g] for g in U_groups]
 
 
-def _fused(owner, U_groups, weights, x, keys, num_elements):
+def _fused(owner, U_groups, weights, x, keys, num_elements, check_keys):
     """Runs the fused operator; None where it does not apply (the caller then composes)."""
     first = U_groups[0][0]
     if not ops.CPP_OPS or torch.compiler.is_compiling() or not x.is_cuda or x.dtype not in _DTYPE_ENUM or first.dtype != x.dtype:
@@ -259,7 +260,7 @@ def _fused(owner, U_groups, weights, x, keys, num_elements):
             return None
         U = [U for g in U_groups for U in g]
         out, _, _, changed = torch.ops.oeq_b200.symmetric_contraction(x, keys, weights, U, plan.U, plan.terms, plan.place, plan.U_rows,
-                                                                      plan.meta, plan.out_dim)
+                                                                      plan.meta, plan.out_dim, check_keys)
         if not changed.item():
             return out
         plan = None
@@ -268,7 +269,7 @@ def _fused(owner, U_groups, weights, x, keys, num_elements):
 
 if ops.CPP_OPS:
     @torch.library.register_fake("oeq_b200::symmetric_contraction")
-    def _(x, keys, weights, U, U_made, terms, place, U_rows, meta, out_dim):
+    def _(x, keys, weights, U, U_made, terms, place, U_rows, meta, out_dim, check_keys):
         return (x.new_empty(x.shape[0], out_dim), x.new_empty(x.shape[0], dtype=torch.int32), x.new_empty(1, dtype=torch.uint8),
                 torch.empty(1, dtype=torch.int32, device="cpu"))
 
@@ -333,7 +334,7 @@ class Contraction(torch.nn.Module):
         """``x [N, F, ell]`` with the nodes sorted by element, ``bincount`` (CPU) nodes per element, ``sorted_indices [N]``
         the element of each (sorted) node."""
         Us, weights = self._tensors(), self._weights()
-        out = _fused(self, [Us], weights, x, sorted_indices, self.num_elements)
+        out = _fused(self, [Us], weights, x, sorted_indices, self.num_elements, True)
         return _composed(Us, weights, x, bincount, sorted_indices, self.num_elements) if out is None else out
 
 
@@ -355,7 +356,7 @@ class SymmetricContraction(torch.nn.Module):
         U_groups = [c._tensors() for c in contractions]
         weights = [w for c in contractions for w in c._weights()]
         if y.shape[1] <= self.num_elements:
-            out = _fused(self, U_groups, weights, x, indices, self.num_elements)
+            out = _fused(self, U_groups, weights, x, indices, self.num_elements, False)
             if out is not None:
                 return out
         return _composed_unsorted([len(g) for g in U_groups], weights, [U for g in U_groups for U in g], x, indices, self.num_elements)

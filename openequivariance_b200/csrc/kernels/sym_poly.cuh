@@ -16,7 +16,7 @@
 #pragma once
 
 struct SymParams {
-    const int* group; long long n;
+    const int* group; long long n;         // (nodes of no element are listed as element G)
     int G, F, out_dim, slices;
     const T* x; const T* cot; const T* coef;
     T* out; T* dx; T* part;
@@ -63,9 +63,14 @@ extern "C" __global__ void __launch_bounds__(32 * SYM_WPB) oeq_sym_forward(const
     const int* tl = off + p.G + 1;
     if ((int)blockIdx.x >= tl[0]) return;
     const int e = tl[1 + 2 * blockIdx.x], first = tl[2 + 2 * blockIdx.x];
-    sym_stage(cs, p, e, f0);
-    const bool live = first + lane < off[e + 1] && f < p.F;
+    const bool live = first + lane < (e < p.G ? off[e + 1] : p.n) && f < p.F;
     const long long node = live ? p.group[first + lane] : 0;
+    if (e == p.G) {
+        if (live)
+            for (int w = 0; w < NOUT; ++w) p.out[node * p.out_dim + p.out_col[w] + f * p.out_stride[w]] = T(0);
+        return;
+    }
+    sym_stage(cs, p, e, f0);
     T x[ELL], P[NOUT];
     sym_load(p.x + (live ? (node * p.F + f) * ELL : 0), x, live);
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -83,9 +88,14 @@ extern "C" __global__ void __launch_bounds__(32 * SYM_WPB) oeq_sym_backward_x(co
     const int* tl = off + p.G + 1;
     if ((int)blockIdx.x >= tl[0]) return;
     const int e = tl[1 + 2 * blockIdx.x], first = tl[2 + 2 * blockIdx.x];
-    sym_stage(cs, p, e, f0);
-    const bool live = first + lane < off[e + 1] && f < p.F;
+    const bool live = first + lane < (e < p.G ? off[e + 1] : p.n) && f < p.F;
     const long long node = live ? p.group[first + lane] : 0;
+    if (e == p.G) {
+        if (live)
+            for (int i = 0; i < ELL; ++i) p.dx[(node * p.F + f) * ELL + i] = T(0);
+        return;
+    }
+    sym_stage(cs, p, e, f0);
     T x[ELL], cot[NOUT], dx[ELL];
     sym_load(p.x + (live ? (node * p.F + f) * ELL : 0), x, live);
 #pragma unroll

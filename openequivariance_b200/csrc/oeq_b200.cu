@@ -1307,8 +1307,8 @@ int status_word(int** dev_ptr) {
     if (code != 0) {
         *(volatile int*)g_status_host[dev] = 0;
         if (code == gprep::STATUS_BAD_INDEX)
-            return fail(OEQB_EINVAL, "an earlier call was given an index array (rows / cols / transpose_perm) with a value "
-                                     "out of range, or a receiver list that is not sorted; its outputs are invalid");
+            return fail(OEQB_EINVAL, "an earlier call was given an index array (rows / cols / transpose_perm, or the nodes' elements) with a "
+                                     "value out of range, or a receiver list that is not sorted; its outputs are invalid");
         if (code == symc::STATUS_CHANGED)
             return fail(OEQB_EINVAL, "a captured symmetric contraction was replayed with other coupling tensors than it was captured "
                                      "with; its outputs are invalid: capture it again");
@@ -2608,6 +2608,14 @@ int symcon_launch(Program* prog, const char* name, dim3 grid, unsigned block, Sy
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return OEQB_OK;
 }
+// Caller holds g_mutex.
+int symcon_group(const int64_t* keys, long long n, int G, int32_t* group, cudaStream_t st) {
+    int* status = nullptr;
+    if (int rc = status_word(&status)) return rc;
+    CUDA_TRY(symc::run_group((const long long*)keys, n, G, group, status, gprep::STATUS_BAD_INDEX, st));
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    return OEQB_OK;
+}
 // as SYM_WPB in kernels/sym_poly.cuh
 unsigned symcon_wpb(const SymPlan& p, size_t elt) { return 8 * (size_t)((p.sets.terms + 3) / 4) * 4 * elt <= 48000 ? 8 : 1; }
 }  // namespace
@@ -2647,6 +2655,14 @@ int oeqb_symcon_compare(int n, const void* const* a, const void* const* b, const
     return OEQB_OK;
 }
 
+int oeqb_symcon_group(int64_t n_nodes, int64_t n_elements, const int64_t* keys, int32_t* group, void* stream) {
+    if (n_nodes < 0 || n_nodes > (1LL << 30) || n_elements < 1 || n_elements > gmm::MAX_GROUPS) return fail(OEQB_EINVAL, "oeqb_symcon_group: bad size");
+    if (n_nodes == 0) return OEQB_OK;
+    if (int rc = check_ptrs({keys, group}, "oeqb_symcon_group")) return rc;
+    std::lock_guard<std::mutex> lock(g_mutex);
+    return symcon_group(keys, n_nodes, (int)n_elements, group, (cudaStream_t)stream);
+}
+
 int oeqb_symcon_forward(int dtype, const int32_t* meta, int n_meta, const int32_t* terms, const int32_t* place, const void* U, int64_t n_nodes,
                         const int64_t* keys, const void* x, const void* const* weights, int32_t* group, void* coef, void* out, void* stream) {
     if (dtype != 1 && dtype != 2) return fail(OEQB_EINVAL, "oeqb_symcon_forward: dtype must be 1 (float32) or 2 (float64)");
@@ -2654,7 +2670,7 @@ int oeqb_symcon_forward(int dtype, const int32_t* meta, int n_meta, const int32_
     if (int rc = symcon_plan(meta, n_meta, &p)) return rc;
     if (n_nodes == 0) return OEQB_OK;
     if (n_nodes < 0 || n_nodes > (1LL << 30)) return fail(OEQB_EINVAL, "oeqb_symcon_forward: bad size");
-    if (int rc = check_ptrs({place, U, keys, x, weights, group, coef, out}, "oeqb_symcon_forward")) return rc;
+    if (int rc = check_ptrs({place, U, x, weights, group, coef, out}, "oeqb_symcon_forward")) return rc;
     if (!aligned16({x, coef})) return fail(OEQB_EINVAL, "oeqb_symcon_forward: x is not 16-byte aligned");
     std::lock_guard<std::mutex> lock(g_mutex);
     Program* prog;
@@ -2663,10 +2679,11 @@ int oeqb_symcon_forward(int dtype, const int32_t* meta, int n_meta, const int32_
     symc::Pointers w{};
     for (int s = 0; s < p.sets.n_sets; ++s) w.p[s] = (void*)weights[s];
     cudaStream_t st = (cudaStream_t)stream;
-    CUDA_TRY(symc::run_group((const long long*)keys, n_nodes, p.G, group, st));
+    if (keys)
+        if (int rc = symcon_group(keys, n_nodes, p.G, group, st)) return rc;
     CUDA_TRY(dtype == 2 ? symc::run_coefficients<double>(p.sets, p.G, (const double*)U, w, (double*)coef, st)
                         : symc::run_coefficients<float>(p.sets, p.G, (const float*)U, w, (float*)coef, st));
-    g_launches.fetch_add(2, std::memory_order_relaxed);
+    g_launches.fetch_add(1, std::memory_order_relaxed);
     SymParams a = symcon_params(p, group, n_nodes);
     a.x = x; a.coef = coef; a.out = out;
     const unsigned wpb = symcon_wpb(p, dtype == 2 ? 8 : 4);

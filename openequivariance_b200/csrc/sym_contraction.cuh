@@ -66,31 +66,32 @@ __global__ void __launch_bounds__(CMP_THREADS) compare(const __grid_constant__ P
 }
 
 // ---- grouping -------------------------------------------------------------------------------------------------
-// group: [0, N) node ids by element, [N, N + G + 1) element offsets, then [1 + 2 * (N / 32 + G)] the number of tiles and
+// group: [0, N) node ids by element, [N, N + G + 1) element offsets, then [1 + 2 * (N / 32 + G + 1)] the number of tiles and
 // (element, first position) of each.  One block, stable: warp v takes a contiguous piece of the nodes; pieces are counted,
-// scanned over (element, warp) and placed in node order.
+// scanned over (element, warp) and placed in node order.  An element counts from the end if it is negative, as an index does.  Nodes of
+// no element come last, as those of element G: they are reported through the status word and their rows are zero.
 constexpr int GROUP_WARPS = 32;
-inline long long max_tiles(long long n, int G) { return n / TILE + G; }
+inline long long max_tiles(long long n, int G) { return n / TILE + G + 1; }
 inline long long group_ints(long long n, int G) { return n + (G + 1) + 1 + 2 * max_tiles(n, G); }
 
-__global__ void __launch_bounds__(32 * GROUP_WARPS) group_nodes(const long long* __restrict__ keys, long long n, int G, int* __restrict__ group) {
-    extern __shared__ int hist[];      // [G][GROUP_WARPS]
+__device__ __forceinline__ int element_of(long long k, int G) { return k >= 0 && k < G ? (int)k : k < 0 && k >= -(long long)G ? (int)k + G : G; }
+
+__global__ void __launch_bounds__(32 * GROUP_WARPS) group_nodes(const long long* __restrict__ keys, long long n, int G, int* __restrict__ group,
+                                                               int* status, int code) {
+    extern __shared__ int hist[];      // [G + 1][GROUP_WARPS]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < G * GROUP_WARPS; i += blockDim.x) hist[i] = 0;
+    for (int i = threadIdx.x; i < (G + 1) * GROUP_WARPS; i += blockDim.x) hist[i] = 0;
     __syncthreads();
     const long long per = ((n + GROUP_WARPS - 1) / GROUP_WARPS + 31) / 32 * 32;
     const long long lo = warp * per, hi = (lo + per < n) ? lo + per : n;
-    for (long long i = lo + lane; i < hi; i += 32) {
-        const long long k = keys[i];
-        if (k >= 0 && k < G) atomicAdd(&hist[(int)k * GROUP_WARPS + warp], 1);
-    }
+    for (long long i = lo + lane; i < hi; i += 32) atomicAdd(&hist[element_of(keys[i], G) * GROUP_WARPS + warp], 1);
     __syncthreads();
     // exclusive scan over (element, warp), one warp, 32 entries at a time: an element's entries are exactly one row
     int* off = group + n;
     if (warp == 0) {
         int carry = 0, tiles = 0;
         int* tl = off + G + 1;
-        for (int g = 0; g < G; ++g) {
+        for (int g = 0; g <= G; ++g) {
             const int v = hist[g * GROUP_WARPS + lane];
             int inc = v;
 #pragma unroll
@@ -107,14 +108,14 @@ __global__ void __launch_bounds__(32 * GROUP_WARPS) group_nodes(const long long*
             }
             tiles += (cnt + TILE - 1) / TILE;
             carry += cnt;
+            if (g == G && cnt > 0 && lane == 0) *(volatile int*)status = code;
         }
-        if (lane == 0) { off[G] = carry; tl[0] = tiles; }
+        if (lane == 0) tl[0] = tiles;
     }
     __syncthreads();
     for (long long i0 = lo; i0 < hi; i0 += 32) {
         const long long i = i0 + lane;
-        const long long kk = i < hi ? keys[i] : -1;
-        const int k = (kk >= 0 && kk < G) ? (int)kk : -1;
+        const int k = i < hi ? element_of(keys[i], G) : -1;
         const unsigned same = __match_any_sync(0xffffffffu, k);
         if (k >= 0) group[hist[k * GROUP_WARPS + warp] + __popc(same & ((1u << lane) - 1u))] = (int)i;
         __syncwarp();
@@ -219,8 +220,8 @@ inline cudaError_t run_compare(const Pairs& p, int* changed, int code, cudaStrea
     return cudaGetLastError();
 }
 
-inline cudaError_t run_group(const long long* keys, long long n, int G, int* group, cudaStream_t st) {
-    group_nodes<<<1, 32 * GROUP_WARPS, sizeof(int) * (size_t)G * GROUP_WARPS, st>>>(keys, n, G, group);
+inline cudaError_t run_group(const long long* keys, long long n, int G, int* group, int* status, int code, cudaStream_t st) {
+    group_nodes<<<1, 32 * GROUP_WARPS, sizeof(int) * (size_t)(G + 1) * GROUP_WARPS, st>>>(keys, n, G, group, status, code);
     return cudaGetLastError();
 }
 

@@ -441,7 +441,8 @@ at::Tensor aligned(const at::Tensor& t) {   // rows are read 16 bytes at a time
 }
 
 Four symcon_forward(const at::Tensor& x_in, const at::Tensor& keys_in, at::TensorList weights, at::TensorList U, at::TensorList U_made,
-                    const at::Tensor& terms, const at::Tensor& place, const at::Tensor& U_rows, const at::Tensor& meta_in, int64_t out_dim) {
+                    const at::Tensor& terms, const at::Tensor& place, const at::Tensor& U_rows, const at::Tensor& meta_in, int64_t out_dim,
+                    bool check_keys) {
     const int32_t* meta = meta_in.data_ptr<int32_t>();
     const int n_meta = (int)meta_in.numel(), dt = symcon_dtype(x_in);
     const int64_t N = first_dim(x_in, "x");
@@ -471,8 +472,9 @@ Four symcon_forward(const at::Tensor& x_in, const at::Tensor& keys_in, at::Tenso
     if (bytes < 0) done((int)-bytes, "symmetric_contraction");
     at::Tensor group = at::empty({oeqb_symcon_group_ints(N, meta[0])}, x.options().dtype(at::kInt));
     at::Tensor out = at::empty({N, out_dim}, x.options()), coef = at::empty({bytes}, x.options().dtype(at::kByte));
-    // the comparison goes first and is waited for last: the work proper is under way meanwhile.  A captured call does not wait, and
-    // has its replays report a difference.
+    // The comparison goes first and is waited for last: the work proper is under way meanwhile.  So does the grouping, which checks
+    // the elements, where these are the caller's (`check_keys`).  A captured call does not wait, and has its replays report what
+    // they find.
     const bool captured = oeqb_stream_is_capturing(current_stream(x)) == 1;
     at::Tensor changed = at::empty({1}, at::TensorOptions().dtype(at::kInt).pinned_memory(!captured));
     *changed.data_ptr<int32_t>() = 0;
@@ -482,18 +484,19 @@ Four symcon_forward(const at::Tensor& x_in, const at::Tensor& keys_in, at::Tenso
     struct Compared {   // `changed` is the device's until then, whatever happens below
         c10::Event event{c10::DeviceType::CUDA};
         bool waits = false;
+        void record(const at::Tensor& t) { event.record(c10::cuda::getCurrentCUDAStream(t.device().index())); waits = true; }
         void wait() { if (waits) event.synchronize(); waits = false; }
         ~Compared() { try { wait(); } catch (...) {} }
     } compared;
-    if (!captured) {
-        compared.event.record(c10::cuda::getCurrentCUDAStream(x.device().index()));
-        compared.waits = true;
-    }
+    if (!captured) compared.record(x);
+    done(oeqb_symcon_group(N, meta[0], keys.data_ptr<int64_t>(), group.data_ptr<int32_t>(), current_stream(x)), "symmetric_contraction");
+    if (!captured && check_keys) compared.record(x);
     done(oeqb_symcon_forward(dt, meta, n_meta, terms.data_ptr<int32_t>(), place.data_ptr<int32_t>(), U_rows.data_ptr(), N,
-                             keys.data_ptr<int64_t>(), ptr(x), w.data(), group.data_ptr<int32_t>(), coef.data_ptr(), mptr(out),
+                             nullptr, ptr(x), w.data(), group.data_ptr<int32_t>(), coef.data_ptr(), mptr(out),
                              current_stream(x)),
          "symmetric_contraction");
     compared.wait();
+    if (!captured && check_keys) done(oeqb_check_status(), "symmetric_contraction");
     return {out, group, coef, changed};
 }
 
@@ -526,7 +529,7 @@ std::tuple<at::Tensor, std::vector<at::Tensor>> symcon_backward(const at::Tensor
 }
 
 typedef Four SymFwdSig(const at::Tensor&, const at::Tensor&, at::TensorList, at::TensorList, at::TensorList, const at::Tensor&,
-                       const at::Tensor&, const at::Tensor&, const at::Tensor&, int64_t);
+                       const at::Tensor&, const at::Tensor&, const at::Tensor&, int64_t, bool);
 typedef std::tuple<at::Tensor, std::vector<at::Tensor>> SymBwdSig(const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
                                                                   const at::Tensor&, at::TensorList, at::TensorList, const at::Tensor&,
                                                                   const at::Tensor&, const at::Tensor&, const at::Tensor&);
@@ -568,9 +571,9 @@ variable_list symcon_composed_gradients(const at::Tensor& cot, const variable_li
 struct SymForward : torch::autograd::Function<SymForward> {
     static variable_list forward(AutogradContext* ctx, const at::Tensor& x, const at::Tensor& keys, at::TensorList weights, at::TensorList U,
                                  at::TensorList U_made, const at::Tensor& terms, const at::Tensor& place, const at::Tensor& U_rows,
-                                 const at::Tensor& meta, int64_t out_dim) {
+                                 const at::Tensor& meta, int64_t out_dim, bool check_keys) {
         at::AutoDispatchBelowADInplaceOrView below;
-        auto [out, group, coef, changed] = sym_fwd_op().call(x, keys, weights, U, U_made, terms, place, U_rows, meta, out_dim);
+        auto [out, group, coef, changed] = sym_fwd_op().call(x, keys, weights, U, U_made, terms, place, U_rows, meta, out_dim, check_keys);
         ctx->mark_non_differentiable({group, coef, changed});
         ctx->set_materialize_grads(false);
         variable_list saved{x};
@@ -601,27 +604,28 @@ struct SymForward : torch::autograd::Function<SymForward> {
             out[0] = dx;
             std::copy(dw.begin(), dw.end(), out.begin() + 2);
         }
-        out.resize(out.size() + 2 * U.size() + 5);   // U, U_made, terms, place, U_rows, meta, out_dim
+        out.resize(out.size() + 2 * U.size() + 6);   // U, U_made, terms, place, U_rows, meta, out_dim, check_keys
         return out;
     }
 };
 
 Four autograd_symcon(const at::Tensor& x, const at::Tensor& keys, at::TensorList weights, at::TensorList U, at::TensorList U_made,
-                     const at::Tensor& terms, const at::Tensor& place, const at::Tensor& U_rows, const at::Tensor& meta, int64_t out_dim) {
+                     const at::Tensor& terms, const at::Tensor& place, const at::Tensor& U_rows, const at::Tensor& meta, int64_t out_dim,
+                     bool check_keys) {
     bool any = records(x);
     for (const at::Tensor& w : weights) any = any || records(w);
     if (any) {
-        const variable_list out = SymForward::apply(x, keys, weights, U, U_made, terms, place, U_rows, meta, out_dim);
+        const variable_list out = SymForward::apply(x, keys, weights, U, U_made, terms, place, U_rows, meta, out_dim, check_keys);
         return {out[0], out[1], out[2], out[3]};
     }
     at::AutoDispatchBelowADInplaceOrView below;
-    return sym_fwd_op().call(x, keys, weights, U, U_made, terms, place, U_rows, meta, out_dim);
+    return sym_fwd_op().call(x, keys, weights, U, U_made, terms, place, U_rows, meta, out_dim, check_keys);
 }
 
 }  // namespace
 
 TORCH_LIBRARY_FRAGMENT(oeq_b200, m) {
-    m.def("symmetric_contraction(Tensor x, Tensor keys, Tensor[] weights, Tensor[] U, Tensor[] U_made, Tensor terms, Tensor place, Tensor U_rows, Tensor meta, int out_dim) -> (Tensor, Tensor, Tensor, Tensor)");
+    m.def("symmetric_contraction(Tensor x, Tensor keys, Tensor[] weights, Tensor[] U, Tensor[] U_made, Tensor terms, Tensor place, Tensor U_rows, Tensor meta, int out_dim, bool check_keys) -> (Tensor, Tensor, Tensor, Tensor)");
     m.def("symmetric_contraction_backward(Tensor grad, Tensor x, Tensor keys, Tensor group, Tensor coef, Tensor[] weights, Tensor[] U, Tensor terms, Tensor place, Tensor U_rows, Tensor meta) -> (Tensor, Tensor[])");
 }
 TORCH_LIBRARY_IMPL(oeq_b200, CUDA, m) {

@@ -46,6 +46,7 @@ _PROTOTYPES = {
     "oeqb_group_mm": (c_int, [c_int, c_int, c_int64, c_int64, c_int64, c_int64, POINTER(c_int64), _P, _P, _P, _P]),
     "oeqb_symcon_compare": (c_int, [c_int] + [_P] * 5),
     "oeqb_stream_is_capturing": (c_int, [_P]),
+    "oeqb_symcon_group": (c_int, [c_int64, c_int64] + [_P] * 3),
     "oeqb_symcon_group_ints": (c_int64, [c_int64, c_int64]),
     "oeqb_symcon_bytes": (c_int64, [c_int, _P, c_int, c_int, c_int64]),
     "oeqb_symcon_forward": (c_int, [c_int, _P, c_int] + [_P] * 3 + [c_int64] + [_P] * 7),

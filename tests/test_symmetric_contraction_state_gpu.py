@@ -93,3 +93,43 @@ def test_tensors_changed_before_a_gradient_that_is_differentiated_again():
         sc.contractions[0].U_matrix_2.mul_(2)
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         torch.autograd.grad(out, x, cot, create_graph=True)
+
+
+@pytest.mark.parametrize("bad", [5, -6, 1 << 40])
+def test_a_node_of_no_element_is_refused(bad):
+    from openequivariance_b200 import native
+    sc, Us, elem, y, x, _, _ = _setup(5, 6, 70, 3, torch.float64, keep=0.4)
+    c, keys = sc.contractions[1], elem.sort().values
+    counts = torch.bincount(keys, minlength=5).cpu()
+    want = c(x, counts, keys)
+    keys[-1] = bad
+    with pytest.raises(RuntimeError, match="out of range"):
+        c(x, counts, keys)
+    assert native.load().oeqb_check_status() == 0                  # the refused call left nothing behind
+    keys[-1] = int(elem.max()) - 5                                  # counted from the end, as an index may be
+    assert torch.equal(c(x, counts, keys), want)
+
+
+def test_captured_nodes_of_no_element_have_zero_rows():
+    from openequivariance_b200 import native
+    sc, Us, elem, y, x, cot, _ = _setup(5, 6, 70, 3, torch.float64, keep=0.4)
+    y = y.clone()
+    c, keys = sc.contractions[1], elem.sort().values
+    counts = torch.bincount(keys, minlength=5).cpu()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        want = torch.autograd.grad(c(x, counts, keys), x, cot[:, :18])[0]
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = c(x, counts, keys)
+        dx = torch.autograd.grad(out, x, cot[:, :18])[0]
+    keys[40:] = 9
+    out.detach().fill_(7.0)
+    dx.fill_(7.0)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert native.load().oeqb_check_status() != 0
+    assert not out[40:].any() and not dx[40:].any() and bool(out[:40].any())
+    assert torch.equal(dx[:40], want[:40])
