@@ -39,6 +39,19 @@ def _check_cuda(t, name):
         raise RuntimeError(f"Tensor '{name}' is not on the GPU.")
 
 
+def _checked_counts(ragged_counts, num_elements, N):
+    """``ragged_counts`` on the host: one non-negative count per element, as many nodes as there are."""
+    counts = ragged_counts.detach().to(device="cpu", dtype=torch.int64).contiguous()
+    if counts.numel() != num_elements:
+        raise RuntimeError(f"Shape mismatch for tensor 'ragged_counts'. Expected: [{num_elements}]. Got: {list(counts.shape)}")
+    values = counts.reshape(-1).tolist()
+    if sum(values) != N:
+        raise RuntimeError(f"ragged_counts sums to {sum(values)} but the node tensors have {N} rows")
+    if N > 0 and min(values) < 0:
+        raise RuntimeError("ragged_counts: negative group size")
+    return counts
+
+
 @torch.library.custom_op("oeq_b200::group_gemm", mutates_args=(), device_types="cuda")
 def group_gemm(A: torch.Tensor, B: torch.Tensor, ragged_counts: torch.Tensor, M: int, K: int, ragged_inner: int,
                num_elements: int) -> torch.Tensor:
@@ -50,12 +63,8 @@ def group_gemm(A: torch.Tensor, B: torch.Tensor, ragged_counts: torch.Tensor, M:
     _check_cuda(B, "B")
     if A.dtype not in _DTYPE_ENUM or B.dtype != A.dtype:
         raise RuntimeError(f"Dtype mismatch for tensor 'A' / 'B': {A.dtype}, {B.dtype}")
-    counts = ragged_counts.detach().to(device="cpu", dtype=torch.int64).contiguous()
-    if counts.numel() != num_elements:
-        raise RuntimeError(f"Shape mismatch for tensor 'ragged_counts'. Expected: [{num_elements}]. Got: {list(counts.shape)}")
     N, F = B.shape[0], B.shape[1]
-    if int(counts.sum()) != N:
-        raise RuntimeError(f"ragged_counts sums to {int(counts.sum())} but the node tensors have {N} rows")
+    counts = _checked_counts(ragged_counts, num_elements, N)
     want_A = (N, F, M) if ragged_inner == 1 else (num_elements, F, M, K)
     want_B = (N, F, M) if ragged_inner == 2 else (N, F, K)
     if tuple(A.shape) != want_A or tuple(B.shape) != want_B:
@@ -333,8 +342,11 @@ class Contraction(torch.nn.Module):
     def forward(self, x: torch.Tensor, bincount: torch.Tensor, sorted_indices: torch.Tensor) -> torch.Tensor:
         """``x [N, F, ell]`` with the nodes sorted by element, ``bincount`` (CPU) nodes per element, ``sorted_indices [N]``
         the element of each (sorted) node."""
-        Us, weights = self._tensors(), self._weights()
-        out = _fused(self, [Us], weights, x, sorted_indices, self.num_elements, True)
+        Us, weights, out = self._tensors(), self._weights(), None
+        # (the one-pass form takes each node's element from the list alone; the composed one takes an index of any kind)
+        if sorted_indices.device == x.device and sorted_indices.dtype in (torch.int32, torch.int64) and sorted_indices.shape == x.shape[:1]:
+            _checked_counts(bincount, self.num_elements, x.shape[0])
+            out = _fused(self, [Us], weights, x, sorted_indices.long(), self.num_elements, True)
         return _composed(Us, weights, x, bincount, sorted_indices, self.num_elements) if out is None else out
 
 

@@ -133,3 +133,18 @@ def test_captured_nodes_of_no_element_have_zero_rows():
     assert native.load().oeqb_check_status() != 0
     assert not out[40:].any() and not dx[40:].any() and bool(out[:40].any())
     assert torch.equal(dx[:40], want[:40])
+
+
+def test_counts_are_checked_and_every_index_type_is_taken():
+    sc, Us, elem, y, x, _, _ = _setup(5, 6, 70, 3, torch.float64, keep=0.4)
+    c, keys = sc.contractions[1], elem.sort().values
+    counts = torch.bincount(keys, minlength=5).cpu()
+    want = c(x, counts, keys)
+    assert torch.equal(c(x, counts.to(torch.int32), keys.int()), want)
+    assert torch.equal(c(x, counts.cuda(), keys), want)
+    assert rel_l2(c(x, counts, keys.cpu()).detach().cpu().numpy(), want.detach().cpu().numpy()) <= TOL[x.dtype]
+    wrong = counts.clone()
+    wrong[0] += 1
+    for bad, message in ((wrong, "sums to 71"), (counts[:4], "Shape mismatch"), (counts + torch.tensor([0, 0, 0, 1, -1]), "negative")):
+        with pytest.raises(RuntimeError, match=message):
+            c(x, bad, keys)
