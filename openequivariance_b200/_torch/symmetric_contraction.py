@@ -183,7 +183,10 @@ def _monomials(ell, device):
             starts.append(sum(f.shape[0] for f in factors))
             factors.append(torch.nn.functional.pad(tuples[first], (0, 3 - degree), value=ell))
             number.append(inverse + starts[-1])
-        _MONOMIALS[key] = (torch.cat(factors), starts, number)
+        made = (torch.cat(factors), starts, number)
+        if device.type == "cuda":
+            torch.cuda.current_stream(device).synchronize()     # whoever finds the entry may use it on another stream
+        _MONOMIALS[key] = made
     return _MONOMIALS[key]
 
 
@@ -243,6 +246,9 @@ class _Plan:
             meta += pair
         # (the number of orders of every irrep comes last: only the gradients that are differentiated again read it)
         self.meta = torch.tensor(meta + self.groups + [len(self.groups)], dtype=torch.int32)
+        # The plan is used by every stream and thread that calls the module: it is finished before anyone finds it, and what uses
+        # its tensors tells their allocator (torch_ops.cpp, used_here).
+        torch.cuda.current_stream(device).synchronize()
 
 
 def _shapes(U_groups):
@@ -270,7 +276,10 @@ def _fused(owner, U_groups, weights, x, keys, num_elements, check_keys):
         U = [U for g in U_groups for U in g]
         out, _, _, changed = torch.ops.oeq_b200.symmetric_contraction(x, keys, weights, U, plan.U, plan.terms, plan.place, plan.U_rows,
                                                                       plan.meta, plan.out_dim, check_keys)
-        if not changed.item():
+        state = changed.item()
+        if state != 1:
+            if state == 2 and plan not in owner.__dict__.setdefault("_captured", []):
+                owner.__dict__["_captured"].append(plan)     # a graph that is replayed later reads this plan, whatever the module's is then
             return out
         plan = None
     return None

@@ -429,11 +429,17 @@ Three autograd_conv_backward(const at::Tensor& json, int64_t hash, const at::Ten
 // `keys` holds the element of each node; `weights` one tensor [elements, columns, channels] per (irrep, order).  The dense
 // tensors `U` are used by gradients that are differentiated again, which Python composes, and to see that they still are what
 // the description was made from (`U_made`).  Besides the result the forward returns what the backward takes again, the nodes by
-// element and the polynomials' coefficients, and on the host whether U has changed: the result is then to be thrown away.
+// element and the polynomials' coefficients, and on the host whether U has changed (1: the result is then to be thrown away) or the
+// call was captured (2: the description has to live as long as the graph may be replayed).
 int symcon_dtype(const at::Tensor& x) {
     if (x.scalar_type() == at::kFloat) return 1;
     if (x.scalar_type() == at::kDouble) return 2;
     refuse("symmetric_contraction: x must be float32 or float64");
+}
+// A plan's tensors were allocated on the stream of the call that made it, and the plan may be dropped by another thread while this
+// call's kernels run: their memory is not given away before those have finished.
+void used_here(const at::Tensor& t) {
+    if (t.is_cuda()) t.record_stream(c10::cuda::getCurrentCUDAStream(t.device().index()).unwrap());
 }
 at::Tensor aligned(const at::Tensor& t) {   // rows are read 16 bytes at a time
     at::Tensor c = t.contiguous();
@@ -472,12 +478,15 @@ Four symcon_forward(const at::Tensor& x_in, const at::Tensor& keys_in, at::Tenso
     if (bytes < 0) done((int)-bytes, "symmetric_contraction");
     at::Tensor group = at::empty({oeqb_symcon_group_ints(N, meta[0])}, x.options().dtype(at::kInt));
     at::Tensor out = at::empty({N, out_dim}, x.options()), coef = at::empty({bytes}, x.options().dtype(at::kByte));
+    for (const at::Tensor& t : U_made) used_here(t);
+    used_here(place);
+    used_here(U_rows);
     // The comparison goes first and is waited for last: the work proper is under way meanwhile.  So does the grouping, which checks
     // the elements, where these are the caller's (`check_keys`).  A captured call does not wait, and has its replays report what
     // they find.
     const bool captured = oeqb_stream_is_capturing(current_stream(x)) == 1;
     at::Tensor changed = at::empty({1}, at::TensorOptions().dtype(at::kInt).pinned_memory(!captured));
-    *changed.data_ptr<int32_t>() = 0;
+    *changed.data_ptr<int32_t>() = captured ? 2 : 0;
     done(oeqb_symcon_compare((int)U.size(), now.data(), made.data(), size.data(), captured ? nullptr : changed.data_ptr<int32_t>(),
                              current_stream(x)),
          "symmetric_contraction");
@@ -521,6 +530,8 @@ std::tuple<at::Tensor, std::vector<at::Tensor>> symcon_backward(const at::Tensor
         dwp.push_back(dw.back().data_ptr());
     }
     at::Tensor ws = at::empty({part / elt + 1}, x.options());
+    used_here(place);
+    used_here(U_rows);
     done(oeqb_symcon_backward(dt, meta, n_meta, terms.data_ptr<int32_t>(), place.data_ptr<int32_t>(), U_rows.data_ptr(), N,
                               group.data_ptr<int32_t>(), coef.data_ptr(), ptr(x), ptr(cot), ws.data_ptr(), mptr(dx), dwp.data(),
                               current_stream(x)),

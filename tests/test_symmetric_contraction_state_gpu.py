@@ -1,5 +1,7 @@
 """What the symmetric contraction keeps between calls: it has to answer for the tensors, weights and devices that a module has
 now, on whatever stream and thread it is called."""
+import weakref
+
 import pytest
 import torch
 
@@ -83,7 +85,9 @@ def test_captured_call_reports_changed_tensors():
     assert native.load().oeqb_check_status() != 0
     assert native.load().oeqb_check_status() == 0                  # reported once
     Us[0][2] = Us[0][2] * 2
+    plan = weakref.ref(sc.__dict__["_plan"])
     assert _right(sc, Us, elem, x, sc(x, y))
+    assert sc.__dict__["_plan"] is not plan() and plan() is not None   # the graph still reads the plan that it was captured with
 
 
 def test_tensors_changed_before_a_gradient_that_is_differentiated_again():
@@ -148,3 +152,47 @@ def test_counts_are_checked_and_every_index_type_is_taken():
     for bad, message in ((wrong, "sums to 71"), (counts[:4], "Shape mismatch"), (counts + torch.tensor([0, 0, 0, 1, -1]), "negative")):
         with pytest.raises(RuntimeError, match=message):
             c(x, bad, keys)
+
+
+def test_a_plan_is_finished_before_another_stream_finds_it():
+    from openequivariance_b200._torch import symmetric_contraction as S
+    sc, Us, elem, y, x, _, _ = _setup(6, 6, 70, 3, torch.float64, keep=0.4)
+    S._MONOMIALS.clear()
+    one, two = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(one):
+        torch.cuda._sleep(200_000_000)       # about 0.1 s: whatever the first call leaves to its stream is far from done
+        S._monomials(6, x.device)
+        assert one.query()                    # nothing of the entry is left to do
+        torch.cuda._sleep(200_000_000)
+        plan = S._Plan([c._tensors() for c in sc.contractions], 5, 6)
+        assert one.query()
+        first = sc(x, y)
+    with torch.cuda.stream(two):
+        second = sc(x, y)
+    torch.cuda.synchronize()
+    assert torch.equal(first, second) and _right(sc, Us, elem, x, second)
+    assert plan.fits
+
+
+def test_a_replaced_plan_outlives_its_last_use():
+    # the allocator has to know every stream that a plan was used on: while `two` is busy, memory of the plan that `one` allocated
+    # is not handed to the next request on `one`
+    sc, Us, elem, y, x, _, _ = _setup(6, 6, 70, 3, torch.float64, keep=0.4)
+    one, two = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(one):
+        sc(x, y)
+    one.synchronize()
+    plan = sc.__dict__["_plan"]
+    held = {t.data_ptr() for t in [plan.place, plan.U_rows, *plan.U]}
+    sizes = [(t.numel() * t.element_size()) for t in [plan.place, plan.U_rows, *plan.U]]
+    with torch.cuda.stream(two):
+        sc(x, y)
+        torch.cuda._sleep(200_000_000)
+    del plan
+    sc.__dict__.pop("_plan")
+    with torch.cuda.stream(one):
+        again = [torch.empty(n, dtype=torch.uint8, device="cuda") for n in sizes for _ in range(4)]
+    assert not held & {t.data_ptr() for t in again}
+    torch.cuda.synchronize()
