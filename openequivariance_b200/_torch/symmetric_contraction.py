@@ -303,7 +303,18 @@ if ops.CPP_OPS:
               "CompositeImplicitAutograd")
 
 
-class Contraction(torch.nn.Module):
+class _Planned(torch.nn.Module):
+    """A module that keeps the plan of its calls.  The plan belongs to a device and is made where it is missing: it is no part of
+    the module's state, so copies and files of the module do not hold it."""
+
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k not in ("_plan", "_captured")}
+
+    def __setstate__(self, state):
+        super().__setstate__({k: v for k, v in state.items() if k not in ("_plan", "_captured")})
+
+
+class Contraction(_Planned):
     """Contraction for one output irrep.  ``U_matrices[nu]`` has shape ``[(2L+1,)] + [ell] * nu + [num_params_nu]``
     for ``nu = 1 ... correlation`` (the leading dimension only when the output irrep has ``L > 0``)."""
 
@@ -359,7 +370,7 @@ class Contraction(torch.nn.Module):
         return _composed(Us, weights, x, bincount, sorted_indices, self.num_elements) if out is None else out
 
 
-class SymmetricContraction(torch.nn.Module):
+class SymmetricContraction(_Planned):
     """``forward(x [N, F, ell], y [N, num_elements] one-hot)`` -> concatenation over the output irreps of
     ``[N, F * (2L+1)]``.  ``U_matrices_per_irrep``: one ``{nu: U}`` dictionary per output irrep (see ``Contraction``)."""
 

@@ -436,6 +436,26 @@ int symcon_dtype(const at::Tensor& x) {
     if (x.scalar_type() == at::kDouble) return 2;
     refuse("symmetric_contraction: x must be float32 or float64");
 }
+// The description's host part: 32-bit integers on the host, as many as its own counts say.
+const int32_t* host_part(const at::Tensor& t, const char* name, int64_t least) {
+    if (!t.is_cpu() || t.scalar_type() != at::kInt || !t.is_contiguous() || t.numel() < least)
+        refuse(std::string("symmetric_contraction: '") + name + "' must be a contiguous int32 tensor on the host with " + std::to_string(least) + " entries");
+    return t.data_ptr<int32_t>();
+}
+struct Plan {
+    const int32_t *meta, *terms;
+    int n_meta;
+};
+Plan checked_plan(const at::Tensor& terms, const at::Tensor& place, const at::Tensor& U_rows, const at::Tensor& meta, const at::Tensor& x) {
+    const int32_t* m = host_part(meta, "meta", 9);
+    host_part(meta, "meta", 9 + 2 * (int64_t)std::max(m[3], 0) + 2 * (int64_t)std::max(m[4], 0));
+    int64_t values = 0;
+    for (int s = 0; s < m[4]; ++s) values += (int64_t)m[9 + 2 * s] * m[10 + 2 * s];
+    check(place, {m[6]}, at::kInt, "place");
+    check(U_rows, {values}, x.scalar_type(), "U");
+    if (!place.is_contiguous() || !U_rows.is_contiguous()) refuse("symmetric_contraction: the plan does not fit the operands");
+    return {m, host_part(terms, "terms", 4 * (int64_t)m[6]), (int)meta.numel()};
+}
 // A plan's tensors were allocated on the stream of the call that made it, and the plan may be dropped by another thread while this
 // call's kernels run: their memory is not given away before those have finished.
 void used_here(const at::Tensor& t) {
@@ -447,14 +467,13 @@ at::Tensor aligned(const at::Tensor& t) {   // rows are read 16 bytes at a time
 }
 
 Four symcon_forward(const at::Tensor& x_in, const at::Tensor& keys_in, at::TensorList weights, at::TensorList U, at::TensorList U_made,
-                    const at::Tensor& terms, const at::Tensor& place, const at::Tensor& U_rows, const at::Tensor& meta_in, int64_t out_dim,
+                    const at::Tensor& terms_in, const at::Tensor& place, const at::Tensor& U_rows, const at::Tensor& meta_in, int64_t out_dim,
                     bool check_keys) {
-    const int32_t* meta = meta_in.data_ptr<int32_t>();
-    const int n_meta = (int)meta_in.numel(), dt = symcon_dtype(x_in);
+    const auto [meta, terms, n_meta] = checked_plan(terms_in, place, U_rows, meta_in, x_in);
+    const int dt = symcon_dtype(x_in);
     const int64_t N = first_dim(x_in, "x");
     check(x_in, {N, meta[1], meta[2]}, x_in.scalar_type(), "x");
     check(keys_in, {N}, at::kLong, "keys");
-    check(U_rows, {-1}, x_in.scalar_type(), "U");
     if (out_dim != meta[5] || (int64_t)weights.size() != meta[4]) refuse("symmetric_contraction: the plan does not fit the operands");
     c10::cuda::CUDAGuard guard(x_in.device());
     at::Tensor x = aligned(x_in), keys = keys_in.contiguous();
@@ -500,7 +519,7 @@ Four symcon_forward(const at::Tensor& x_in, const at::Tensor& keys_in, at::Tenso
     if (!captured) compared.record(x);
     done(oeqb_symcon_group(N, meta[0], keys.data_ptr<int64_t>(), group.data_ptr<int32_t>(), current_stream(x)), "symmetric_contraction");
     if (!captured && check_keys) compared.record(x);
-    done(oeqb_symcon_forward(dt, meta, n_meta, terms.data_ptr<int32_t>(), place.data_ptr<int32_t>(), U_rows.data_ptr(), N,
+    done(oeqb_symcon_forward(dt, meta, n_meta, terms, place.data_ptr<int32_t>(), U_rows.data_ptr(), N,
                              nullptr, ptr(x), w.data(), group.data_ptr<int32_t>(), coef.data_ptr(), mptr(out),
                              current_stream(x)),
          "symmetric_contraction");
@@ -511,13 +530,20 @@ Four symcon_forward(const at::Tensor& x_in, const at::Tensor& keys_in, at::Tenso
 
 std::tuple<at::Tensor, std::vector<at::Tensor>> symcon_backward(const at::Tensor& cot_in, const at::Tensor& x_in, const at::Tensor& keys,
                                                                const at::Tensor& group, const at::Tensor& coef, at::TensorList weights,
-                                                               at::TensorList U, const at::Tensor& terms, const at::Tensor& place,
+                                                               at::TensorList U, const at::Tensor& terms_in, const at::Tensor& place,
                                                                const at::Tensor& U_rows, const at::Tensor& meta_in) {
     (void)U; (void)keys;
-    const int32_t* meta = meta_in.data_ptr<int32_t>();
-    const int n_meta = (int)meta_in.numel(), dt = symcon_dtype(x_in);
-    const int64_t N = x_in.size(0);
+    const auto [meta, terms, n_meta] = checked_plan(terms_in, place, U_rows, meta_in, x_in);
+    const int dt = symcon_dtype(x_in);
+    const int64_t N = first_dim(x_in, "x");
+    check(x_in, {N, meta[1], meta[2]}, x_in.scalar_type(), "x");
     check(cot_in, {N, meta[5]}, x_in.scalar_type(), "grad");
+    const int64_t bytes = oeqb_symcon_bytes(dt, meta, n_meta, 0, N);
+    if (bytes < 0) done((int)-bytes, "symmetric_contraction_backward");
+    check(group, {oeqb_symcon_group_ints(N, meta[0])}, at::kInt, "group");
+    check(coef, {bytes}, at::kByte, "coef");
+    if ((int64_t)weights.size() != meta[4]) refuse("symmetric_contraction: the plan does not fit the operands");
+    for (size_t s = 0; s < weights.size(); ++s) check(weights[s], {meta[0], meta[9 + 2 * s], meta[1]}, x_in.scalar_type(), "weights");
     c10::cuda::CUDAGuard guard(x_in.device());
     at::Tensor x = aligned(x_in), cot = cot_in.contiguous(), dx = at::empty_like(x);
     // one allocation for the weight gradients and the scratch
@@ -532,7 +558,7 @@ std::tuple<at::Tensor, std::vector<at::Tensor>> symcon_backward(const at::Tensor
     at::Tensor ws = at::empty({part / elt + 1}, x.options());
     used_here(place);
     used_here(U_rows);
-    done(oeqb_symcon_backward(dt, meta, n_meta, terms.data_ptr<int32_t>(), place.data_ptr<int32_t>(), U_rows.data_ptr(), N,
+    done(oeqb_symcon_backward(dt, meta, n_meta, terms, place.data_ptr<int32_t>(), U_rows.data_ptr(), N,
                               group.data_ptr<int32_t>(), coef.data_ptr(), ptr(x), ptr(cot), ws.data_ptr(), mptr(dx), dwp.data(),
                               current_stream(x)),
          "symmetric_contraction_backward");
@@ -570,6 +596,7 @@ variable_list symcon_composed_gradients(const at::Tensor& cot, const variable_li
         if (t.requires_grad()) wanted.push_back(alias.back());
     }
     const int32_t* end = meta.data_ptr<int32_t>() + meta.numel() - 1;   // orders of every irrep, then their number
+    if (*end < 0 || *end >= meta.numel()) refuse("symmetric_contraction: the plan does not fit the operands");
     const std::vector<int64_t> orders(end - *end, end);
     const std::vector<at::Tensor> weights(alias.begin() + 1, alias.end());
     const at::Tensor out = sym_composed_op().call(alias[0], keys, weights, U, orders, meta.data_ptr<int32_t>()[0]);

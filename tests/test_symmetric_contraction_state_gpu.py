@@ -1,5 +1,6 @@
 """What the symmetric contraction keeps between calls: it has to answer for the tensors, weights and devices that a module has
 now, on whatever stream and thread it is called."""
+import io
 import weakref
 
 import pytest
@@ -196,3 +197,39 @@ def test_a_replaced_plan_outlives_its_last_use():
         again = [torch.empty(n, dtype=torch.uint8, device="cuda") for n in sizes for _ in range(4)]
     assert not held & {t.data_ptr() for t in again}
     torch.cuda.synchronize()
+
+
+def test_a_module_that_was_run_saved_and_loaded():
+    sc, Us, elem, y, x, _, _ = _setup(5, 6, 37, 3, torch.float64, keep=0.4)
+    want = sc(x, y)
+    sc.load_state_dict(sc.state_dict())
+    buffer = io.BytesIO()
+    torch.save(sc, buffer)
+    for where in ("cuda", "cpu"):
+        buffer.seek(0)
+        other = torch.load(buffer, map_location=where, weights_only=False).to("cuda")
+        assert torch.equal(other(x, y), want)
+        assert torch.equal(other(x, y), want)
+
+
+def test_the_host_part_of_a_plan_is_checked():
+    sc, Us, elem, y, x, cot, _ = _setup(5, 6, 37, 3, torch.float64, keep=0.4)
+    x = x.detach()
+    sc(x, y)
+    plan, U = sc.__dict__["_plan"], [U for c in sc.contractions for U in c._tensors()]
+    weights = [w.detach() for c in sc.contractions for w in c._weights()]
+    op, back = torch.ops.oeq_b200.symmetric_contraction, torch.ops.oeq_b200.symmetric_contraction_backward
+    good = dict(terms=plan.terms, place=plan.place, U_rows=plan.U_rows, meta=plan.meta)
+    out, group, coef, _ = op(x, elem, weights, U, plan.U, *good.values(), plan.out_dim, True)
+    assert torch.equal(out, sc(x, y))
+    for name, bad in (("terms", plan.terms.cuda()), ("meta", plan.meta.cuda()), ("meta", plan.meta.long()), ("meta", plan.meta[:8]),
+                      ("meta", plan.meta[:12]), ("terms", plan.terms[:-1]), ("place", plan.place.long()), ("place", plan.place[:-1]),
+                      ("place", plan.place.cpu()), ("U_rows", plan.U_rows[:-1]), ("U_rows", plan.U_rows.float())):
+        args = list(dict(good, **{name: bad}).values())
+        with pytest.raises(RuntimeError):
+            op(x, elem, weights, U, plan.U, *args, plan.out_dim, True)
+        with pytest.raises(RuntimeError):
+            back(cot, x, elem, group, coef, weights, U, *args)
+    for bad in ((group[:-1], coef), (group, coef[:-1])):
+        with pytest.raises(RuntimeError):
+            back(cot, x, elem, *bad, weights, U, *good.values())
