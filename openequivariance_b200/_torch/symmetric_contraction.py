@@ -262,14 +262,14 @@ def _fused(owner, U_groups, weights, x, keys, num_elements, check_keys):
         return None
     plan = owner.__dict__.get("_plan")
     for _ in range(2):
-        if plan is None or plan.F != x.shape[1] or plan.shapes != _shapes(U_groups) or plan.U[0].dtype != x.dtype:
+        if plan is None or plan.device != x.device or plan.F != x.shape[1] or plan.shapes != _shapes(U_groups) or plan.U[0].dtype != x.dtype:
             ell, n_out = first.shape[-2], sum(g[0].shape[0] if g[0].dim() == len(g) + 2 else 1 for g in U_groups)
             fits = all(len(g) <= 3 and all(U.device == x.device and U.dtype == x.dtype and U.shape[-2] == ell for U in g) for g in U_groups)
             if not fits or ell > 25 or n_out > 64 or sum(len(g) for g in U_groups) > 48 or num_elements > 256:
                 return None
             with torch.no_grad(), torch.cuda.device(x.device):
                 plan = _Plan(U_groups, num_elements, x.shape[1])
-            plan.F = x.shape[1]
+            plan.device, plan.F = x.device, x.shape[1]
             owner.__dict__["_plan"] = plan
         if not plan.fits:
             return None

@@ -442,6 +442,12 @@ const int32_t* host_part(const at::Tensor& t, const char* name, int64_t least) {
         refuse(std::string("symmetric_contraction: '") + name + "' must be a contiguous int32 tensor on the host with " + std::to_string(least) + " entries");
     return t.data_ptr<int32_t>();
 }
+void same_device(const at::Tensor& x, std::initializer_list<at::TensorList> lists) {
+    for (const at::TensorList& list : lists)
+        for (const at::Tensor& t : list)
+            if (t.device() != x.device())
+                refuse("symmetric_contraction: expected all tensors to be on the same device, but found " + x.device().str() + " and " + t.device().str());
+}
 struct Plan {
     const int32_t *meta, *terms;
     int n_meta;
@@ -474,6 +480,7 @@ Four symcon_forward(const at::Tensor& x_in, const at::Tensor& keys_in, at::Tenso
     const int64_t N = first_dim(x_in, "x");
     check(x_in, {N, meta[1], meta[2]}, x_in.scalar_type(), "x");
     check(keys_in, {N}, at::kLong, "keys");
+    same_device(x_in, {{keys_in, place, U_rows}, weights, U, U_made});
     if (out_dim != meta[5] || (int64_t)weights.size() != meta[4]) refuse("symmetric_contraction: the plan does not fit the operands");
     c10::cuda::CUDAGuard guard(x_in.device());
     at::Tensor x = aligned(x_in), keys = keys_in.contiguous();
@@ -542,6 +549,7 @@ std::tuple<at::Tensor, std::vector<at::Tensor>> symcon_backward(const at::Tensor
     if (bytes < 0) done((int)-bytes, "symmetric_contraction_backward");
     check(group, {oeqb_symcon_group_ints(N, meta[0])}, at::kInt, "group");
     check(coef, {bytes}, at::kByte, "coef");
+    same_device(x_in, {{cot_in, group, coef, place, U_rows}, weights});
     if ((int64_t)weights.size() != meta[4]) refuse("symmetric_contraction: the plan does not fit the operands");
     for (size_t s = 0; s < weights.size(); ++s) check(weights[s], {meta[0], meta[9 + 2 * s], meta[1]}, x_in.scalar_type(), "weights");
     c10::cuda::CUDAGuard guard(x_in.device());

@@ -233,3 +233,16 @@ def test_the_host_part_of_a_plan_is_checked():
     for bad in ((group[:-1], coef), (group, coef[:-1])):
         with pytest.raises(RuntimeError):
             back(cot, x, elem, *bad, weights, U, *good.values())
+
+
+def test_a_plan_is_for_one_device():
+    sc, Us, elem, y, x, cot, _ = _setup(5, 6, 37, 3, torch.float64, keep=0.4)
+    want = sc(x, y)
+    plan = sc.__dict__["_plan"]
+    assert plan.device == x.device
+    plan.device = torch.device("cuda", 1)      # as if the module had been called there before
+    assert torch.equal(sc(x, y), want) and sc.__dict__["_plan"] is not plan
+    if torch.cuda.device_count() > 1:
+        with pytest.raises(RuntimeError):
+            sc(x.detach().to("cuda:1"), y.to("cuda:1"))
+        assert torch.equal(sc(x, y), want)
