@@ -255,11 +255,14 @@ def _shapes(U_groups):
     return [[U.shape for U in g] for g in U_groups]
 
 
-def _fused(owner, U_groups, weights, x, keys, num_elements, check_keys):
-    """Runs the fused operator; None where it does not apply (the caller then composes)."""
+def _fused(owner, U_groups, weights, x, keys, num_elements, counts=None):
+    """Runs the fused operator; None where it does not apply (the caller then composes).  ``counts``: nodes per element, given
+    where the elements are the caller's; both are then checked."""
     first = U_groups[0][0]
     if not ops.CPP_OPS or torch.compiler.is_compiling() or not x.is_cuda or x.dtype not in _DTYPE_ENUM or first.dtype != x.dtype:
         return None
+    if counts is not None:
+        _checked_counts(counts, num_elements, x.shape[0])
     plan = owner.__dict__.get("_plan")
     for _ in range(2):
         if plan is None or plan.device != x.device or plan.F != x.shape[1] or plan.shapes != _shapes(U_groups) or plan.U[0].dtype != x.dtype:
@@ -275,7 +278,7 @@ def _fused(owner, U_groups, weights, x, keys, num_elements, check_keys):
             return None
         U = [U for g in U_groups for U in g]
         out, _, _, changed = torch.ops.oeq_b200.symmetric_contraction(x, keys, weights, U, plan.U, plan.terms, plan.place, plan.U_rows,
-                                                                      plan.meta, plan.out_dim, check_keys)
+                                                                      plan.meta, plan.out_dim, counts is not None)
         state = changed.item()
         if state != 1:
             if state == 2 and plan not in owner.__dict__.setdefault("_captured", []):
@@ -314,6 +317,10 @@ class _Planned(torch.nn.Module):
         super().__setstate__({k: v for k, v in state.items() if k not in ("_plan", "_captured")})
 
 
+_HOOKS = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")
+_GLOBAL_HOOKS = ("_global_forward_hooks", "_global_forward_pre_hooks", "_global_backward_hooks", "_global_backward_pre_hooks")
+
+
 class Contraction(_Planned):
     """Contraction for one output irrep.  ``U_matrices[nu]`` has shape ``[(2L+1,)] + [ell] * nu + [num_params_nu]``
     for ``nu = 1 ... correlation`` (the leading dimension only when the output irrep has ``L > 0``)."""
@@ -325,7 +332,6 @@ class Contraction(_Planned):
         self.correlation = max(U_matrices)
         assert sorted(U_matrices) == list(range(1, self.correlation + 1)), "U_matrices needs every order 1 ... correlation"
         self.num_features, self.num_elements = num_features, num_elements
-        self._names = [f"U_matrix_{nu}" for nu in range(self.correlation, 0, -1)]
         for nu, U in U_matrices.items():
             U = U.to(dtype)
             self.register_buffer(f"U_matrix_{nu}", U)
@@ -349,15 +355,17 @@ class Contraction(_Planned):
         return getattr(self, f"U_matrix_{nu}")
 
     def _tensors(self):
-        """``U`` from the highest order down, without ``nn.Module``'s attribute look-up."""
-        buffers = self._buffers
-        return [buffers[name] for name in self._names]
+        """``U`` from the highest order down."""
+        return [self.U(nu) for nu in range(self.correlation, 0, -1)]
 
     def _weights(self):
-        weights = self._modules.get("weights")     # (iterating a ParameterList costs several microseconds)
-        if weights is None:
-            return [self.weights_max, *self.weights]
-        return [self._parameters["weights_max"], *weights._parameters.values()]
+        # (as attributes: a parametrization, a weight normalisation or a data-parallel replica keeps them elsewhere than in `_parameters`)
+        return [self.weights_max, *self.weights]
+
+    def _plainly_called(self):
+        """Whether calling this module runs ``forward`` below and nothing else."""
+        return (type(self) is Contraction and "forward" not in self.__dict__ and getattr(self, "_compiled_call_impl", None) is None
+                and not any(self.__dict__.get(hooks) for hooks in _HOOKS))
 
     def forward(self, x: torch.Tensor, bincount: torch.Tensor, sorted_indices: torch.Tensor) -> torch.Tensor:
         """``x [N, F, ell]`` with the nodes sorted by element, ``bincount`` (CPU) nodes per element, ``sorted_indices [N]``
@@ -365,8 +373,7 @@ class Contraction(_Planned):
         Us, weights, out = self._tensors(), self._weights(), None
         # (the one-pass form takes each node's element from the list alone; the composed one takes an index of any kind)
         if sorted_indices.device == x.device and sorted_indices.dtype in (torch.int32, torch.int64) and sorted_indices.shape == x.shape[:1]:
-            _checked_counts(bincount, self.num_elements, x.shape[0])
-            out = _fused(self, [Us], weights, x, sorted_indices.long(), self.num_elements, True)
+            out = _fused(self, [Us], weights, x, sorted_indices.long(), self.num_elements, bincount)
         return _composed(Us, weights, x, bincount, sorted_indices, self.num_elements) if out is None else out
 
 
@@ -384,11 +391,16 @@ class SymmetricContraction(_Planned):
 
     def forward(self, x: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
         indices = torch.argmax(y, dim=1)
-        contractions = list(self._modules["contractions"]._modules.values())
-        U_groups = [c._tensors() for c in contractions]
-        weights = [w for c in contractions for w in c._weights()]
-        if y.shape[1] <= self.num_elements:
-            out = _fused(self, U_groups, weights, x, indices, self.num_elements, False)
+        # All output irreps in one pass, where that is what calling the contractions one by one comes to.
+        if y.shape[1] <= self.num_elements and all(isinstance(c, Contraction) and c._plainly_called() for c in self.contractions) \
+                and not any(getattr(torch.nn.modules.module, hooks, None) for hooks in _GLOBAL_HOOKS):
+            weights = [w for c in self.contractions for w in c._weights()]
+            out = _fused(self, [c._tensors() for c in self.contractions], weights, x, indices, self.num_elements)
             if out is not None:
                 return out
-        return _composed_unsorted([len(g) for g in U_groups], weights, [U for g in U_groups for U in g], x, indices, self.num_elements)
+        bincount = torch.bincount(indices, minlength=self.num_elements).to("cpu")
+        permutation = torch.argsort(indices, stable=True)
+        inverse = torch.argsort(permutation)
+        xs, sorted_indices = x[permutation], indices[permutation]
+        outs = [c(xs, bincount, sorted_indices) for c in self.contractions]
+        return torch.cat(outs, dim=-1)[inverse]

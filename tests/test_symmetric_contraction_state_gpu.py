@@ -246,3 +246,34 @@ def test_a_plan_is_for_one_device():
         with pytest.raises(RuntimeError):
             sc(x.detach().to("cuda:1"), y.to("cuda:1"))
         assert torch.equal(sc(x, y), want)
+
+
+class _Double(torch.nn.Module):
+    def forward(self, w):
+        return 2 * w
+
+
+def test_reparametrised_weights_and_hooks():
+    sc, Us, elem, y, x, cot, _ = _setup(5, 6, 37, 3, torch.float64, keep=0.4)
+    plain = sc(x, y)
+    first, second = sc.contractions
+    called = []
+    handle = second.register_forward_hook(lambda *_: called.append(1))
+    assert rel_l2(sc(x, y).detach().cpu().numpy(), plain.detach().cpu().numpy()) <= TOL[x.dtype] and called == [1]
+    handle.remove()
+    everywhere = torch.nn.modules.module.register_module_forward_hook(lambda m, *_: called.append(type(m).__name__))
+    sc(x, y)
+    everywhere.remove()
+    assert called == [1, "Contraction", "Contraction", "SymmetricContraction"]
+    torch.nn.utils.weight_norm(first, "weights_max")          # a hook makes the weight from its two parts before each call
+    with torch.no_grad():
+        first.weights_max_g.mul_(2)
+    torch.nn.utils.parametrize.register_parametrization(second, "weights_max", _Double())
+    out = sc(x, y)
+    grads = torch.autograd.grad(out, [x, first.weights_max_g, second.parametrizations.weights_max.original], cot)
+    want, xd, params = _oracle(sc, Us, elem, x)                # (the weights as they now are)
+    assert rel_l2(out.detach().cpu().numpy(), want.detach().cpu().numpy()) <= TOL[x.dtype]
+    ref = torch.autograd.grad(want, [xd, params[3]], cot)
+    assert rel_l2(grads[0].cpu().numpy(), ref[0].cpu().numpy()) <= TOL[x.dtype]
+    assert rel_l2(grads[2].cpu().numpy(), 2 * ref[1].cpu().numpy()) <= TOL[x.dtype]
+    assert bool(grads[1].any())
