@@ -27,6 +27,8 @@ import struct
 from typing import Dict, List, Optional, Sequence
 
 import torch
+from torch._subclasses.fake_tensor import FakeTensor
+from torch.fx.experimental.proxy_tensor import get_proxy_mode
 
 from .. import native
 from . import ops
@@ -251,6 +253,15 @@ class _Plan:
         torch.cuda.current_stream(device).synchronize()
 
 
+def _transformed(x):
+    """Whether something records, maps over or pushes derivatives through what is called, instead of just running it: the one-pass
+    operator has no rule for that, the composed form's operations do.  (Fake tensors take the operator's own fake.)"""
+    if torch.compiler.is_compiling() or torch.jit.is_tracing() or torch._C._are_functorch_transforms_active() \
+            or torch.autograd.forward_ad._current_level >= 0:
+        return True
+    return torch._C._len_torch_dispatch_stack() > 0 and (not isinstance(x, FakeTensor) or get_proxy_mode() is not None)
+
+
 def _shapes(U_groups):
     return [[U.shape for U in g] for g in U_groups]
 
@@ -259,7 +270,7 @@ def _fused(owner, U_groups, weights, x, keys, num_elements, counts=None):
     """Runs the fused operator; None where it does not apply (the caller then composes).  ``counts``: nodes per element, given
     where the elements are the caller's; both are then checked."""
     first = U_groups[0][0]
-    if not ops.CPP_OPS or torch.compiler.is_compiling() or not x.is_cuda or x.dtype not in _DTYPE_ENUM or first.dtype != x.dtype:
+    if not ops.CPP_OPS or _transformed(x) or not x.is_cuda or x.dtype not in _DTYPE_ENUM or first.dtype != x.dtype:
         return None
     if counts is not None:
         _checked_counts(counts, num_elements, x.shape[0])
@@ -277,9 +288,11 @@ def _fused(owner, U_groups, weights, x, keys, num_elements, counts=None):
         if not plan.fits:
             return None
         U = [U for g in U_groups for U in g]
+        if any(t.requires_grad for t in U):      # (the one-pass form has no gradient for U)
+            return None
         out, _, _, changed = torch.ops.oeq_b200.symmetric_contraction(x, keys, weights, U, plan.U, plan.terms, plan.place, plan.U_rows,
                                                                       plan.meta, plan.out_dim, counts is not None)
-        state = changed.item()
+        state = 0 if isinstance(changed, FakeTensor) else changed.item()
         if state != 1:
             if state == 2 and plan not in owner.__dict__.setdefault("_captured", []):
                 owner.__dict__["_captured"].append(plan)     # a graph that is replayed later reads this plan, whatever the module's is then

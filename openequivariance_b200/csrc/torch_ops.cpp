@@ -593,14 +593,20 @@ const c10::TypedOperatorHandle<SymComposedSig>& sym_composed_op() {
     return op;
 }
 
-// Gradients (of x, then of the weights; undefined where none is needed) that may be differentiated again: those of the composed
-// form, whose recorded graph the next order continues.  It is formed on aliases of the operands: the graph stays connected to
+bool mapped(const at::Tensor& t) {   // a transform maps over it
+    return t.key_set().has(c10::DispatchKey::FuncTorchBatched) || t.key_set().has(c10::DispatchKey::Batched);
+}
+
+// Gradients (of x, then of the weights; undefined where none is needed) that may be differentiated again, or that a transform maps
+// over: those of the composed form, whose recorded graph the next order continues.  It is formed on aliases of the operands: the graph stays connected to
 // them, so every order is right, and a gradient ends at the operand it is for even where one operand was made from another.
 variable_list symcon_composed_gradients(const at::Tensor& cot, const variable_list& operands, const at::Tensor& keys, at::TensorList U,
                                         const at::Tensor& meta) {
+    const bool again = at::GradMode::is_enabled();
+    at::AutoGradMode recording(true);
     variable_list alias, wanted, found(operands.size());
     for (const at::Tensor& t : operands) {
-        alias.push_back(t.view_as(t));
+        alias.push_back(again ? t.view_as(t) : t.detach().requires_grad_(t.requires_grad()));
         if (t.requires_grad()) wanted.push_back(alias.back());
     }
     const int32_t* end = meta.data_ptr<int32_t>() + meta.numel() - 1;   // orders of every irrep, then their number
@@ -608,7 +614,7 @@ variable_list symcon_composed_gradients(const at::Tensor& cot, const variable_li
     const std::vector<int64_t> orders(end - *end, end);
     const std::vector<at::Tensor> weights(alias.begin() + 1, alias.end());
     const at::Tensor out = sym_composed_op().call(alias[0], keys, weights, U, orders, meta.data_ptr<int32_t>()[0]);
-    const variable_list got = torch::autograd::grad({out}, wanted, {cot}, c10::nullopt, true, true);
+    const variable_list got = torch::autograd::grad({out}, wanted, {cot}, c10::nullopt, again, true);
     for (size_t i = 0, j = 0; i < alias.size(); ++i)
         if (alias[i].requires_grad()) found[i] = got[j++];
     return found;
@@ -636,7 +642,7 @@ struct SymForward : torch::autograd::Function<SymForward> {
         const variable_list v = ctx->get_saved_variables();
         const std::vector<at::Tensor> U = ctx->saved_data["U"].toTensorVector(), fixed = ctx->saved_data["fixed"].toTensorVector();
         variable_list out(v.size() + 1);
-        if (grads[0].defined() && at::GradMode::is_enabled()) {
+        if (grads[0].defined() && (at::GradMode::is_enabled() || mapped(grads[0]))) {
             const std::vector<int64_t> versions = ctx->saved_data["versions"].toIntVector();
             for (size_t s = 0; s < U.size(); ++s)
                 if (!U[s].is_inference() && (int64_t)U[s]._version() != versions[s])

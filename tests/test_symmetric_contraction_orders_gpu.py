@@ -1,4 +1,5 @@
-"""Gradients of the symmetric contraction that are differentiated again, up to third order, against einsum in fp64."""
+"""Gradients of the symmetric contraction that are differentiated again, up to third order, and calls that a transform maps
+over or records, against einsum in fp64."""
 import pytest
 import torch
 
@@ -57,3 +58,39 @@ def test_weights_made_from_the_features():
         second = torch.autograd.grad(first, operands, tangents, retain_graph=True)
         found.append([*torch.autograd.grad(out, operands, cot, retain_graph=True), *first, *second])
     _close(*found)
+
+
+def test_mapped_over_features_and_over_cotangents():
+    sc, Us, elem, y, x, cot, rnd = _setup(4, 6, 37, 3, torch.float64, keep=0.4)
+    weights = [w for c in sc.contractions for w in c._weights()]
+    want, xd, params = _oracle(sc, Us, elem, x)
+    cots = rnd(3, *cot.shape)
+    got = torch.autograd.grad(sc(x, y), [x] + weights, cots, is_grads_batched=True)
+    _close(got, torch.autograd.grad(want, [xd] + params, cots, is_grads_batched=True, retain_graph=True))
+    xs = torch.stack([x.detach(), 2 * x.detach()])
+    for p in sc.parameters():
+        p.requires_grad_(False)
+    _close(torch.func.vmap(lambda t: sc(t, y))(xs), [_oracle(sc, Us, elem, t)[0] for t in xs])
+
+
+def test_recorded_calls_follow_the_module():
+    from torch.fx.experimental.proxy_tensor import make_fx
+    sc, Us, elem, y, x, _, _ = _setup(4, 6, 37, 3, torch.float64, keep=0.4)
+    x = x.detach()
+    for p in sc.parameters():
+        p.requires_grad_(False)
+    sc(x, y)
+    recorded = [torch.jit.trace(sc, (x, y)), make_fx(sc)(x, y)]
+    sc.contractions[0].U_matrix_2.mul_(2)
+    Us[0][2] = sc.contractions[0].U_matrix_2.clone()
+    for f in recorded:
+        _close([f(x, y)], [_oracle(sc, Us, elem, x)[0]])
+
+
+def test_tensors_that_want_a_gradient():
+    sc, Us, elem, y, x, cot, _ = _setup(4, 6, 37, 3, torch.float64, keep=0.4)
+    U = sc.contractions[0].U_matrix_2.requires_grad_(True)
+    (got,) = torch.autograd.grad(sc(x, y), U, cot)
+    Us[0][2].requires_grad_(True)
+    (want,) = torch.autograd.grad(_oracle(sc, Us, elem, x)[0], Us[0][2], cot)
+    _close([got], [want])
