@@ -910,9 +910,15 @@ std::string default_cache_dir() {
     return "/tmp/oeq_b200_cubin_cache";
 }
 
-const std::string& cache_dir() {
+std::mutex g_cache_mutex;   // of the name: not every compilation holds g_mutex
+std::string cache_dir() {
+    std::lock_guard<std::mutex> lock(g_cache_mutex);
     if (g_cache_dir.empty()) g_cache_dir = default_cache_dir();
     return g_cache_dir;
+}
+void set_cache_dir(const char* dir) {
+    std::lock_guard<std::mutex> lock(g_cache_mutex);
+    g_cache_dir = dir;
 }
 
 bool read_file(const std::string& path, std::string& out) {
@@ -1759,7 +1765,7 @@ int oeqb_set_option(const char* name, const char* value) {
     if (!name || !value) return fail(OEQB_EINVAL, "oeqb_set_option: null argument");
     std::lock_guard<std::mutex> lock(g_mutex);
     std::string n = name;
-    if (n == "cache_dir") g_cache_dir = value;
+    if (n == "cache_dir") set_cache_dir(value);
     else if (n == "force_generic") g_force_generic = atoi(value) != 0;
     else if (n == "log") g_log = atoi(value) != 0;
     else if (n == "single_group") g_single_group = atoi(value) != 0;
@@ -2569,20 +2575,30 @@ std::string emit_sym(const SymPlan& p, int dtype, const SymTerm* t) {
 
 std::map<std::pair<uint64_t, int>, std::unique_ptr<Program>> g_sym_programs;   // by (key of the terms, dtype)
 
-// Caller holds g_mutex.
+std::mutex g_sym_compile_mutex;
+
+// Takes g_mutex, and leaves it while it compiles (about a second per hundred terms): the other operators of the process go on.
+// Threads that want new programs wait for one another, so that each is compiled once.
 int symcon_program(const SymPlan& p, int dtype, const int32_t* terms, Program** out) {
-    std::unique_ptr<Program>& slot = g_sym_programs[{p.key, dtype}];
-    if (!slot) {
-        if (int rc = check_ptrs({terms}, "oeqb_symcon")) return rc;
-        const SymTerm* t = (const SymTerm*)terms;
-        for (int q = 0; q < p.sets.terms; ++q)
-            if (t[q].w < 0 || t[q].w >= p.n_out || t[q].i < 0 || t[q].i >= p.ell || t[q].j < t[q].i || t[q].j > p.ell || t[q].k < t[q].j || t[q].k > p.ell)
-                return fail(OEQB_EINVAL, "oeqb_symcon: bad term");
-        auto fresh = std::make_unique<Program>();
-        if (int rc = load_program(emit_sym(p, dtype, t) + K_COMMON + K_SYM_POLY, "symmetric_contraction", fresh.get())) return rc;
-        slot = std::move(fresh);
-    }
-    *out = slot.get();
+    const std::pair<uint64_t, int> key{p.key, dtype};
+    auto known = [&] {
+        std::lock_guard<std::mutex> lock(g_mutex);
+        auto it = g_sym_programs.find(key);
+        if (it != g_sym_programs.end()) *out = it->second.get();
+        return it != g_sym_programs.end();
+    };
+    if (known()) return OEQB_OK;
+    std::lock_guard<std::mutex> compiling(g_sym_compile_mutex);
+    if (known()) return OEQB_OK;
+    if (int rc = check_ptrs({terms}, "oeqb_symcon")) return rc;
+    const SymTerm* t = (const SymTerm*)terms;
+    for (int q = 0; q < p.sets.terms; ++q)
+        if (t[q].w < 0 || t[q].w >= p.n_out || t[q].i < 0 || t[q].i >= p.ell || t[q].j < t[q].i || t[q].j > p.ell || t[q].k < t[q].j || t[q].k > p.ell)
+            return fail(OEQB_EINVAL, "oeqb_symcon: bad term");
+    auto fresh = std::make_unique<Program>();
+    if (int rc = load_program(emit_sym(p, dtype, t) + K_COMMON + K_SYM_POLY, "symmetric_contraction", fresh.get())) return rc;
+    std::lock_guard<std::mutex> lock(g_mutex);
+    *out = (g_sym_programs[key] = std::move(fresh)).get();
     return OEQB_OK;
 }
 
@@ -2672,9 +2688,9 @@ int oeqb_symcon_forward(int dtype, const int32_t* meta, int n_meta, const int32_
     if (n_nodes < 0 || n_nodes > (1LL << 30)) return fail(OEQB_EINVAL, "oeqb_symcon_forward: bad size");
     if (int rc = check_ptrs({place, U, x, weights, group, coef, out}, "oeqb_symcon_forward")) return rc;
     if (!aligned16({x, coef})) return fail(OEQB_EINVAL, "oeqb_symcon_forward: x is not 16-byte aligned");
-    std::lock_guard<std::mutex> lock(g_mutex);
     Program* prog;
     if (int rc = symcon_program(p, dtype, terms, &prog)) return rc;
+    std::lock_guard<std::mutex> lock(g_mutex);
     p.sets.place = place;
     symc::Pointers w{};
     for (int s = 0; s < p.sets.n_sets; ++s) w.p[s] = (void*)weights[s];
@@ -2706,9 +2722,9 @@ int oeqb_symcon_backward(int dtype, const int32_t* meta, int n_meta, const int32
     }
     if (int rc = check_ptrs({place, U, group, coef, x, cot, workspace, dx}, "oeqb_symcon_backward")) return rc;
     if (!aligned16({x, coef, dx})) return fail(OEQB_EINVAL, "oeqb_symcon_backward: an operand is not 16-byte aligned");
-    std::lock_guard<std::mutex> lock(g_mutex);
     Program* prog;
     if (int rc = symcon_program(p, dtype, terms, &prog)) return rc;
+    std::lock_guard<std::mutex> lock(g_mutex);
     p.sets.place = place;
     symc::Pointers dw{};
     for (int s = 0; s < p.sets.n_sets; ++s) dw.p[s] = dweights[s];

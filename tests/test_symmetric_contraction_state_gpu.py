@@ -1,6 +1,9 @@
 """What the symmetric contraction keeps between calls: it has to answer for the tensors, weights and devices that a module has
 now, on whatever stream and thread it is called."""
 import io
+import os
+import threading
+import time
 import weakref
 
 import pytest
@@ -277,3 +280,42 @@ def test_reparametrised_weights_and_hooks():
     assert rel_l2(grads[0].cpu().numpy(), ref[0].cpu().numpy()) <= TOL[x.dtype]
     assert rel_l2(grads[2].cpu().numpy(), 2 * ref[1].cpu().numpy()) <= TOL[x.dtype]
     assert bool(grads[1].any())
+
+
+def test_other_operators_run_while_a_contraction_compiles(tmp_path):
+    import openequivariance_b200 as oeq
+    from openequivariance_b200 import native
+    from openequivariance_b200.core import problems
+    p = problems.readme_problem()
+    tp = oeq.TensorProduct(p)
+    rnd = lambda *s: torch.randn(*s, device="cuda")  # noqa: E731
+    operands = [rnd(100, p.irreps_in1.dim), rnd(100, p.irreps_in2.dim), rnd(100, p.weight_numel)]
+    tp(*operands)
+    sc, Us, elem, y, x, _, _ = _setup(9, 6, 37, 3, torch.float64, seed=7, keep=0.1)     # (terms of no other test)
+    gate, done, times = threading.Event(), threading.Event(), []
+
+    def compile_it():
+        gate.set()
+        times.append(time.perf_counter())
+        try:
+            sc(x, y)
+        finally:
+            times.append(time.perf_counter())
+            done.set()
+
+    native.set_option("cache_dir", str(tmp_path))            # empty: the program has to be compiled
+    thread = threading.Thread(target=compile_it)
+    thread.start()
+    gate.wait()
+    longest, calls = 0.0, 0
+    while not done.is_set():
+        start = time.perf_counter()
+        tp(*operands)
+        if not done.is_set():
+            longest, calls = max(longest, time.perf_counter() - start), calls + 1
+        time.sleep(0.001)
+    thread.join()
+    native.set_option("cache_dir", os.path.join(os.path.dirname(oeq.__file__), "csrc", "_cubin_cache"))
+    assert times[1] - times[0] > 0.2                         # it was compiled here
+    assert calls > 10 and longest < 0.5 * (times[1] - times[0]), (calls, longest, times)
+    assert _right(sc, Us, elem, x, sc(x, y))
