@@ -21,7 +21,7 @@ EMBED = {"K_COMMON": "common.cuh", "K_GENERIC": "generic_tp.cuh", "K_FAST_UVU": 
 
 
 def _sources():
-    out = [os.path.join(CSRC, "oeq_b200.cu"), os.path.join(CSRC, "graph_prep.cuh"), os.path.join(CSRC, "group_mm.cuh"),
+    out = [os.path.join(CSRC, "oeq_b200.cu"), os.path.join(CSRC, "dealing.h"), os.path.join(CSRC, "graph_prep.cuh"), os.path.join(CSRC, "group_mm.cuh"),
            os.path.join(CSRC, "sym_contraction.cuh"), os.path.join(CSRC, "partition_plan.cuh"),
            os.path.join(HERE, "..", "include", "oeq_b200.h")]
     out += [os.path.join(CSRC, "kernels", f) for f in EMBED.values()]

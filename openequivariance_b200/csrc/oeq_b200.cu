@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "../../include/oeq_b200.h"
+#include "dealing.h"
 #include "kernels_embed.inc"  // generated at build time: K_COMMON, K_GENERIC, ... as raw strings
 #include "graph_prep.cuh"         // problem-independent kernels: grouping / sorting of edge lists
 #include "partition_plan.cuh"     // ... and the plans of the partitioned / streamed drivers
@@ -1002,8 +1003,6 @@ struct TcCuts {
     int n[9] = {0};                           // parts that S asks for (fewer when there are fewer groups)
     int cut[9][9] = {{0}};
     double part[9][8] = {{0}};
-    long long seen_tiles = -1;                // the last choice
-    int seen_splits = 0;
 };
 
 struct Entry {
@@ -1567,22 +1566,16 @@ TcCuts& tc_cuts(Entry* e, int mode) {
 // of 32 x 32, second order of 2,500 items (20 tiles on 148 SMs): 619 / 455 / 585 / 314 us (forward, dx, dy, dW) in one part, 222 / 164 /
 // 151 / 127 us in parts.
 int tc_splits(Entry* e, int mode, long long tiles) {
-    TcCuts& c = tc_cuts(e, mode);
-    if (c.seen_tiles == tiles) return c.seen_splits;
+    const TcCuts& c = tc_cuts(e, mode);
     const int sms = sm_count();
     int best = 1;
     double best_time = 0;
-    std::vector<double> load;
     for (int S = 1; S <= 8; ++S) {
         const int n = c.n[S];
         if (S > 1 && (n < S || tiles >= 16LL * sms)) break;   // too few groups, or so many tiles that the last wave hardly counts
-        load.assign(sms, 0.0);
-        for (long long u = 0; u < std::min<long long>(tiles, 16LL * sms) * n; ++u) load[u % sms] += c.part[S][u % n] + (mode == 3 ? 2.0 : 8.0);
-        const double t = *std::max_element(load.begin(), load.end()) + (mode == 2 && n > 1 ? 4.0 : 0.0);
+        const double t = busiest_load(tiles * n, n, c.part[S], mode == 3 ? 2.0 : 8.0, sms) + (mode == 2 && n > 1 ? 4.0 : 0.0);
         if (S == 1 || t < 0.95 * best_time) { best = S; best_time = t; }
     }
-    c.seen_tiles = tiles;
-    c.seen_splits = best;
     return best;
 }
 unsigned tc_set_cut(Entry* e, int mode, long long tiles, int* splits, int* cut) {   // returns the grid
