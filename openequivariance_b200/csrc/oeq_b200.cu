@@ -1194,6 +1194,24 @@ int generic_backward(Entry* e, BwdParams p, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------------------------- 'uvw' with a weight row per item
+// Where a block per item pays.  It has a fixed price (three or four barriers, four warps that start and end together: 1 to 2 ns an
+// item on a full chip), and the general kernel, a warp per item, has none.  In the forward pass that kernel's time goes with the number
+// of weight tile rows it walks (25 to 40 ps each); in the backward pass with the weights, whose gradients it stores strided, and with
+// the paths.  Few items leave the chip empty, and four warps then finish an item sooner than one.  Measured over 1 to 23 paths,
+// multiplicities 1 to 128, 500 to 200,000 items, us, general / block (same results from both):
+//   forward   4 paths 8 x 8, 100,000 items 73 / 163;    4 paths 32 x 8 216 / 175;     11 paths 16 x 16 419 / 433;   11 paths 32 x 32, 10,000 items 122 / 92
+//   backward  1 path 8 x 8, 100,000 items 71 / 159;     4 paths 8 x 8 244 / 202;      11 paths 1 x 1 322 / 247;     1 path 8 x 8, 5,000 items 9.4 / 9.1
+// The lines below are within 1.6 of the faster kernel wherever they take the block, and within 2.3 (10 to 20 us calls) where they do not.
+bool item_forward_pays(const Desc& d, long long batch) {
+    if (!d.item || g_force_generic) return false;
+    size_t rows = 0;
+    for (auto& I : d.ins) rows += d.L[0][I.a].mul;
+    return batch <= 600 || rows >= (d.dtype == 2 ? 24 + 4 * d.ins.size() : 48 + 8 * d.ins.size());
+}
+bool item_backward_pays(const Desc& d, long long batch) {
+    return d.item && !g_force_generic && (batch <= 4800 || d.ins.size() >= 8 || d.wn >= (d.dtype == 2 ? 512 : 256));
+}
+
 struct ItemFwdParams {
     const void* x; const void* y; const void* W; void* z;
     long long items;
@@ -1855,7 +1873,7 @@ int oeqb_tp_forward(const void* desc, size_t desc_len, int64_t key, int64_t batc
         return tc_forward(e, t, (cudaStream_t)stream);
     }
     if (f64_route(e->d, batch)) return f64_forward(e, x, y, W, z, batch, 0, (cudaStream_t)stream);
-    if (e->d.item && !g_force_generic && aligned16({W})) return item_forward(e, x, y, W, z, batch, 0, (cudaStream_t)stream);
+    if (item_forward_pays(e->d, batch) && aligned16({W})) return item_forward(e, x, y, W, z, batch, 0, (cudaStream_t)stream);
     FwdParams p{x, y, W, z, nullptr, nullptr, batch, batch, UNIT_ITEM, OUT_STORE};
     return generic_forward(e, p, (cudaStream_t)stream);
 }
@@ -1876,7 +1894,7 @@ int oeqb_tp_backward(const void* desc, size_t desc_len, int64_t key, int64_t bat
         return fast_launch(e, 3, f, st);
     }
     if (f64_route(d, batch)) return f64_backward(e, x, y, y, W, g, dx, dy, dW, batch, 0, st);
-    if (d.item && !g_force_generic && aligned16({W, dW})) return item_backward(e, x, y, y, W, g, dx, dy, dW, batch, 0, st);
+    if (item_backward_pays(d, batch) && aligned16({W, dW})) return item_backward(e, x, y, y, W, g, dx, dy, dW, batch, 0, st);
     const int tcb = (d.tc_bwd && !g_force_generic && !g_no_tc && aligned16({x, dx, g})) ? g_tc_backward : 0;
     if (tcb != 7) {
         CUDA_TRY(cudaMemsetAsync(dy, 0, batch * d.dim[1] * d.elt(), st));
@@ -1936,22 +1954,25 @@ int oeqb_tp_double_backward(const void* desc, size_t desc_len, int64_t key, int6
         if ((rc = f64_backward(e, x2, y2, y, W, g, dx, dy, dW, batch, 0, st))) return rc;
         return f64_backward(e, x, y, y2, W2, g, dx, dy, dW, batch, 1, st);
     }
-    if (d.item && !g_force_generic && aligned16({W, W2, dW})) {   // the five passes of the general path below
+    // dg = F(x2, y, W) + F(x, y2, W) + F(x, y, W2): the product is linear in each argument
+    if (item_forward_pays(d, batch) && aligned16({W, W2})) {
         if ((rc = item_forward(e, x2, y, W, dg, batch, 0, st))) return rc;
         if ((rc = item_forward(e, x, y2, W, dg, batch, 1, st))) return rc;
         if ((rc = item_forward(e, x, y, W2, dg, batch, 1, st))) return rc;
+    } else {
+        FwdParams f{x2, y, W, dg, nullptr, nullptr, batch, batch, UNIT_ITEM, OUT_STORE};
+        if ((rc = generic_forward(e, f, st))) return rc;
+        f.x = x; f.y = y2; f.out_mode = OUT_ADD;
+        if ((rc = generic_forward(e, f, st))) return rc;
+        f.y = y; f.W = W2;
+        if ((rc = generic_forward(e, f, st))) return rc;
+    }
+    // (dx, dy, dW) = mixed second derivatives contracted with g
+    if (item_backward_pays(d, batch) && aligned16({W, W2, dW})) {
         if ((rc = item_backward(e, x2, y2, y, W, g, dx, dy, dW, batch, 0, st))) return rc;
         return item_backward(e, x, y, y2, W2, g, dx, dy, dW, batch, 1, st);
     }
     CUDA_TRY(cudaMemsetAsync(dy, 0, batch * d.dim[1] * d.elt(), st));
-    // dg = F(x2, y, W) + F(x, y2, W) + F(x, y, W2): the product is linear in each argument
-    FwdParams f{x2, y, W, dg, nullptr, nullptr, batch, batch, UNIT_ITEM, OUT_STORE};
-    if ((rc = generic_forward(e, f, st))) return rc;
-    f.x = x; f.y = y2; f.out_mode = OUT_ADD;
-    if ((rc = generic_forward(e, f, st))) return rc;
-    f.y = y; f.W = W2;
-    if ((rc = generic_forward(e, f, st))) return rc;
-    // (dx, dy, dW) = mixed second derivatives contracted with g
     BwdParams b{x2, y2, y, W, g, dx, dy, dW, nullptr, nullptr, nullptr, batch, batch, UNIT_ITEM, 0};
     if ((rc = generic_backward(e, b, st))) return rc;
     b.x = x; b.y_dx = y; b.y_dw = y2; b.W = W2; b.accum = 1;

@@ -1,4 +1,4 @@
-"""Per-item-weight 'uvw' product (one block per item) against the fp64 oracle at the edges of its tiles: multiplicities around
+"""Per-item-weight 'uvw' product (one block per item, or the general kernels where that does not pay) against the fp64 oracle at the edges of its tiles: multiplicities around
 the 32-wide weight tiles and the widths of an access, blocks without a path, one item and many."""
 import numpy as np
 import pytest
@@ -39,3 +39,35 @@ def test_item_product_orders_0_to_2(m1, m3, l1, l3, batch, dt):
     want = (want[0], want[1], tp.reorder_weights_from_e3nn(want[2]), want[3])
     for a, b in zip(tp.double_backward_cpu(x, y, g, w, w2, x2, y2), want):
         assert rel_l2(a, b) <= REL_L2[dt]
+
+
+# a batch of the general kernels' on either side of each line: forward above 600 items with few weight rows, backward above 4,800 with
+# few weights and paths
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("batch,forward,backward", [(600, "item", "item"), (601, "generic", "item"), (4800, "generic", "item"), (4801, "generic", "generic")])
+def test_narrow_products_take_the_kernel_that_pays(batch, forward, backward, dt):
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    import openequivariance_b200 as oeq
+    p = with_dtype(_problem(4, 5), dt)
+    tp = oeq.TensorProduct(p)
+    x, y, w, g, x2, y2, w2 = uniform_inputs(p, batch)
+    we, we2 = tp.reorder_weights_to_e3nn(w), tp.reorder_weights_to_e3nn(w2)
+    leaves = [torch.tensor(t, device="cuda", requires_grad=True) for t in (x, y, w, g)]
+    with profile(activities=[ProfilerActivity.CUDA]) as record:
+        z = tp(*leaves[:3])
+        first = torch.autograd.grad(z, leaves[:3], leaves[3], create_graph=True)
+        second = torch.autograd.grad(first, leaves, [torch.tensor(t, device="cuda") for t in (x2, y2, w2)])
+        torch.cuda.synchronize()
+    count = {k: sum(e.count for e in record.key_averages() if k in e.key) for k in
+             [f"oeq_{a}_{b}" for a in ("uvw_item", "generic") for b in ("forward", "backward")]}
+    name = {"item": "oeq_uvw_item_", "generic": "oeq_generic_"}
+    assert count[name[forward] + "forward"] == 4 and count[name[backward] + "backward"] == 3, count
+    assert sum(count.values()) == 7, count
+    want = tp_oracle.double_backward(p, x, y, we, g, x2, y2, we2)
+    want = [tp_oracle.forward(p, x, y, we), *tp_oracle.backward(p, x, y, we, g), want[0], want[1], tp.reorder_weights_from_e3nn(want[2]), want[3]]
+    for n, (a, b) in enumerate(zip([z, *first, *second], want)):
+        a = a.detach().cpu().numpy()
+        a = tp.reorder_weights_to_e3nn(a) if n == 3 else a
+        assert rel_l2(a, b) <= REL_L2[dt], n
