@@ -99,3 +99,14 @@ def small_graph(n_nodes=40, mean_degree=6.0, seed=3, isolated=(5, 17)):
     order, perm = sort_edges(rows, cols)
     return {"n_nodes": n_nodes, "rows": rows[order].contiguous(), "cols": cols[order].contiguous(),
             "vec": vec[order].contiguous(), "transpose_perm": perm.contiguous()}
+
+
+def kernels_launched(call):
+    """``call()``'s result and the names of the kernels that ran in it.  (It is made twice: the profiler can miss the first kernels.)"""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as record:
+        for _ in range(2):
+            result = call()
+            torch.cuda.synchronize()
+    return result, {e.key for e in record.key_averages()}

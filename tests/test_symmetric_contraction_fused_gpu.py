@@ -1,9 +1,9 @@
-"""The one-pass symmetric contraction against einsum in fp64 at the edges of its tiles (32 nodes, 128 channels, warps of 32
-terms), with sparse tensors like the real generalised Clebsch-Gordan ones: forward, both gradients, second order."""
+"""The one-pass symmetric contraction against einsum in fp64 at the edges of its tiles (32 nodes, 128 channels, chunks of 56
+terms or 28 in doubles), with sparse tensors like the real generalised Clebsch-Gordan ones: forward, both gradients, second order."""
 import pytest
 import torch
 
-from helpers import rel_l2
+from helpers import kernels_launched, rel_l2
 from test_symmetric_contraction_gpu import _einsum_contraction
 
 pytestmark = pytest.mark.gpu
@@ -44,9 +44,13 @@ def _oracle(sc, Us, elem, x):
 def test_one_pass_contraction_at_tile_edges(ell, F, N, corr, dtype):
     sc, Us, elem, y, x, cot, rnd = _setup(ell, F, N, corr, dtype)
     weights = [w for c in sc.contractions for w in c._weights()]
-    out = sc(x, y)
-    assert sc.__dict__.get("_plan") is not None              # the one-pass operator ran
-    got = torch.autograd.grad(out, [x] + weights, cot)
+    def forward_and_gradients():
+        out = sc(x, y)
+        return out, torch.autograd.grad(out, [x] + weights, cot)
+
+    (out, got), ran = kernels_launched(forward_and_gradients)
+    assert sc.__dict__["_plan"].fits                         # the one-pass operator ran
+    assert {"oeq_sym_forward", "oeq_sym_backward_x", "oeq_sym_backward_c"} <= ran, ran
     want, xd, params = _oracle(sc, Us, elem, x)
     ref = torch.autograd.grad(want, [xd] + params, cot.double())
     assert rel_l2(out.detach().cpu().numpy(), want.detach().cpu().numpy()) <= TOL[dtype]
@@ -76,3 +80,28 @@ def test_one_pass_contraction_second_order_and_reloaded_tensors():
     for a, b in zip(got, ref):
         b = torch.zeros_like(a) if b is None else b
         assert rel_l2(a.cpu().numpy(), b.cpu().numpy()) <= 1e-12
+
+
+@pytest.mark.parametrize("dtype,terms", [(torch.float32, 55), (torch.float32, 56), (torch.float32, 57), (torch.float32, 112),
+                                         (torch.float64, 27), (torch.float64, 28), (torch.float64, 29), (torch.float64, 56)])
+def test_one_pass_contraction_at_the_chunks_of_its_terms(dtype, terms):
+    # 1 + 3 components of 25 features to the first order, and pairs of the scalar one beyond them: `terms` of them non-zero
+    from openequivariance_b200._torch.symmetric_contraction import SymmetricContraction
+    gen = torch.Generator(device="cuda").manual_seed(terms)
+    rnd = lambda *s: torch.randn(*s, device="cuda", dtype=torch.float64, generator=gen)  # noqa: E731
+    one, two, three = torch.zeros(25, 2), torch.zeros(25, 25, 1), torch.zeros(3, 25, 2)
+    places = [(one, (i,)) for i in range(25)] + [(three, (w, i)) for w in range(3) for i in range(25)] + [(two, (i, 24)) for i in range(12)]
+    for U, at in places[:terms]:
+        U[at] = 1 + len(at)
+    Us = [{1: one.double().cuda(), 2: two.double().cuda()}, {1: three.double().cuda()}]
+    sc = SymmetricContraction(Us, 5, 3, dtype=dtype).to("cuda")
+    elem = torch.randint(0, 3, (70,), device="cuda", generator=gen)
+    x, cot = rnd(70, 5, 25).to(dtype).requires_grad_(True), rnd(70, 20).to(dtype)
+    weights = [w for c in sc.contractions for w in c._weights()]
+    out = sc(x, torch.nn.functional.one_hot(elem, 3).to(dtype))
+    plan = sc.__dict__["_plan"]
+    assert plan.fits and plan.terms.shape[0] == terms
+    want, xd, params = _oracle(sc, Us, elem, x)
+    ref = torch.autograd.grad(want, [xd] + params, cot.double())
+    for a, b in zip([out, *torch.autograd.grad(out, [x] + weights, cot)], [want, *ref]):
+        assert rel_l2(a.detach().cpu().numpy(), b.detach().cpu().numpy()) <= TOL[dtype]

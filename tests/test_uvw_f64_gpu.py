@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import REL_L2, rel_l2, with_dtype
+from helpers import REL_L2, kernels_launched, rel_l2, with_dtype
 from openequivariance_b200.core.problem import TPProblem
 from oracle import tp_oracle
 
@@ -20,7 +20,8 @@ def shared_problem(wide):
                      shared_weights=True, internal_weights=False)
 
 
-def orders_0_to_2(p, batch):
+def orders_0_to_2(p, batch, kernels):
+    """All orders against the oracle; ``kernels``: names that have to be among those that ran."""
     import openequivariance_b200 as oeq
     dt = torch.float32 if p.irrep_dtype == np.float32 else torch.float64
     tp = oeq.TensorProduct(p)
@@ -29,9 +30,13 @@ def orders_0_to_2(p, batch):
     x, y, w, g = rnd(batch, p.irreps_in1.dim), rnd(batch, p.irreps_in2.dim), rnd(p.weight_numel), rnd(batch, p.irreps_out.dim)
     x2, y2, w2 = rnd(*x.shape), rnd(*y.shape), rnd(*w.shape)
     leaves = [t.cuda().requires_grad_(True) for t in (x, y, w, g)]
-    z = tp(*leaves[:3])
-    first = torch.autograd.grad(z, leaves[:3], leaves[3], create_graph=True)
-    second = torch.autograd.grad(first, leaves, [t.cuda() for t in (x2, y2, w2)])
+    def forward_and_gradients():
+        z = tp(*leaves[:3])
+        first = torch.autograd.grad(z, leaves[:3], leaves[3], create_graph=True)
+        return z, first, torch.autograd.grad(first, leaves, [t.cuda() for t in (x2, y2, w2)])
+
+    (z, first, second), ran = kernels_launched(forward_and_gradients)
+    assert set(kernels) <= ran, ran
     again = torch.autograd.grad(tp(*leaves[:3]), leaves[:3], leaves[3])
     assert all(torch.equal(a, b) for a, b in zip(first, again))        # sums run in a fixed order
     to_e3nn = lambda t: np.asarray(tp.reorder_weights_to_e3nn(t.detach().cpu().numpy()))  # noqa: E731
@@ -44,14 +49,17 @@ def orders_0_to_2(p, batch):
         assert rel_l2(a, b) <= REL_L2[p.irrep_dtype], n
 
 
+F64 = ["oeq_uvw_f64_forward", "oeq_uvw_f64_backward", "oeq_uvw_f64_backward_dw"]
+
+
 @pytest.mark.parametrize("wide", [False, True])
 @pytest.mark.parametrize("batch", [1, 7, 8, 9, 33, 1301])
 def test_doubles(batch, wide):
-    orders_0_to_2(with_dtype(shared_problem(wide), np.float64), batch)
+    orders_0_to_2(with_dtype(shared_problem(wide), np.float64), batch, F64)
 
 
 def test_degree_three_and_blocks_without_a_path():
     p = TPProblem("32x3o+32x0e+64x1o", "1x3o+1x1o", "32x3e+32x1o+64x0e+32x1e", [(0, 1, 0, "uvw", True), (0, 0, 2, "uvw", True),
                                                                                 (2, 0, 0, "uvw", True)],
                   shared_weights=True, internal_weights=False)
-    orders_0_to_2(with_dtype(p, np.float64), 45)
+    orders_0_to_2(with_dtype(p, np.float64), 45, F64)

@@ -3,7 +3,7 @@ the 32-wide weight tiles and the widths of an access, blocks without a path, one
 import numpy as np
 import pytest
 
-from helpers import REL_L2, rel_l2, uniform_inputs, with_dtype
+from helpers import REL_L2, kernels_launched, rel_l2, uniform_inputs, with_dtype
 from openequivariance_b200.core.problem import TPProblem
 from oracle import tp_oracle
 
@@ -28,11 +28,13 @@ def test_item_product_orders_0_to_2(m1, m3, l1, l3, batch, dt):
     x, y, w, g, x2, y2, w2 = uniform_inputs(p, batch)
     we, we2 = tp.reorder_weights_to_e3nn(w), tp.reorder_weights_to_e3nn(w2)
     z = np.zeros((batch, p.irreps_out.dim), dtype=dt)
-    tp.forward_cpu(x, y, z, we)
+    _, ran = kernels_launched(lambda: tp.forward_cpu(x, y, z, we))
+    assert "oeq_uvw_item_forward" in ran, ran
     # sums of at most 65 * 9 positive and negative products of numbers below one: the bounds of the other product tests hold
     assert rel_l2(z, tp_oracle.forward(p, x, y, we)) <= REL_L2[dt]
     dx, dy, dw = np.zeros_like(x), np.zeros_like(y), np.zeros_like(w)
-    tp.backward_cpu(x, dx, y, dy, g, we, dw)
+    _, ran = kernels_launched(lambda: tp.backward_cpu(x, dx, y, dy, g, we, dw))
+    assert "oeq_uvw_item_backward" in ran, ran
     for a, b in zip((dx, dy, dw), tp_oracle.backward(p, x, y, we, g)):
         assert rel_l2(a, b) <= REL_L2[dt]
     want = tp_oracle.double_backward(p, x, y, we, g, x2, y2, we2)
@@ -47,7 +49,6 @@ def test_item_product_orders_0_to_2(m1, m3, l1, l3, batch, dt):
 @pytest.mark.parametrize("batch,forward,backward", [(600, "item", "item"), (601, "generic", "item"), (4800, "generic", "item"), (4801, "generic", "generic")])
 def test_narrow_products_take_the_kernel_that_pays(batch, forward, backward, dt):
     import torch
-    from torch.profiler import ProfilerActivity, profile
 
     import openequivariance_b200 as oeq
     p = with_dtype(_problem(4, 5), dt)
@@ -55,16 +56,15 @@ def test_narrow_products_take_the_kernel_that_pays(batch, forward, backward, dt)
     x, y, w, g, x2, y2, w2 = uniform_inputs(p, batch)
     we, we2 = tp.reorder_weights_to_e3nn(w), tp.reorder_weights_to_e3nn(w2)
     leaves = [torch.tensor(t, device="cuda", requires_grad=True) for t in (x, y, w, g)]
-    with profile(activities=[ProfilerActivity.CUDA]) as record:
+
+    def forward_and_gradients():
         z = tp(*leaves[:3])
         first = torch.autograd.grad(z, leaves[:3], leaves[3], create_graph=True)
-        second = torch.autograd.grad(first, leaves, [torch.tensor(t, device="cuda") for t in (x2, y2, w2)])
-        torch.cuda.synchronize()
-    count = {k: sum(e.count for e in record.key_averages() if k in e.key) for k in
-             [f"oeq_{a}_{b}" for a in ("uvw_item", "generic") for b in ("forward", "backward")]}
+        return z, first, torch.autograd.grad(first, leaves, [torch.tensor(t, device="cuda") for t in (x2, y2, w2)])
+
+    (z, first, second), ran = kernels_launched(forward_and_gradients)
     name = {"item": "oeq_uvw_item_", "generic": "oeq_generic_"}
-    assert count[name[forward] + "forward"] == 4 and count[name[backward] + "backward"] == 3, count
-    assert sum(count.values()) == 7, count
+    assert ran & {n + k for n in name.values() for k in ("forward", "backward")} == {name[forward] + "forward", name[backward] + "backward"}, ran
     want = tp_oracle.double_backward(p, x, y, we, g, x2, y2, we2)
     want = [tp_oracle.forward(p, x, y, we), *tp_oracle.backward(p, x, y, we, g), want[0], want[1], tp.reorder_weights_from_e3nn(want[2]), want[3]]
     for n, (a, b) in enumerate(zip([z, *first, *second], want)):
