@@ -404,13 +404,15 @@ class SymmetricContraction(_Planned):
 
     def forward(self, x: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
         indices = torch.argmax(y, dim=1)
-        # All output irreps in one pass, where that is what calling the contractions one by one comes to.
-        if y.shape[1] <= self.num_elements and all(isinstance(c, Contraction) and c._plainly_called() for c in self.contractions) \
+        # All output irreps together, where that is what calling the contractions one by one comes to.
+        if not torch.compiler.is_compiling() and all(isinstance(c, Contraction) and c._plainly_called() for c in self.contractions) \
                 and not any(getattr(torch.nn.modules.module, hooks, None) for hooks in _GLOBAL_HOOKS):
+            U_groups, out = [c._tensors() for c in self.contractions], None
             weights = [w for c in self.contractions for w in c._weights()]
-            out = _fused(self, [c._tensors() for c in self.contractions], weights, x, indices, self.num_elements)
-            if out is not None:
-                return out
+            if y.shape[1] <= self.num_elements:
+                out = _fused(self, U_groups, weights, x, indices, self.num_elements)
+            return out if out is not None else _composed_unsorted([len(g) for g in U_groups], weights, [U for g in U_groups for U in g], x,
+                                                                  indices, self.num_elements)
         bincount = torch.bincount(indices, minlength=self.num_elements).to("cpu")
         permutation = torch.argsort(indices, stable=True)
         inverse = torch.argsort(permutation)

@@ -94,3 +94,10 @@ def test_tensors_that_want_a_gradient():
     Us[0][2].requires_grad_(True)
     (want,) = torch.autograd.grad(_oracle(sc, Us, elem, x)[0], Us[0][2], cot)
     _close([got], [want])
+
+
+def test_compiled_calls():
+    sc, Us, elem, y, x, cot, _ = _setup(4, 6, 37, 3, torch.float64, keep=0.4)
+    out = torch.compile(sc, backend="aot_eager", fullgraph=True)(x, y)
+    want, xd, _ = _oracle(sc, Us, elem, x)
+    _close([out, *torch.autograd.grad(out, [x], cot)], [want, *torch.autograd.grad(want, [xd], cot)])

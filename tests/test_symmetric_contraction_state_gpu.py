@@ -9,7 +9,7 @@ import weakref
 import pytest
 import torch
 
-from helpers import rel_l2
+from helpers import kernels_launched, rel_l2
 from test_symmetric_contraction_fused_gpu import TOL, _oracle, _setup
 
 pytestmark = pytest.mark.gpu
@@ -319,3 +319,11 @@ def test_other_operators_run_while_a_contraction_compiles(tmp_path):
     assert times[1] - times[0] > 0.2                         # it was compiled here
     assert calls > 10 and longest < 0.5 * (times[1] - times[0]), (calls, longest, times)
     assert _right(sc, Us, elem, x, sc(x, y))
+
+
+def test_tensors_of_too_many_terms_are_composed_at_once():
+    # 1,816 terms together, 454 of them the scalar irrep's: no kernels are compiled for a part of them
+    sc, Us, elem, y, x, cot, _ = _setup(12, 3, 20, 3, torch.float64, keep=100.0)
+    out, ran = kernels_launched(lambda: sc(x, y))
+    assert not sc.__dict__["_plan"].fits and not any("oeq_sym" in k for k in ran), ran
+    assert _right(sc, Us, elem, x, out)
