@@ -13,8 +13,9 @@
 // All sums run in an order fixed by the problem: bitwise reproducible.
 //
 // DiffDock L = 2 (multiplicities 10 and 48, 7,128 weights), 8,191 items: forward 65 us (3.8 TB/s of rows), backward 122 us (4.1 TB/s;
-// 195 us with five blocks of 127 registers to an SM instead of eight of 64 and no staged row); the general kernels (a warp per item, strided stores of
-// dW, a shuffle per product) took 733 us for both.
+// 195 us with five blocks of 127 registers to an SM and no staged row, 147 us with eight of 64 registers and none; with the row, 28 KB, and the
+// static arrays, 7 KB, six blocks fit an SM's shared memory); the general kernels (a warp per item, strided stores of dW, a shuffle per
+// product) took 733 us for both.  Narrow products do not earn the block's barriers back: the host decides (item_forward_pays, item_backward_pays).
 #pragma once
 
 // ITEM_VEC (emitted): the largest power of two up to 16 bytes that divides the row length and every weight offset.
@@ -66,8 +67,8 @@ OEQ_DEV void item_rows(int warp, int lane, F&& f) {
     });
 }
 
-// The item's weight row, requested whole by asynchronous copies before anything else is read (ITEM_STAGE_W, emitted: rows that
-// leave room for several blocks in an SM's shared memory); longer rows are read from global memory where they are used.  The backward
+// The item's weight row, requested whole by asynchronous copies before anything else is read (ITEM_STAGE_W, emitted: rows up
+// to 40 KB); longer rows are read from global memory where they are used.  The backward
 // gained (147 -> 122 us, DiffDock L = 2, 8,191 items); the forward, whose loads are already far ahead of their use, lost (65 -> 72 us) and
 // reads global memory.
 OEQ_DEV void item_request(const T* src, T* dst) {
