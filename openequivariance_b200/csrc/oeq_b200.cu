@@ -851,7 +851,8 @@ int item_vec(const Desc& d) {
     return v;
 }
 
-// Shared memory for an item's weight row: rows up to 40 KB leave room for four blocks or more in an SM; 0: not staged.
+// Shared memory for an item's weight row, 0: not staged.  Beside a row of 40 KB, the largest, two blocks fit an SM where the static arrays
+// are near their limit (48 KB), five where they are small.
 size_t item_row_bytes(const Desc& d) {
     const size_t b = (size_t)d.wn * d.elt();
     return b <= 40 * 1024 ? b : 0;
