@@ -285,8 +285,13 @@ OEQB_API int oeqb_plan_fill(int64_t n_nodes, int64_t n_edges, const void* rows, 
  * leaves the status word clear. */
 OEQB_API int oeqb_selftest_bounded_wait(const void* desc, size_t desc_len, int64_t key, void* stream);
 
-/* String options: "cache_dir" (cubin cache directory), "log" ("0"/"1"), "validate" ("0"/"1"/"2": index checks), and the
- * tuning aids "force_generic", "single_group", "single_producer", "no_tc", "tc_backward" ("0".."7"), "streams",
+/* Names of the specialised kernels (those compiled for a problem) that were launched since option "record" was set to "1", each
+ * once, in alphabetical order and followed by a newline.  A host-side record: it does not depend on a profiler.  Writes at most cap bytes and the
+ * closing zero; *needed receives the bytes that the whole text takes. */
+OEQB_API int oeqb_launched_kernels(char* buf, size_t cap, size_t* needed);
+
+/* String options: "cache_dir" (cubin cache directory), "log" ("0"/"1"), "validate" ("0"/"1"/"2": index checks), "record" ("1" empties
+ * the record of launched kernels and starts it, "0" ends it), and the tuning aids "force_generic", "single_group", "single_producer", "no_tc", "tc_backward" ("0".."7"), "streams",
  * "streams_forward".  Unknown names are refused with OEQB_EINVAL. */
 OEQB_API int oeqb_set_option(const char* name, const char* value);
 

@@ -55,6 +55,7 @@ int g_validate = 1;            // index checks of convolution calls: 0 never, 1 
 bool g_streams_fwd = false;    // the forward kernels take part in `streams` too (the backward kernels always do)
 int g_streams = 1;             // edge streams per CTA on the channel-parallel path (1: two CTAs per SM; 2-4: one CTA with
                                // that many consumer sets and a register hand-over; measured slower on the benchmark graph)
+bool g_record = false;         // keep the names of the kernels that are launched (oeqb_launched_kernels)
 std::string g_cache_dir;
 std::mutex g_mutex;
 
@@ -1247,6 +1248,10 @@ int get_program(Entry* e, int fam, Program** out, bool allow_streams = true) {
     return OEQB_OK;
 }
 
+std::map<cudaKernel_t, std::string> g_kernel_names;   // of the specialised kernels (guarded by g_mutex, as what follows)
+std::set<std::string> g_recorded;                     // those launched since the option "record" was set
+
+// Caller holds g_mutex.
 int get_kernel(Program* p, const char* name, size_t smem, cudaKernel_t* out) {
     auto it = p->kernels.find(name);
     if (it == p->kernels.end()) {
@@ -1254,6 +1259,7 @@ int get_kernel(Program* p, const char* name, size_t smem, cudaKernel_t* out) {
         cudaError_t ce = cudaLibraryGetKernel(&k, p->lib, name);
         if (ce != cudaSuccess) return fail(OEQB_ECOMPILE, "kernel %s not found: %s", name, cudaGetErrorString(ce));
         it = p->kernels.emplace(name, k).first;
+        g_kernel_names[k] = name;
     }
     if (smem > 48 * 1024) {
         int dev = 0;
@@ -1268,10 +1274,12 @@ int get_kernel(Program* p, const char* name, size_t smem, cudaKernel_t* out) {
     return OEQB_OK;
 }
 
-int launch(cudaKernel_t k, unsigned grid, unsigned block, size_t smem, void** args, cudaStream_t st) {
-    cudaError_t ce = cudaLaunchKernel((const void*)k, dim3(grid), dim3(block), args, smem, st);
-    if (ce != cudaSuccess) return fail(OEQB_ECUDA, "kernel launch failed: %s", cudaGetErrorString(ce));
+int launch(cudaKernel_t k, dim3 grid, unsigned block, size_t smem, void** args, cudaStream_t st) {
+    const auto name = g_kernel_names.find(k);
+    cudaError_t ce = cudaLaunchKernel((const void*)k, grid, dim3(block), args, smem, st);
+    if (ce != cudaSuccess) return fail(OEQB_ECUDA, "launch of %s failed: %s", name != g_kernel_names.end() ? name->second.c_str() : "a kernel", cudaGetErrorString(ce));
     g_launches.fetch_add(1, std::memory_order_relaxed);
+    if (g_record && name != g_kernel_names.end()) g_recorded.insert(name->second);
     return OEQB_OK;
 }
 
@@ -1423,10 +1431,7 @@ int f64_launch(Entry* e, const char* name, dim3 grid, void* params, cudaStream_t
     cudaKernel_t k;
     if (int rc = get_kernel(prog, name, 0, &k)) return rc;
     void* args[] = {params};
-    cudaError_t ce = cudaLaunchKernel((const void*)k, grid, dim3(128), args, 0, st);
-    if (ce != cudaSuccess) return fail(OEQB_ECUDA, "%s: %s", name, cudaGetErrorString(ce));
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    return OEQB_OK;
+    return launch(k, grid, 128, 0, args, st);
 }
 int f64_forward(Entry* e, const void* x, const void* y, const void* W, void* z, long long batch, int accum, cudaStream_t st) {
     int tiles = 0;
@@ -1981,6 +1986,7 @@ int oeqb_set_option(const char* name, const char* value) {
     if (n == "cache_dir") set_cache_dir(value);
     else if (n == "force_generic") g_force_generic = atoi(value) != 0;
     else if (n == "log") g_log = atoi(value) != 0;
+    else if (n == "record") { g_record = atoi(value) != 0; if (g_record) g_recorded.clear(); }
     else if (n == "single_group") g_single_group = atoi(value) != 0;
     else if (n == "single_producer") g_single_producer = atoi(value) != 0;
     else if (n == "streams") g_streams = atoi(value);
@@ -1989,6 +1995,20 @@ int oeqb_set_option(const char* name, const char* value) {
     else if (n == "no_tc") g_no_tc = atoi(value) != 0;
     else if (n == "tc_backward") g_tc_backward = atoi(value) & 7;
     else return fail(OEQB_EINVAL, "unknown option '%s'", name);
+    return OEQB_OK;
+}
+
+int oeqb_launched_kernels(char* buf, size_t cap, size_t* needed) {
+    if (!needed || (cap && !buf)) return fail(OEQB_EINVAL, "oeqb_launched_kernels: null argument");
+    std::lock_guard<std::mutex> lock(g_mutex);
+    std::string all;
+    for (const std::string& n : g_recorded) all += n + "\n";
+    *needed = all.size() + 1;
+    if (cap) {
+        const size_t n = std::min(all.size(), cap - 1);
+        memcpy(buf, all.data(), n);
+        buf[n] = '\0';
+    }
     return OEQB_OK;
 }
 
@@ -2831,10 +2851,7 @@ int symcon_launch(Program* prog, const char* name, dim3 grid, unsigned block, Sy
     cudaKernel_t k;
     if (int rc = get_kernel(prog, name, 0, &k)) return rc;
     void* args[] = {&a};
-    cudaError_t ce = cudaLaunchKernel((const void*)k, grid, dim3(block), args, 0, st);
-    if (ce != cudaSuccess) return fail(OEQB_ECUDA, "%s: %s", name, cudaGetErrorString(ce));
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    return OEQB_OK;
+    return launch(k, grid, block, 0, args, st);
 }
 // Caller holds g_mutex.
 int symcon_group(const int64_t* keys, long long n, int G, int32_t* group, cudaStream_t st) {

@@ -62,6 +62,7 @@ _PROTOTYPES = {
     "oeqb_precompile": (c_int, _DESC),
     "oeqb_set_option": (c_int, [c_char_p, c_char_p]),
     "oeqb_launch_count": (c_int64, []),
+    "oeqb_launched_kernels": (c_int, [c_char_p, c_size_t, POINTER(c_size_t)]),
     "oeqb_last_error": (c_char_p, []),
     "oeqb_version": (c_char_p, []),
 }
@@ -149,6 +150,16 @@ def precompile(desc: bytes, key: int = 0) -> int:
 
 def launch_count() -> int:
     return int(load().oeqb_launch_count())
+
+
+def launched_kernels() -> set:
+    """Names of the specialised kernels launched since ``set_option("record", "1")``."""
+    lib = load()
+    need = c_size_t(0)
+    check(lib.oeqb_launched_kernels(None, 0, ctypes.byref(need)), "oeqb_launched_kernels")
+    buf = ctypes.create_string_buffer(need.value)
+    check(lib.oeqb_launched_kernels(buf, need.value, ctypes.byref(need)), "oeqb_launched_kernels")
+    return set(buf.value.decode().split())
 
 
 def set_option(name: str, value: str):

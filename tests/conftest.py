@@ -13,7 +13,9 @@ def pytest_configure(config):
 
 
 def pytest_collection_modifyitems(config, items):
-    """GPU tests are skipped, not failed, when no device is visible (the CPU suite runs with -m 'not gpu')."""
+    """GPU tests are skipped, not failed, when no device is visible (the CPU suite runs with -m 'not gpu').  The test that reads a
+    profiler's trace runs first: in a process some minutes old the profiler's clock is so far from the device's that it drops kernels."""
+    items.sort(key=lambda item: "kernels_are_named_by_pass" not in item.nodeid)
     try:
         import torch
         has_gpu = torch.cuda.is_available()

@@ -102,15 +102,14 @@ def small_graph(n_nodes=40, mean_degree=6.0, seed=3, isolated=(5, 17)):
 
 
 def kernels_launched(call):
-    """``call()``'s result and the names of the kernels that ran in it.  (The profiler drops kernels that its clock puts before the
-    record's start, and minutes into a process that clock is some milliseconds behind: the call waits for it, and is made twice.)"""
-    import time
-
+    """``call()``'s result and the names of this library's specialised kernels that it launched, from the library's own record: a profiler
+    drops kernels when its clock and the device's differ."""
     import torch
-    from torch.profiler import ProfilerActivity, profile
-    with profile(activities=[ProfilerActivity.CUDA]) as record:
-        time.sleep(0.1)
-        for _ in range(2):
-            result = call()
-            torch.cuda.synchronize()
-    return result, {e.key for e in record.key_averages()}
+    from openequivariance_b200 import native
+    native.set_option("record", "1")
+    try:
+        result = call()
+        torch.cuda.synchronize()
+        return result, native.launched_kernels()
+    finally:
+        native.set_option("record", "0")

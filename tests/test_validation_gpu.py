@@ -157,7 +157,6 @@ def test_kernels_are_named_by_pass():
     """Profiler trace of forward + backward + double backward issued on a side stream: the kernels of this library show
     up with names that carry ``forward`` / ``backward`` / ``double_backward`` (the substrings the reference's timing
     helper and stream test select kernels by: core/utils.py:174-203, tests/stream_test.py:97-391)."""
-    import time
     from torch.profiler import ProfilerActivity, profile
     import openequivariance_b200 as oeq
     p = MATRIX["mace_medium"]
@@ -177,7 +176,6 @@ def test_kernels_are_named_by_pass():
     side.synchronize()
     try:
         with profile(activities=[ProfilerActivity.CUDA, ProfilerActivity.CPU]) as prof:
-            time.sleep(0.1)      # (the profiler's clock lags in a long process: it drops kernels that seem to precede the record)
             with torch.cuda.stream(side):
                 run()
             side.synchronize()
