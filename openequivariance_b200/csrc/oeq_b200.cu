@@ -786,6 +786,20 @@ std::shared_ptr<const TcPlan> make_tc_plan(const Desc& d, int mode) {
     return plan;
 }
 
+// Index tables of a tensor-core program: in constant memory where they fit it (64 KB a program; a weight gradient with 512 weight tiles of 128
+// channels passes that), else in global memory.
+std::string emit_tables(const std::vector<std::pair<const char*, std::vector<long long>>>& tables) {
+    size_t words = 0;
+    for (auto& t : tables) words += std::max<size_t>(t.second.size(), 1);
+    std::ostringstream s;
+    for (auto& t : tables) {
+        s << (words <= 15000 ? "__constant__ int " : "__device__ const int ") << t.first << "[" << std::max<size_t>(t.second.size(), 1) << "] = {";
+        for (long long v : t.second) s << v << ", ";
+        s << "};\n";
+    }
+    return s.str();
+}
+
 // Sets, tables and straight-line sums of the tensor-core kernels of mode 0 and 1 (kernels/uvw_tc.cuh).
 std::string emit_tc(const Desc& d, int mode, bool parts) {
     std::ostringstream s;
@@ -797,12 +811,6 @@ std::string emit_tc(const Desc& d, int mode, bool parts) {
       << (mode == 0 ? "oeq_uvw_tc_forward" : "oeq_uvw_tc_backward_dx") << (parts ? "_parts\n" : "\n");
     s << "constexpr int TC_OUT_DIM = " << d.dim[mode == 0 ? 2 : 0] << ", TC_TW = " << p.tw << ", TC_NSUB = " << p.nsub << ", TC_MAXD = " << p.maxd
       << ", TC_NXS = " << p.nxs << ", TC_NCOARSE = " << p.ncoarse << ", TC_MAX_PARTS = " << kTcMaxParts << ";\nconstexpr size_t TC_SMEM_BYTES = " << p.smem << ";\n";
-    auto ilist = [&](const char* name, const std::vector<long long>& v) {
-        s << "__constant__ int " << name << "[" << (v.empty() ? 1 : v.size()) << "] = {";
-        for (size_t i = 0; i < v.size(); ++i) s << v[i] << (i + 1 < v.size() ? ", " : "");
-        if (v.empty()) s << "0";
-        s << "};\n";
-    };
     std::vector<long long> iset, iwc, sv, scode, soff, vd, voff, vnu, vnsub, vw, vws;
     size_t maxnb = 1;
     for (auto& i : p.inst) { iset.push_back(i.first); iwc.push_back(i.second); }
@@ -836,9 +844,8 @@ std::string emit_tc(const Desc& d, int mode, bool parts) {
         }
     }
     sv.push_back((long long)vd.size());
-    ilist("TC_SET_CODE", scode); ilist("TC_SET_OFF", soff);
-    ilist("TC_INST_SET", iset); ilist("TC_INST_WC", iwc); ilist("TC_SET_V", sv);
-    ilist("TC_V_D", vd); ilist("TC_V_OFF", voff); ilist("TC_V_NU", vnu); ilist("TC_V_NSUB", vnsub); ilist("TC_V_W", vw); ilist("TC_V_WS", vws);
+    s << emit_tables({{"TC_SET_CODE", scode}, {"TC_SET_OFF", soff}, {"TC_INST_SET", iset}, {"TC_INST_WC", iwc}, {"TC_SET_V", sv}, {"TC_V_D", vd},
+                      {"TC_V_OFF", voff}, {"TC_V_NU", vnu}, {"TC_V_NSUB", vnsub}, {"TC_V_W", vw}, {"TC_V_WS", vws}});
     return s.str();
 }
 
@@ -901,12 +908,6 @@ std::string emit_tc_dw(const Desc& d) {
     const std::vector<TcSub> subs = tc_subpaths(d);
     int boxes, pairs, maxd = 1;
     const size_t smem = tc_dw_smem_of(d, groups, &boxes, &pairs);
-    auto ilist = [&](const char* name, const std::vector<long long>& v) {
-        s << "__constant__ int " << name << "[" << (v.empty() ? 1 : v.size()) << "] = {";
-        for (size_t i = 0; i < v.size(); ++i) s << v[i] << (i + 1 < v.size() ? ", " : "");
-        if (v.empty()) s << "0";
-        s << "};\n";
-    };
     std::vector<long long> d3s, d1s, box0, gbox0, nbox, box, woff, cell, pair0, cy0, pj;
     std::vector<double> pc;
     int terms = 1, npairs = 0;
@@ -960,8 +961,8 @@ std::string emit_tc_dw(const Desc& d) {
     cy0.push_back(npairs);
     s << "constexpr int TCW_BOXES = " << boxes << ", TCW_PAIRS = " << pairs << ", TCW_MAXD = " << maxd << ", TCW_TERMS = " << terms << ", TC_MAX_PARTS = " << kTcMaxParts
       << ";\nconstexpr size_t TC_SMEM_BYTES = " << smem << ";\n";
-    ilist("TCW_D3", d3s); ilist("TCW_D1", d1s); ilist("TCW_BOX0", box0); ilist("TCW_GBOX0", gbox0); ilist("TCW_NBOX", nbox); ilist("TCW_BOX", box);
-    ilist("TCW_WOFF", woff); ilist("TCW_CELL", cell); ilist("TCW_PAIR0", pair0); ilist("TCW_CY0", cy0);
+    s << emit_tables({{"TCW_D3", d3s}, {"TCW_D1", d1s}, {"TCW_BOX0", box0}, {"TCW_GBOX0", gbox0}, {"TCW_NBOX", nbox}, {"TCW_BOX", box}, {"TCW_WOFF", woff},
+                      {"TCW_CELL", cell}, {"TCW_PAIR0", pair0}, {"TCW_CY0", cy0}});
     s << "__device__ const int TCW_PJ[" << std::max<size_t>(pj.size(), 1) << "] = {";
     for (size_t i = 0; i < pj.size(); ++i) s << pj[i] << ", ";
     s << "};\n__device__ const float TCW_PC[" << std::max<size_t>(pc.size(), 1) << "] = {";

@@ -37,3 +37,25 @@ def test_weights_at_any_address_and_batches_between(batch):
         found.append([z, *torch.ops.libtorch_tp_jit.jit_tp_backward(tp.kernel, tp.hash, *args)])
     for a, b, bound in zip(*found, (1e-6, 1e-6, 1e-6, 4e-6)):     # (dW: sums of 64 items in the tensor cores, which truncate)
         assert float((a.double() - b).norm() / b.norm()) <= bound
+
+
+def test_weight_gradient_of_a_product_whose_tables_pass_constant_memory():
+    """512 weight tiles or more: the weight-gradient kernel reads its tables from global memory, in several launches of 16 groups."""
+    import numpy as np
+    import torch
+
+    import openequivariance_b200 as oeq
+    from helpers import kernels_launched, rel_l2, uniform_inputs
+    from openequivariance_b200.core import problems as P
+    from oracle import tp_oracle
+    feats = "128x0e+128x0o+128x1e+128x1o+128x2e+128x2o"
+    p = P.FullyConnectedTPProblem(feats, "1x0e+1x1o+1x2e+1x3o", feats, shared_weights=True, irrep_dtype=np.float32, weight_dtype=np.float32)
+    tp = oeq.TensorProduct(p)
+    x, y, w, g, *_ = uniform_inputs(p, 65)
+    args = [torch.tensor(t, device="cuda") for t in (x, y, w, g)]
+    got, ran = kernels_launched(lambda: torch.ops.libtorch_tp_jit.jit_tp_backward(tp.kernel, tp.hash, *args))
+    assert "oeq_uvw_tc_backward_dw" in ran
+    want = list(tp_oracle.backward(p, x, y, tp.reorder_weights_to_e3nn(w), g))
+    want[2] = tp.reorder_weights_from_e3nn(want[2])
+    for a, b in zip(got, want):
+        assert rel_l2(a.cpu().numpy(), b) <= 1e-5
