@@ -940,7 +940,8 @@ std::string emit_tc_dw(const Desc& d) {
                             c.push_back(pr.i);
                             for (int e = 0; e < terms; ++e) {
                                 const bool real = e < (int)pr.terms.size();
-                                pj.push_back(real ? d.L[1][I->b].off + pr.terms[e].j : 0);
+                                // (padded with a harmonic that the pair has: one that is not finite stays in the pairs that it is part of)
+                                pj.push_back(d.L[1][I->b].off + pr.terms[real ? e : 0].j);
                                 pc.push_back(real ? pr.terms[e].c : 0.0);
                             }
                             ++np;

@@ -59,3 +59,31 @@ def test_weight_gradient_of_a_product_whose_tables_pass_constant_memory():
     want[2] = tp.reorder_weights_from_e3nn(want[2])
     for a, b in zip(got, want):
         assert rel_l2(a.cpu().numpy(), b) <= 1e-5
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_a_harmonic_that_is_not_finite_stays_in_its_paths(bad):
+    import torch
+
+    import openequivariance_b200 as oeq
+    p = shared_problem(False)
+    tp = oeq.TensorProduct(p)
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    x, y, w, g = (torch.randn(*n, device="cuda", generator=gen) for n in
+                  ((70, p.irreps_in1.dim), (70, p.irreps_in2.dim), (p.weight_numel,), (70, p.irreps_out.dim)))
+
+    def of(first):
+        y[33, 0] = first
+        z = torch.ops.libtorch_tp_jit.jit_tp_forward(tp.kernel, tp.hash, x, y, w, p.irreps_out.dim)
+        return z, *torch.ops.libtorch_tp_jit.jit_tp_backward(tp.kernel, tp.hash, x, y, w, g)
+    (z, dx, dy, dw), (_, _, _, dw0) = of(bad), of(0.0)
+    others = torch.arange(70, device="cuda") != 33
+    assert all(t[others].isfinite().all() and not t[33].isfinite().all() for t in (z, dx)) and dy.isfinite().all()
+    at = 0
+    for ins in p.instructions:
+        n = int(torch.tensor(ins.path_shape).prod())
+        path, path0, at = dw[at:at + n], dw0[at:at + n], at + n
+        if ins.i_in2 == 0:
+            assert not path.isfinite().any()
+        else:
+            assert torch.equal(path, path0)
