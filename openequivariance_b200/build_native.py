@@ -16,7 +16,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(CSRC, "liboeq_b200.so")
 STAMP = LIB + ".srchash"
-EMBED = {"K_COMMON": "common.cuh", "K_GENERIC": "generic_tp.cuh", "K_FAST_UVU": "fast_uvu.cuh",
+EMBED = {"K_COMMON": "common.cuh", "K_GENERIC": "generic_tp.cuh", "K_DW_REDUCE": "dw_reduce.cuh", "K_FAST_UVU": "fast_uvu.cuh",
          "K_UVW_TC": "uvw_tc.cuh", "K_UVW_ITEM": "uvw_item.cuh", "K_UVW_F64": "uvw_f64.cuh", "K_SYM_POLY": "sym_poly.cuh"}
 
 

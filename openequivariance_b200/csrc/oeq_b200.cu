@@ -990,12 +990,13 @@ enum Family {
     FAM_UVW_TC_PARTS, FAM_UVW_TC_DX_PARTS,                       // forward and gradients of x and y with a tile dealt to several CTAs
     FAM_UVW_ITEM,                                                // 'uvw' with a weight row per item
     FAM_UVW_F64,                                                 // 'uvw' in doubles on the FP64 matrix instruction
+    FAM_DW_REDUCE,                                               // rows of partial sums -> gradient of shared weights
     FAM_COUNT
 };
 const char* const kFamilyNames[FAM_COUNT] = {"generic", "fast_fwd_tp", "fast_fwd_det", "fast_fwd_atomic", "fast_bwd_tp",
                                              "fast_bwd_det", "fast_bwd_atomic", "fast_scatter", "fast_bwd2_tp",
                                              "fast_bwd2_det", "fast_bwd2_atomic", "uvw_tc", "fast_fwd3_tp", "fast_fwd3_det",
-                                             "uvw_tc_dx", "uvw_tc_dw", "uvw_tc_parts", "uvw_tc_dx_parts", "uvw_item", "uvw_f64"};
+                                             "uvw_tc_dx", "uvw_tc_dw", "uvw_tc_parts", "uvw_tc_dx_parts", "uvw_item", "uvw_f64", "dw_reduce"};
 const char* family_name(int f) { return (f >= 0 && f < FAM_COUNT) ? kFamilyNames[f] : "?"; }
 int family_from_name(const std::string& n) {
     for (int f = 0; f < FAM_COUNT; ++f)
@@ -1031,6 +1032,7 @@ size_t item_row_bytes(const Desc& d) {
 }
 
 std::string family_source(const Desc& d, const std::string& header, int fam, bool allow_streams = true) {
+    if (fam == FAM_DW_REDUCE) return std::string("typedef ") + (d.dtype == 2 ? "double" : "float") + " T;\nconstexpr int WN = " + std::to_string(d.wn) + ";\n" + K_DW_REDUCE;
     std::string src = header;
     if (fam == FAM_GENERIC) {
         src += K_COMMON;
@@ -1335,6 +1337,16 @@ int generic_forward(Entry* e, FwdParams p, cudaStream_t st) {
 
 int keep_pool_memory();
 
+// dW (+)= the rows of partial sums, in order
+int dw_reduce(Entry* e, const void* part, long long rows, void* dW, int accum, cudaStream_t st) {
+    Program* prog;
+    cudaKernel_t k;
+    if (int rc = get_program(e, FAM_DW_REDUCE, &prog)) return rc;
+    if (int rc = get_kernel(prog, "oeq_generic_dw_reduce", 0, &k)) return rc;
+    void* args[] = {&part, &rows, &dW, &accum};
+    return launch(k, (unsigned)((e->d.wn + 31) / 32), 256, 0, args, st);
+}
+
 int generic_backward(Entry* e, BwdParams p, cudaStream_t st) {
     if (p.n_units <= 0) return OEQB_OK;
     Program* prog;
@@ -1348,9 +1360,8 @@ int generic_backward(Entry* e, BwdParams p, cudaStream_t st) {
         const Desc& d = e->d;
         if (p.unit_mode == UNIT_ITEM && !p.accum)
             CUDA_TRY(cudaMemsetAsync(p.dx, 0, (size_t)p.n_edges * d.dim[0] * d.elt(), st));
-        cudaKernel_t ks, kr;
+        cudaKernel_t ks;
         if ((rc = get_kernel(prog, "oeq_generic_backward_shared", 0, &ks))) return rc;
-        if ((rc = get_kernel(prog, "oeq_generic_dw_reduce", 0, &kr))) return rc;
         int chunk = 32;
         long long chunks = (p.n_edges + chunk - 1) / chunk;
         void* part = nullptr;
@@ -1359,12 +1370,8 @@ int generic_backward(Entry* e, BwdParams p, cudaStream_t st) {
         p.dW_part = part;
         void* args[] = {&p, &chunk};
         rc = launch(ks, generic_grid(chunks), 128, 0, args, st);
-        if (!rc) {
-            // the entry points zero dW before the first pass, so the reduce always adds to what is there
-            int accum = 1;
-            void* rargs[] = {&part, &chunks, &p.dW, &accum};
-            rc = launch(kr, (unsigned)((d.wn + 31) / 32), 256, 0, rargs, st);
-        }
+        // the entry points zero dW before the first pass, so the reduce always adds to what is there
+        if (!rc) rc = dw_reduce(e, part, chunks, p.dW, 1, st);
         cudaFreeAsync(part, st);
         return rc;
     }
@@ -1448,10 +1455,6 @@ int f64_backward(Entry* e, const void* x, const void* y_dx, const void* y_dw, co
     F64BwdParams p{x, y_dx, W, g, dx, dy, batch, accum};
     int rc = f64_launch(e, "oeq_uvw_f64_backward", dim3((unsigned)((batch + 7) / 8)), &p, st);
     if (rc) return rc;
-    Program* gen;
-    if ((rc = get_program(e, FAM_GENERIC, &gen))) return rc;
-    cudaKernel_t kr;
-    if ((rc = get_kernel(gen, "oeq_generic_dw_reduce", 0, &kr))) return rc;
     // Items per row of partial sums, by the batch alone (so results do not depend on the device): about 80 rows keep the chip
     // busy with few paths, and a row costs wn doubles written and read once.
     int chunk = (int)std::min<long long>(std::max<long long>((batch + 79) / 80, 16), 4096);
@@ -1462,11 +1465,7 @@ int f64_backward(Entry* e, const void* x, const void* y_dx, const void* y_dw, co
     CUDA_TRY(cudaMallocAsync(&part, (size_t)chunks * d.wn * sizeof(double), st));
     F64DwParams q{x, y_dw, g, part, batch, chunk};
     rc = f64_launch(e, "oeq_uvw_f64_backward_dw", dim3((unsigned)chunks, (unsigned)((d.f64mm + 3) / 4)), &q, st);
-    if (!rc) {
-        int add = 1;
-        void* rargs[] = {&part, &chunks, &dW, &add};
-        rc = launch(kr, (unsigned)((d.wn + 31) / 32), 256, 0, rargs, st);
-    }
+    if (!rc) rc = dw_reduce(e, part, chunks, dW, 1, st);
     cudaFreeAsync(part, st);
     return rc;
 }
@@ -1866,13 +1865,11 @@ int tc_backward_dw(Entry* e, const void* x, const void* y, const void* g, void* 
     TcDwParams p{{}, {}, y, nullptr, batch, nullptr, 1, {0}};
     if ((rc = encode_map(&p.x, x, batch, d.dim[0], 32, false)) || (rc = encode_map(&p.g, g, batch, d.dim[2], 32, false))) return rc;
     if ((rc = status_word(&p.status))) return rc;
-    Program *prog, *gen;
+    Program* prog;
     if ((rc = get_program(e, FAM_UVW_TC_DW, &prog))) return rc;
-    if ((rc = get_program(e, FAM_GENERIC, &gen))) return rc;
-    cudaKernel_t k, kr;
+    cudaKernel_t k;
     const size_t smem = d.tc_dw_smem;
     if ((rc = get_kernel(prog, "oeq_uvw_tc_backward_dw", smem, &k))) return rc;
-    if ((rc = get_kernel(gen, "oeq_generic_dw_reduce", 0, &kr))) return rc;
     long long tiles = (batch + 63) / 64;
     if ((rc = keep_pool_memory())) return rc;
     void* part = nullptr;
@@ -1896,10 +1893,7 @@ int tc_backward_dw(Entry* e, const void* x, const void* y, const void* g, void* 
         }
         rc = launch(k, (unsigned)std::min<long long>(sms, tiles * p.splits), 21 * 32, smem, args, st);   // TC_THREADS
     }
-    if (!rc) {
-        void* rargs[] = {&part, &tiles, &dW, &accum};
-        rc = launch(kr, (unsigned)((d.wn + 31) / 32), 256, 0, rargs, st);
-    }
+    if (!rc) rc = dw_reduce(e, part, tiles, dW, accum, st);
     cudaFreeAsync(part, st);
     return rc;
 }
@@ -2060,6 +2054,7 @@ int oeqb_precompile(const void* desc, size_t desc_len, int64_t key) {
         else if (fam >= FAM_UVW_TC_DX && fam <= FAM_UVW_TC_DX_PARTS) { if (!d.tc_bwd) continue; }
         else if (fam == FAM_UVW_ITEM) { if (!d.item) continue; }
         else if (fam == FAM_UVW_F64) { if (!d.f64mm) continue; }
+        else if (fam == FAM_DW_REDUCE) { if (!d.shared) continue; }
         else if (fam != FAM_GENERIC && !d.fast) continue;
         if (fam >= FAM_FAST_BWD2_TP && fam <= FAM_FAST_BWD2_ATOMIC && d.fast_S4 < 3) continue;
         if (fam == FAM_FAST_FWD_ATOMIC && d.fast_S3 < 2) continue;

@@ -32,3 +32,11 @@ def test_the_widest_products_compile(in1, in2, family, tmp_path):
     (tmp_path / "t.cu").write_text(native.emit_source(text.encode(), family))
     subprocess.run([NVCC, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-cubin", "-o", str(tmp_path / "t.cubin"), str(tmp_path / "t.cu")],
                    check=True, stdout=subprocess.DEVNULL)
+
+
+def test_the_sum_of_the_partial_rows_is_a_small_program():
+    """Every backward with shared weights needs it, and the general kernels take a minute and more to compile."""
+    text = _descriptor(_both(32, 2), "1x0e+1x1o+1x2e", _both(32, 2))
+    assert "oeq_generic_dw_reduce(" not in native.emit_source(text.encode(), "generic")
+    source = native.emit_source(text.encode(), "dw_reduce")
+    assert "oeq_generic_dw_reduce(" in source and len(source) < 4000
