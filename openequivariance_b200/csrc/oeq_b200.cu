@@ -1777,8 +1777,17 @@ int encode_map(CUtensorMap* map, const void* data, long long rows, long long col
     }
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)cols * 4};
     const cuuint32_t box[2] = {32, box_rows}, step[2] = {1, 1};
-    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(data), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              swizzled ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    auto run = [&] {
+        return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(data), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                      swizzled ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult r = run();
+    if (r == CUDA_ERROR_INVALID_CONTEXT) {   // the thread's first use of the device: the runtime's context is not current yet
+        int dev = 0;
+        CUDA_TRY(cudaGetDevice(&dev));
+        CUDA_TRY(cudaSetDevice(dev));
+        r = run();
+    }
     if (r != CUDA_SUCCESS) return fail(OEQB_ECUDA, "cuTensorMapEncodeTiled(%lld x %lld) failed: %d", rows, cols, (int)r);
     return OEQB_OK;
 }

@@ -87,3 +87,30 @@ def test_a_harmonic_that_is_not_finite_stays_in_its_paths(bad):
             assert not path.isfinite().any()
         else:
             assert torch.equal(path, path0)
+
+
+def test_a_thread_whose_first_use_of_the_device_is_a_product():
+    """(Its outputs come from memory that torch keeps: nothing else has made a context current in the thread.)"""
+    import threading
+
+    import torch
+
+    import openequivariance_b200 as oeq
+    p = shared_problem(False)
+    tp = oeq.TensorProduct(p)
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    x, y, w, g = (torch.randn(*n, device="cuda", generator=gen) for n in
+                  ((70, p.irreps_in1.dim), (70, p.irreps_in2.dim), (p.weight_numel,), (70, p.irreps_out.dim)))
+    found = []
+
+    def call():
+        found.append(torch.ops.libtorch_tp_jit.jit_tp_forward(tp.kernel, tp.hash, x, y, w, p.irreps_out.dim))
+    call()
+    want = found.pop().clone()
+    for backward in (False, True):
+        torch.ops.libtorch_tp_jit.jit_tp_backward(tp.kernel, tp.hash, x, y, w, g)     # (compiled; its memory is free again)
+        target = call if not backward else lambda: found.append(torch.ops.libtorch_tp_jit.jit_tp_backward(tp.kernel, tp.hash, x, y, w, g))
+        thread = threading.Thread(target=target)
+        thread.start()
+        thread.join()
+    assert len(found) == 2 and torch.equal(found[0], want) and all(t.isfinite().all() for t in found[1])
