@@ -134,7 +134,6 @@ struct TcParams {
     long long batch;
     int accum;          // add to what dst (and dy, when there is one part) holds instead of overwriting it
     int* status;
-    int inst0;          // first instance of the list that is walked
     int parts;          // a tile's instances are shared by this many CTAs: part s takes cut[s] .. cut[s + 1] of the list
     int cut[TC_MAX_PARTS + 1];
 };
@@ -196,28 +195,29 @@ OEQ_DEV float tc_half(TcPair v, int h) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
     return h ? b : a;
 }
-// What the sets' code (emitted with the tables) is made of: sums += c * products, and a dot product over the thread's channels.
-struct TcMath {
-    static constexpr int H = TC_CH / 2;
-    typedef TcPair P;
-    static OEQ_DEV void axpy(float c, const P (&u)[H], P* z) {
-        const P cc = tc_pack(c, c);
-#pragma unroll
-        for (int q = 0; q < H; ++q) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(z[q]) : "l"(cc), "l"(u[q]));
-    }
-    static OEQ_DEV float dot(const P* x, const P (&u)[H]) {
-        P s0, s1;
-        asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(s0) : "l"(x[0]), "l"(u[0]));
-        asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(s1) : "l"(x[1]), "l"(u[1]));
-#pragma unroll
-        for (int q = 2; q < H; q += 2) {
-            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(s0) : "l"(x[q]), "l"(u[q]));
-            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(s1) : "l"(x[q + 1]), "l"(u[q + 1]));
-        }
-        asm("add.rn.f32x2 %0, %0, %1;" : "+l"(s0) : "l"(s1));
-        return tc_half(s0, 0) + tc_half(s0, 1);
-    }
-};
+// What the sets' code (emitted) is made of: sums += c * products, and a dot product over the thread's channels.  One statement each: the
+// compiler's time goes with their number.
+constexpr int TC_H = TC_CH / 2;
+OEQ_DEV void tc_axpy(float c, const TcPair (&u)[TC_H], TcPair* z) {
+    if constexpr (TC_H == 4)
+        asm("{ .reg .b64 c; mov.b64 c, {%4, %4}; fma.rn.f32x2 %0, c, %5, %0; fma.rn.f32x2 %1, c, %6, %1; fma.rn.f32x2 %2, c, %7, %2; fma.rn.f32x2 %3, c, %8, %3; }"
+            : "+&l"(z[0]), "+&l"(z[1]), "+&l"(z[2]), "+&l"(z[3]) : "f"(c), "l"(u[0]), "l"(u[1]), "l"(u[2]), "l"(u[3]));
+    else
+        asm("{ .reg .b64 c; mov.b64 c, {%8, %8}; fma.rn.f32x2 %0, c, %9, %0; fma.rn.f32x2 %1, c, %10, %1; fma.rn.f32x2 %2, c, %11, %2; fma.rn.f32x2 %3, c, %12, %3;\n"
+            "  fma.rn.f32x2 %4, c, %13, %4; fma.rn.f32x2 %5, c, %14, %5; fma.rn.f32x2 %6, c, %15, %6; fma.rn.f32x2 %7, c, %16, %7; }"
+            : "+&l"(z[0]), "+&l"(z[1]), "+&l"(z[2]), "+&l"(z[3]), "+&l"(z[4]), "+&l"(z[5]), "+&l"(z[6]), "+&l"(z[7])
+            : "f"(c), "l"(u[0]), "l"(u[1]), "l"(u[2]), "l"(u[3]), "l"(u[4]), "l"(u[5]), "l"(u[6]), "l"(u[7]));
+}
+#if TC_MODE == 1
+static_assert(TC_H == 4, "channels of a thread");
+OEQ_DEV float tc_dot(const TcPair* x, const TcPair (&u)[TC_H]) {
+    float s;
+    asm("{ .reg .b64 a, b; .reg .f32 f, g; mul.rn.f32x2 a, %1, %5; mul.rn.f32x2 b, %2, %6; fma.rn.f32x2 a, %3, %7, a; fma.rn.f32x2 b, %4, %8, b;\n"
+        "  add.rn.f32x2 a, a, b; mov.b64 {f, g}, a; add.rn.f32 %0, f, g; }"
+        : "=f"(s) : "l"(x[0]), "l"(x[1]), "l"(x[2]), "l"(x[3]), "l"(u[0]), "l"(u[1]), "l"(u[2]), "l"(u[3]));
+    return s;
+}
+#endif
 
 // A thread's channels of a destination (or first-input) block are TC_CH * D consecutive floats of its item's row; component k of channels
 // 2 q, 2 q + 1 is v[k * TC_CH / 2 + q].  Global memory is read and written 8 floats of a row (a sector) at a time by two neighbouring lanes,
@@ -289,67 +289,40 @@ OEQ_DEV void tc_rows_store(float* rows, int live, const TcPair* v, int lane, boo
     }
 }
 
-// One set of one tile for a summing warp: `live` items from row0 on, channels col .. col + TC_CH of every destination tile.  C: the set's code
-// (sets that differ only in where their blocks and weights lie share it: the two parities do).
-template <int C>
-OEQ_DEV bool tc_sum_set(const TcParams& p, TcShared& sh, const int set, const unsigned tmem, unsigned& nd, float (&y)[L2_DIM], float (&dy)[TC_MODE == 1 ? L2_DIM : 1],
-                        const long long row0, const int live, const int col, const int lane) {
-    using Set = TcSet<C>;
-    TcPair z[Set::SUMD * TC_CH / 2];
-    TcPair xv[TC_MODE == 1 ? Set::SUMD * TC_CH / 2 : 1];
-    if constexpr (TC_MODE == 1)
-        static_for<0, Set::NB>([&](auto bc) {
-            using B = TcBlk<C, decltype(bc)::value>;
-            tc_rows_load<B::D>(p.x + row0 * TC_OUT_DIM + TC_SET_OFF[set * TC_MAXNB + decltype(bc)::value] + col * B::D, live, xv + B::AT * (TC_CH / 2), lane);
-        });
+// A step of a summing warp: wait for the products of a chunk, number nd, ...
+OEQ_DEV bool tc_step(TcShared& sh, unsigned nd, float (&y)[L2_DIM]) {
+    const bool ok = tc_warp_wait(&sh.d_full[nd & 1u], (nd >> 1) & 1u, &sh.abort_flag);
+    // (coefficients of other steps are not kept for this one: as common subexpressions they spilled 70 registers)
 #pragma unroll
-    for (int k = 0; k < Set::SUMD * TC_CH / 2; ++k) z[k] = 0;
-    bool ok = true;
-    static_for<0, Set::NV>([&](auto vc) {
-        constexpr int V = decltype(vc)::value;
-        using Vis = TcVis<C, V>;
-#pragma unroll 1
-        for (int uc = 0; uc < Vis::NU; ++uc)
-            static_for<0, Vis::D>([&](auto ic) {
-                constexpr int I = decltype(ic)::value;
-                const unsigned buf = nd & 1u;
-                if (ok) ok = tc_warp_wait(&sh.d_full[buf], (nd >> 1) & 1u, &sh.abort_flag);
-                if (!ok) return;
-                // (coefficients of other steps are not kept for this one: as common subexpressions they spilled 70 registers)
-#pragma unroll
-                for (int j = 0; j < L2_DIM; ++j) asm volatile("" : "+f"(y[j]));
-                tc_fence_after();
-                const unsigned t = tmem + buf * TC_DW;
-                static_for<0, Vis::NSUB>([&](auto sc) {
-                    constexpr int Q = decltype(sc)::value;
-                    float u[TC_CH];
-                    tc_ld(t + Q * TC_TW, u);
-                    tc_ld_wait(u);
-                    TcPair up[TC_CH / 2];
-#pragma unroll
-                    for (int q = 0; q < TC_CH / 2; ++q) up[q] = tc_pack(u[2 * q], u[2 * q + 1]);
-                    if constexpr (Q + 1 == Vis::NSUB) {
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) tc_mbar_arrive(&sh.d_empty[buf]);
-                    }
-                    TcFold<C, V, Q>::template run<I, TcMath>(up, y, z, xv, dy);
-                });
-                ++nd;
-            });
-    });
-    if (!ok) return false;
-    static_for<0, Set::NB>([&](auto bc) {
-        using B = TcBlk<C, decltype(bc)::value>;
-        tc_rows_store<B::D>(p.dst + row0 * TC_OUT_DIM + TC_SET_OFF[set * TC_MAXNB + decltype(bc)::value] + col * B::D, live, z + B::AT * (TC_CH / 2), lane, p.accum != 0);
-    });
-    return true;
+    for (int j = 0; j < L2_DIM; ++j) asm volatile("" : "+f"(y[j]));
+    tc_fence_after();
+    return ok;
 }
+// ... take those of one weight tile ...
+OEQ_DEV void tc_products(unsigned taddr, TcPair (&u)[TC_H]) {
+    float v[TC_CH];
+    tc_ld(taddr, v);
+    tc_ld_wait(v);
+#pragma unroll
+    for (int q = 0; q < TC_H; ++q) u[q] = tc_pack(v[2 * q], v[2 * q + 1]);
+}
+// ... and give the accumulator back.
+OEQ_DEV void tc_step_done(TcShared& sh, unsigned nd, int lane) {
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) tc_mbar_arrive(&sh.d_empty[nd & 1u]);
+}
+// One set of one tile for a summing warp: `live` items from row0 on, channels col .. col + TC_CH of every destination tile.  Sets that differ only
+// in where their blocks and weights lie share their code (the two parities do).  The functions are emitted (emit_tc_sets):
+//   bool tc_set_<code>(TC_SET_ARGS) for each code, bool tc_sum_set(code, TC_SET_ARGS)
+#define TC_SET_ARGS const TcParams& p, TcShared& sh, const int set, const unsigned tmem, unsigned& nd, float (&y)[L2_DIM], float (&dy)[TC_MODE == 1 ? L2_DIM : 1], \
+                    const long long row0, const int live, const int col, const int lane
+#define TC_SET_PASS p, sh, set, tmem, nd, y, dy, row0, live, col, lane
+//@ sets
 
-// PARTS: a tile's instances, of the large sets or of those with one destination tile each (p.inst0), are dealt to p.parts CTAs; otherwise a CTA walks
-// the large sets of a tile in turn.
-template <bool PARTS>
-OEQ_DEV void tc_kernel(const TcParams& p) {
+// A program holds the large sets of the problem, which a CTA walks in turn, or (TC_PARTS) the large sets or those of one destination tile each, whose
+// instances are dealt to p.parts CTAs.
+extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const __grid_constant__ TcParams p) {
     extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
     TcShared& sh = *reinterpret_cast<TcShared*>(tc_smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -372,7 +345,7 @@ OEQ_DEV void tc_kernel(const TcParams& p) {
     __syncthreads();
     tc_fence_after();
     const unsigned tmem = sh.tmem_base, tmem_a = tmem + 2 * TC_DW;
-    const int parts = PARTS ? p.parts : 1;
+    const int parts = TC_PARTS ? p.parts : 1;
     const long long nunits = (p.batch + 127) / 128 * parts;
     // Every role walks the same list: units of this CTA, instances of the unit's part, visits of the instance's set, 32-channel chunks of the
     // visit's block.  f(tile, visit, chunk of the source block, tile of the destination) returns false to leave.
@@ -381,7 +354,7 @@ OEQ_DEV void tc_kernel(const TcParams& p) {
         for (long long unit = blockIdx.x; unit < nunits; unit += gridDim.x) {
             const long long tile = unit / parts;
             const int part = (int)(unit % parts);
-            const int n0 = PARTS ? p.inst0 + p.cut[part] : 0, n1 = PARTS ? p.inst0 + p.cut[part + 1] : TC_NCOARSE;
+            const int n0 = TC_PARTS ? p.cut[part] : 0, n1 = TC_PARTS ? p.cut[part + 1] : TC_NINST;
 #pragma unroll 1
             for (int n = n0; n < n1; ++n) {
                 const int set = TC_INST_SET[n], wc = TC_INST_WC[n];
@@ -414,14 +387,11 @@ OEQ_DEV void tc_kernel(const TcParams& p) {
             for (int j = 0; j < L2_DIM; ++j) y[j] = __ldg(p.y + b * L2_DIM + j);
 #pragma unroll
             for (int j = 0; j < (TC_MODE == 1 ? L2_DIM : 1); ++j) dy[j] = 0.f;
-            const int n0 = PARTS ? p.inst0 + p.cut[part] : 0, n1 = PARTS ? p.inst0 + p.cut[part + 1] : TC_NCOARSE;
+            const int n0 = TC_PARTS ? p.cut[part] : 0, n1 = TC_PARTS ? p.cut[part + 1] : TC_NINST;
 #pragma unroll 1
             for (int n = n0; n < n1 && ok; ++n) {
                 const int set = TC_INST_SET[n], col = TC_INST_WC[n] * TC_TW + half * TC_CH;
-                const int code = TC_SET_CODE[set];
-                static_for<0, PARTS ? TC_NCODE : TC_NCCODE>([&](auto cc) {
-                    if (code == decltype(cc)::value) ok = tc_sum_set<decltype(cc)::value>(p, sh, set, t, nd, y, dy, rows > 0 ? row0 : 0, rows, col, lane);
-                });
+                ok = tc_sum_set(TC_SET_CODE[set], p, sh, set, t, nd, y, dy, rows > 0 ? row0 : 0, rows, col, lane);
             }
             if (TC_MODE == 1 && ok) {
                 // both halves of the channels: warps 4 to 7 pass theirs on
@@ -443,7 +413,7 @@ OEQ_DEV void tc_kernel(const TcParams& p) {
                         if (lane == 0) tc_mbar_arrive(&sh.dy_empty);
                         if (live) {
                             float* out = p.dy + (part * p.batch + b) * L2_DIM;
-                            const bool add = !PARTS && p.accum;
+                            const bool add = !TC_PARTS && p.accum;
 #pragma unroll
                             for (int j = 0; j < (TC_MODE == 1 ? L2_DIM : 1); ++j) out[j] = add ? out[j] + dy[j] : dy[j];
                         }
@@ -628,8 +598,6 @@ OEQ_DEV void tc_kernel(const TcParams& p) {
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
-// (a program of its own each: compiling one takes 5 to 15 seconds, and most callers need one)
-extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const __grid_constant__ TcParams p) { tc_kernel<TC_PARTS != 0>(p); }
 
 #if TC_MODE == 1 && TC_PARTS
 // dy[e] = (accum ? dy[e] : 0) + sum of the parts' rows, in order

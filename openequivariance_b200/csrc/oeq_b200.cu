@@ -647,30 +647,24 @@ std::string emit_tc_dw(const Desc& d);
 int tc_src(const Instr& I, int mode) { return mode == 0 ? I.a : I.o; }
 int tc_dst(const Instr& I, int mode) { return mode == 0 ? I.o : I.a; }
 
-// The sums of one instruction's products into a set: for every source component the (i, k) pairs that it is part of.
-std::string tc_fold_code(const Desc& d, const TcPlan::Set& t, int n, int mode) {
+// The sums of one instruction's products, component c of its source, into a set: a statement for every (i, k) pair that it is part of.
+std::string tc_fold_code(const Desc& d, const TcPlan::Set& t, int n, int mode, int c) {
     std::ostringstream s;
     const Instr& I = d.ins[n];
     const size_t slot = std::find(t.dest.begin(), t.dest.end(), tc_dst(I, mode)) - t.dest.begin();
-    const int yoff = d.L[1][I.b].off, nsrc = d.L[mode == 0 ? 0 : 2][tc_src(I, mode)].d();
-    s << "  template <int I, class M> static OEQ_DEV void run(const typename M::P (&u)[M::H], const float (&y)[L2_DIM], typename M::P* z, const typename M::P* x, float* dy) {\n";
-    for (int c = 0; c < nsrc; ++c) {
-        s << "    if constexpr (I == " << c << ") {\n";
-        for (auto& pr : ik_pairs(I)) {
-            if ((mode == 0 ? pr.i : pr.k) != c) continue;
-            const int at = t.at[slot] + (mode == 0 ? pr.k : pr.i);
-            s << "      { float c = float(" << hexf(pr.terms[0].c) << ") * y[" << yoff + pr.terms[0].j << "];";
-            for (size_t e = 1; e < pr.terms.size(); ++e) s << " c = fmaf(float(" << hexf(pr.terms[e].c) << "), y[" << yoff + pr.terms[e].j << "], c);";
-            s << " M::axpy(c, u, z + " << at << " * M::H);";
-            if (mode == 1) {
-                s << " const float t = M::dot(x + " << at << " * M::H, u);";
-                for (auto& e : pr.terms) s << " dy[" << yoff + e.j << "] = fmaf(float(" << hexf(e.c) << "), t, dy[" << yoff + e.j << "]);";
-            }
-            s << " }\n";
+    const int yoff = d.L[1][I.b].off;
+    for (auto& pr : ik_pairs(I)) {
+        if ((mode == 0 ? pr.i : pr.k) != c) continue;
+        const int at = t.at[slot] + (mode == 0 ? pr.k : pr.i);
+        s << "      { float c = float(" << hexf(pr.terms[0].c) << ") * y[" << yoff + pr.terms[0].j << "];";
+        for (size_t e = 1; e < pr.terms.size(); ++e) s << " c = fmaf(float(" << hexf(pr.terms[e].c) << "), y[" << yoff + pr.terms[e].j << "], c);";
+        s << " tc_axpy(c, u, z + " << at << " * TC_H);";
+        if (mode == 1) {
+            s << " const float t = tc_dot(x + " << at << " * TC_H, u);";
+            for (auto& e : pr.terms) s << " dy[" << yoff + e.j << "] = fmaf(float(" << hexf(e.c) << "), t, dy[" << yoff + e.j << "]);";
         }
-        s << "    }\n";
+        s << " }\n";
     }
-    s << "  }\n";
     return s.str();
 }
 
@@ -715,7 +709,10 @@ std::shared_ptr<const TcPlan> make_tc_plan(const Desc& d, int mode) {
         std::vector<std::pair<std::string, TcPlan::Visit>> coded;
         for (auto& v : s.visits) {
             std::vector<std::pair<std::string, int>> subs;
-            for (int n : v.ins) subs.push_back({tc_fold_code(d, s, n, mode), n});
+            for (int n : v.ins) {
+                subs.push_back({"", n});
+                for (int c = 0; c < S[v.src].d(); ++c) subs.back().first += std::to_string(c) + "\n" + tc_fold_code(d, s, n, mode, c);
+            }
             std::sort(subs.begin(), subs.end());
             std::ostringstream text;
             text << "D = " << S[v.src].d() << ", NU = " << S[v.src].mul / 32 << ", NSUB = " << subs.size() << "\n";
@@ -800,8 +797,9 @@ std::string emit_tables(const std::vector<std::pair<const char*, std::vector<lon
     return s.str();
 }
 
-// Sets, tables and straight-line sums of the tensor-core kernels of mode 0 and 1 (kernels/uvw_tc.cuh).
-std::string emit_tc(const Desc& d, int mode, bool parts) {
+// Tables of the tensor-core kernels of mode 0 and 1 (kernels/uvw_tc.cuh), for the large sets or for the small ones; parts: for tiles that are dealt to
+// several CTAs.
+std::string emit_tc(const Desc& d, int mode, bool small, bool parts) {
     std::ostringstream s;
     if (!d.tc || (mode != 0 && !d.tc_bwd)) { s << "#define OEQ_TC 0\n"; return s.str(); }
     if (mode == 3) return emit_tc_dw(d);
@@ -809,43 +807,73 @@ std::string emit_tc(const Desc& d, int mode, bool parts) {
     const std::vector<Block>&S = d.L[mode == 0 ? 0 : 2], &D = d.L[mode == 0 ? 2 : 0];
     s << "#define OEQ_TC 1\n#define TC_MODE " << mode << "\n#define TC_PARTS " << (parts ? 1 : 0) << "\n#define TC_KERNEL_NAME "
       << (mode == 0 ? "oeq_uvw_tc_forward" : "oeq_uvw_tc_backward_dx") << (parts ? "_parts\n" : "\n");
-    s << "constexpr int TC_OUT_DIM = " << d.dim[mode == 0 ? 2 : 0] << ", TC_TW = " << p.tw << ", TC_NSUB = " << p.nsub << ", TC_MAXD = " << p.maxd
-      << ", TC_NXS = " << p.nxs << ", TC_NCOARSE = " << p.ncoarse << ", TC_MAX_PARTS = " << kTcMaxParts << ";\nconstexpr size_t TC_SMEM_BYTES = " << p.smem << ";\n";
     std::vector<long long> iset, iwc, sv, scode, soff, vd, voff, vnu, vnsub, vw, vws;
     size_t maxnb = 1;
-    for (auto& i : p.inst) { iset.push_back(i.first); iwc.push_back(i.second); }
-    for (auto& t : p.sets) maxnb = std::max(maxnb, t.dest.size());
-    s << "constexpr int TC_MAXNB = " << maxnb << ", TC_NCCODE = " << p.ncode_coarse << ", TC_NCODE = " << p.codes.size() << ";\n";
-    s << "template <int C> struct TcSet;\ntemplate <int C, int B> struct TcBlk;\ntemplate <int C, int V> struct TcVis;\ntemplate <int C, int V, int Q> struct TcFold;\n";
-    int known = 0;
-    for (auto& t : p.sets) {
+    const size_t s0 = small ? p.ncset : 0, s1 = small ? p.sets.size() : p.ncset;
+    for (size_t n = small ? p.ncoarse : 0; n < (small ? p.inst.size() : p.ncoarse); ++n) { iset.push_back(p.inst[n].first - s0); iwc.push_back(p.inst[n].second); }
+    for (size_t k = s0; k < s1; ++k) maxnb = std::max(maxnb, p.sets[k].dest.size());
+    s << "constexpr int TC_OUT_DIM = " << d.dim[mode == 0 ? 2 : 0] << ", TC_TW = " << p.tw << ", TC_NSUB = " << p.nsub << ", TC_MAXD = " << p.maxd
+      << ", TC_NXS = " << p.nxs << ", TC_MAX_PARTS = " << kTcMaxParts << ", TC_MAXNB = " << maxnb << ", TC_NINST = " << iset.size() << ";\nconstexpr size_t TC_SMEM_BYTES = " << p.smem << ";\n";
+    for (size_t k = s0; k < s1; ++k) {
+        const TcPlan::Set& t = p.sets[k];
         sv.push_back((long long)vd.size());
         scode.push_back(t.code);
         for (size_t b = 0; b < maxnb; ++b) soff.push_back(b < t.dest.size() ? D[t.dest[b]].off : 0);
-        const bool fresh = t.code == known;
-        known += fresh;
-        if (fresh) {
-            s << "template <> struct TcSet<" << t.code << "> { static constexpr int SUMD = " << t.sumd << ", NB = " << t.dest.size() << ", NV = " << t.visits.size() << "; };\n";
-            for (size_t b = 0; b < t.dest.size(); ++b)
-                s << "template <> struct TcBlk<" << t.code << ", " << b << "> { static constexpr int D = " << D[t.dest[b]].d() << ", AT = " << t.at[b] << "; };\n";
-        }
-        for (size_t v = 0; v < t.visits.size(); ++v) {
-            const Block& A = S[t.visits[v].src];
-            const int nsub = (int)t.visits[v].ins.size();
+        for (auto& v : t.visits) {
+            const Block& A = S[v.src];
+            const int nsub = (int)v.ins.size();
             vd.push_back(A.d()); voff.push_back(A.off); vnu.push_back(A.mul / 32); vnsub.push_back(nsub);
-            if (fresh)
-                s << "template <> struct TcVis<" << t.code << ", " << v << "> { static constexpr int D = " << A.d() << ", NU = " << A.mul / 32 << ", NSUB = " << nsub << "; };\n";
             for (int q = 0; q < p.nsub; ++q) {
-                const Instr& I = d.ins[t.visits[v].ins[q < nsub ? q : 0]];
+                const Instr& I = d.ins[v.ins[q < nsub ? q : 0]];
                 vw.push_back(I.woff);
                 vws.push_back(32LL * d.L[2][I.o].mul);   // a weight tile row (32 channels of the first input) further on
-                if (q < nsub && fresh) s << "template <> struct TcFold<" << t.code << ", " << v << ", " << q << "> {\n" << tc_fold_code(d, t, t.visits[v].ins[q], mode) << "};\n";
             }
         }
     }
     sv.push_back((long long)vd.size());
     s << emit_tables({{"TC_SET_CODE", scode}, {"TC_SET_OFF", soff}, {"TC_INST_SET", iset}, {"TC_INST_WC", iwc}, {"TC_SET_V", sv}, {"TC_V_D", vd},
                       {"TC_V_OFF", voff}, {"TC_V_NU", vnu}, {"TC_V_NSUB", vnsub}, {"TC_V_W", vw}, {"TC_V_WS", vws}});
+    return s.str();
+}
+
+// The sets' sums: a function for each code, as text, because a compiler takes straight-line statements several times faster than the same
+// unrolled from templates (52 paths of 32 x 32 with l <= 3: 21 s, and 6 s).
+std::string emit_tc_sets(const Desc& d, int mode, bool small) {
+    std::ostringstream s;
+    const TcPlan& p = *d.tc_plan[mode];
+    const std::vector<Block>&S = d.L[mode == 0 ? 0 : 2], &D = d.L[mode == 0 ? 2 : 0];
+    std::vector<int> codes;
+    for (size_t k = small ? p.ncset : 0; k < (small ? p.sets.size() : p.ncset); ++k) {
+        const TcPlan::Set& t = p.sets[k];
+        if (std::count(codes.begin(), codes.end(), t.code)) continue;
+        codes.push_back(t.code);
+        s << "OEQ_DEV bool tc_set_" << t.code << "(TC_SET_ARGS) {\n  TcPair z[" << t.sumd << " * TC_H], x[TC_MODE == 1 ? " << t.sumd << " * TC_H : 1];\n";
+        auto rows = [&](const char* call, size_t b, const char* at, const char* v, const char* more) {
+            s << "  " << call << "<" << D[t.dest[b]].d() << ">(" << at << " + row0 * TC_OUT_DIM + TC_SET_OFF[set * TC_MAXNB + " << b << "] + col * " << D[t.dest[b]].d()
+              << ", live, " << v << " + " << t.at[b] << " * TC_H, lane" << more << ");\n";
+        };
+        if (mode == 1) for (size_t b = 0; b < t.dest.size(); ++b) rows("tc_rows_load", b, "p.x", "x", "");
+        s << "#pragma unroll\n  for (int k = 0; k < " << t.sumd << " * TC_H; ++k) z[k] = 0;\n  bool ok = true;\n  TcPair u[TC_H];\n";
+        for (auto& v : t.visits) {
+            s << "#pragma unroll 1\n  for (int uc = 0; uc < " << S[v.src].mul / 32 << "; ++uc) {\n";
+            for (int c = 0; c < S[v.src].d(); ++c) {
+                s << "    if (ok) ok = tc_step(sh, nd, y);\n    if (ok) {\n";
+                for (size_t q = 0; q < v.ins.size(); ++q) {
+                    s << "      tc_products(tmem + (nd & 1u) * TC_DW + " << q << " * TC_TW, u);\n";
+                    if (q + 1 == v.ins.size()) s << "      tc_step_done(sh, nd, lane);\n";
+                    s << tc_fold_code(d, t, v.ins[q], mode, c);
+                }
+                s << "      ++nd;\n    }\n";
+            }
+            s << "  }\n";
+        }
+        s << "  if (!ok) return false;\n";
+        for (size_t b = 0; b < t.dest.size(); ++b) rows("tc_rows_store", b, "p.dst", "z", ", p.accum != 0");
+        s << "  return true;\n}\n";
+    }
+    s << "OEQ_DEV bool tc_sum_set(const int code, TC_SET_ARGS) {\n  bool ok = true;\n";
+    for (int c : codes) s << "  if (code == " << c << ") ok = tc_set_" << c << "(TC_SET_PASS);\n";
+    s << "  return ok;\n}\n";
     return s.str();
 }
 
@@ -987,7 +1015,8 @@ enum Family {
     FAM_UVW_TC,                                                  // tcgen05 'uvw' forward
     FAM_FAST_FWD3_TP, FAM_FAST_FWD3_DET,                         // fused second-order forward (three terms in one pass)
     FAM_UVW_TC_DX, FAM_UVW_TC_DW,                                // tcgen05 'uvw' backward: gradients of x and y, of the weights
-    FAM_UVW_TC_PARTS, FAM_UVW_TC_DX_PARTS,                       // forward and gradients of x and y with a tile dealt to several CTAs
+    FAM_UVW_TC_PARTS, FAM_UVW_TC_DX_PARTS,                       // forward and gradients of x and y with a tile's large sets dealt to several CTAs
+    FAM_UVW_TC_SMALL, FAM_UVW_TC_DX_SMALL,                       // ... its small sets
     FAM_UVW_ITEM,                                                // 'uvw' with a weight row per item
     FAM_UVW_F64,                                                 // 'uvw' in doubles on the FP64 matrix instruction
     FAM_DW_REDUCE,                                               // rows of partial sums -> gradient of shared weights
@@ -996,7 +1025,7 @@ enum Family {
 const char* const kFamilyNames[FAM_COUNT] = {"generic", "fast_fwd_tp", "fast_fwd_det", "fast_fwd_atomic", "fast_bwd_tp",
                                              "fast_bwd_det", "fast_bwd_atomic", "fast_scatter", "fast_bwd2_tp",
                                              "fast_bwd2_det", "fast_bwd2_atomic", "uvw_tc", "fast_fwd3_tp", "fast_fwd3_det",
-                                             "uvw_tc_dx", "uvw_tc_dw", "uvw_tc_parts", "uvw_tc_dx_parts", "uvw_item", "uvw_f64", "dw_reduce"};
+                                             "uvw_tc_dx", "uvw_tc_dw", "uvw_tc_parts", "uvw_tc_dx_parts", "uvw_tc_small", "uvw_tc_dx_small", "uvw_item", "uvw_f64", "dw_reduce"};
 const char* family_name(int f) { return (f >= 0 && f < FAM_COUNT) ? kFamilyNames[f] : "?"; }
 int family_from_name(const std::string& n) {
     for (int f = 0; f < FAM_COUNT; ++f)
@@ -1044,10 +1073,16 @@ std::string family_source(const Desc& d, const std::string& header, int fam, boo
     } else if (fam == FAM_UVW_F64) {
         src += K_COMMON;
         src += K_UVW_F64;
-    } else if (fam == FAM_UVW_TC || (fam >= FAM_UVW_TC_DX && fam <= FAM_UVW_TC_DX_PARTS)) {
-        src += emit_tc(d, fam == FAM_UVW_TC_DW ? 3 : fam == FAM_UVW_TC_DX || fam == FAM_UVW_TC_DX_PARTS ? 1 : 0, fam >= FAM_UVW_TC_PARTS);
+    } else if (fam == FAM_UVW_TC || (fam >= FAM_UVW_TC_DX && fam <= FAM_UVW_TC_DX_SMALL)) {
+        const int mode = fam == FAM_UVW_TC_DW ? 3 : fam == FAM_UVW_TC_DX || fam == FAM_UVW_TC_DX_PARTS || fam == FAM_UVW_TC_DX_SMALL ? 1 : 0;
+        const bool small = fam == FAM_UVW_TC_SMALL || fam == FAM_UVW_TC_DX_SMALL;
+        src += emit_tc(d, mode, small, fam >= FAM_UVW_TC_PARTS);
         src += K_COMMON;
-        src += K_UVW_TC;
+        static const std::string kernel = K_UVW_TC, here = "//@ sets\n";   // (where the emitted functions go: behind what they call)
+        const size_t at = kernel.find(here);
+        src += kernel.substr(0, at);
+        if (mode == 0 ? d.tc : mode == 1 && d.tc_bwd) src += emit_tc_sets(d, mode, small);
+        src += kernel.substr(at + here.size());
     } else {
         // Forward kernels carry two channels per thread in two block-owning groups (their code is small enough to stay
         // in the instruction cache); the backward kernels, three times larger, keep one channel per thread and one
@@ -1667,7 +1702,6 @@ struct TcParams {
     long long batch;
     int accum;
     int* status;
-    int inst0;
     int parts;
     int cut[kTcMaxParts + 1];
 };
@@ -1742,6 +1776,10 @@ TcCuts& tc_cuts(Entry* e, int which) {   // 2 * mode + (0 large sets, 1 small on
     tc_cut(*slot, which == kTcCutsDw ? 8 : kTcMaxParts);
     return *slot;
 }
+int tc_family(int mode, int list, bool parts) {
+    const int fam[3][2] = {{FAM_UVW_TC, FAM_UVW_TC_DX}, {FAM_UVW_TC_PARTS, FAM_UVW_TC_DX_PARTS}, {FAM_UVW_TC_SMALL, FAM_UVW_TC_DX_SMALL}};
+    return fam[list ? 2 : parts ? 1 : 0][mode];
+}
 // How the sets of `tiles` tiles are walked: which list of instances, and in how many parts (1: by one CTA per tile): whatever leaves the busiest
 // CTA least to do when units are dealt out in turn.  Beside its sets a unit fills and drains the pipeline (about 3,000 cycles).
 // 30 paths of 32 x 32, 20 tiles on 148 SMs: 20 us a forward in parts where a tile takes one CTA 40 us; 391 tiles: 119 us in one part.
@@ -1796,7 +1834,7 @@ int encode_map(CUtensorMap* map, const void* data, long long rows, long long col
 int tc_launch(Entry* e, const void* src, const void* y, const void* W, void* dst, const void* x, void* dy, long long batch, int accum, cudaStream_t st, int mode) {
     static const char* names[2][2] = {{"oeq_uvw_tc_forward", "oeq_uvw_tc_forward_parts"}, {"oeq_uvw_tc_backward_dx", "oeq_uvw_tc_backward_dx_parts"}};
     const Desc& d = e->d;
-    TcParams p{{}, y, W, dst, x, dy, batch, accum, nullptr, 0, 1, {0}};
+    TcParams p{{}, y, W, dst, x, dy, batch, accum, nullptr, 1, {0}};
     int rc = encode_map(&p.src, src, batch, d.dim[mode == 0 ? 0 : 2], 128, true);
     if (rc) return rc;
     if (!accum && (mode == 0 ? d.tc_zero_z : d.tc_zero_dx))
@@ -1807,12 +1845,11 @@ int tc_launch(Entry* e, const void* src, const void* y, const void* W, void* dst
     const long long tiles = (batch + 127) / 128;
     int list = 0;
     p.parts = tc_parts(e, mode, tiles, &list);
-    const bool parts = p.parts > 1;
     const TcCuts& c = tc_cuts(e, 2 * mode + list);
     for (int i = 0; i <= p.parts; ++i) p.cut[i] = c.cut[p.parts][i];
-    if (list) p.inst0 = d.tc_plan[mode]->ncoarse;
+    const bool parts = p.parts > 1;
     const char* name = names[mode][parts];
-    if ((rc = get_program(e, mode == 0 ? (parts ? FAM_UVW_TC_PARTS : FAM_UVW_TC) : parts ? FAM_UVW_TC_DX_PARTS : FAM_UVW_TC_DX, &prog))) return rc;
+    if ((rc = get_program(e, tc_family(mode, list, parts), &prog))) return rc;
     cudaKernel_t k, ks = nullptr;
     if ((rc = get_kernel(prog, name, smem, &k))) return rc;
     // The warpgroups hand registers over (setmaxnreg): the shares only add up when the launch gives every thread 65536 / 512 of them.
@@ -2059,8 +2096,8 @@ int oeqb_precompile(const void* desc, size_t desc_len, int64_t key) {
     const std::string header = emit_header(d);
     int done = 0;
     for (int fam = 0; fam < FAM_COUNT; ++fam) {
-        if (fam == FAM_UVW_TC || fam == FAM_UVW_TC_PARTS) { if (!d.tc) continue; }
-        else if (fam >= FAM_UVW_TC_DX && fam <= FAM_UVW_TC_DX_PARTS) { if (!d.tc_bwd) continue; }
+        if (fam == FAM_UVW_TC || fam == FAM_UVW_TC_PARTS || fam == FAM_UVW_TC_SMALL) { if (!d.tc) continue; }
+        else if (fam >= FAM_UVW_TC_DX && fam <= FAM_UVW_TC_DX_SMALL) { if (!d.tc_bwd) continue; }
         else if (fam == FAM_UVW_ITEM) { if (!d.item) continue; }
         else if (fam == FAM_UVW_F64) { if (!d.f64mm) continue; }
         else if (fam == FAM_DW_REDUCE) { if (!d.shared) continue; }

@@ -2,6 +2,7 @@
 import os
 import shutil
 import subprocess
+import time
 
 import numpy as np
 import pytest
@@ -24,7 +25,7 @@ def _descriptor(in1, in2, out):
 @pytest.mark.skipif(not shutil.which(NVCC), reason="needs nvcc")
 @pytest.mark.parametrize("in1,in2,family", [
     (_both(128, 2), "1x0e+1x1o+1x2e+1x3o", "uvw_tc_dw"), (_both(96, 3), "1x0e+1x1o+1x2e+1x3o", "uvw_tc_dw"),
-    (_both(128, 3), "1x0e+1x1o+1x2e", "uvw_tc_dw"), ("+".join(["32x0e"] * 32), "1x0e", "uvw_tc_dx_parts")])
+    (_both(128, 3), "1x0e+1x1o+1x2e", "uvw_tc_dw"), ("+".join(["32x0e"] * 32), "1x0e", "uvw_tc_dx_small")])
 def test_the_widest_products_compile(in1, in2, family, tmp_path):
     text = _descriptor(in1, in2, in1)
     if native.query(text.encode(), descriptor_hash(text)).fast_path != 2:
@@ -32,6 +33,17 @@ def test_the_widest_products_compile(in1, in2, family, tmp_path):
     (tmp_path / "t.cu").write_text(native.emit_source(text.encode(), family))
     subprocess.run([NVCC, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-cubin", "-o", str(tmp_path / "t.cubin"), str(tmp_path / "t.cu")],
                    check=True, stdout=subprocess.DEVNULL)
+
+
+@pytest.mark.skipif(not shutil.which(NVCC), reason="needs nvcc")
+def test_long_sums_compile_in_seconds(tmp_path):
+    """The first call of a problem waits for the compiler: 6 s here; unrolled from templates, and with both kinds of sets in one program, 60 s."""
+    text = _descriptor(_both(32, 3), "1x1e+1x1o+1x2e+1x2o", _both(32, 3))
+    (tmp_path / "t.cu").write_text(native.emit_source(text.encode(), "uvw_tc_dx_parts"))
+    start = time.perf_counter()
+    subprocess.run([NVCC, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-cubin", "-o", str(tmp_path / "t.cubin"), str(tmp_path / "t.cu")],
+                   check=True, stdout=subprocess.DEVNULL)
+    assert time.perf_counter() - start < 25
 
 
 def test_the_sum_of_the_partial_rows_is_a_small_program():
