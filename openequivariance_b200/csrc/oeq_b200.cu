@@ -1276,6 +1276,25 @@ int load_program(const std::string& src, const char* label, Program* p) {
     return OEQB_OK;
 }
 
+// Held by a thread that compiles without g_mutex: threads that want new programs wait for one another, so that each is compiled once.
+std::mutex g_compile_mutex;
+
+// As get_program, but `lock` (on g_mutex, held) is left while the program compiles: the other operators of the process go on.  An entry lasts as long
+// as the process and its description does not change.
+int program_off_lock(std::unique_lock<std::mutex>& lock, Entry* e, int fam) {
+    if (e->prog[fam]) return OEQB_OK;
+    lock.unlock();
+    std::lock_guard<std::mutex> compiling(g_compile_mutex);
+    lock.lock();
+    if (e->prog[fam]) return OEQB_OK;
+    lock.unlock();
+    auto fresh = std::make_unique<Program>();
+    const int rc = load_program(family_source(e->d, e->header, fam), family_name(fam), fresh.get());
+    lock.lock();
+    if (!rc && !e->prog[fam]) e->prog[fam] = std::move(fresh);   // (get_program may have compiled it meanwhile)
+    return rc;
+}
+
 // Caller holds g_mutex.
 int get_program(Entry* e, int fam, Program** out, bool allow_streams = true) {
     std::unique_ptr<Program>& slot = allow_streams ? e->prog[fam] : e->prog_single[fam];
@@ -1830,6 +1849,18 @@ int encode_map(CUtensorMap* map, const void* data, long long rows, long long col
     return OEQB_OK;
 }
 
+// Compiles what a call on `batch` items needs before anything of it is launched, without g_mutex (`lock`, held).
+int tc_prepare(std::unique_lock<std::mutex>& lock, Entry* e, bool forward, bool backward, long long batch) {
+    for (int mode = forward ? 0 : 1; mode <= (backward ? 1 : 0); ++mode) {
+        int list;
+        const int parts = tc_parts(e, mode, (batch + 127) / 128, &list);
+        if (int rc = program_off_lock(lock, e, tc_family(mode, list, parts > 1))) return rc;
+    }
+    if (!backward) return OEQB_OK;
+    if (int rc = program_off_lock(lock, e, FAM_UVW_TC_DW)) return rc;
+    return program_off_lock(lock, e, FAM_DW_REDUCE);
+}
+
 // mode 0: dst = z from (src = x, y, W); mode 1: dst = dx from (src = g, y, W), and dy with x
 int tc_launch(Entry* e, const void* src, const void* y, const void* W, void* dst, const void* x, void* dy, long long batch, int accum, cudaStream_t st, int mode) {
     static const char* names[2][2] = {{"oeq_uvw_tc_forward", "oeq_uvw_tc_forward_parts"}, {"oeq_uvw_tc_backward_dx", "oeq_uvw_tc_backward_dx_parts"}};
@@ -2126,7 +2157,7 @@ int oeqb_tp_forward(const void* desc, size_t desc_len, int64_t key, int64_t batc
     if (batch < 0) return fail(OEQB_EINVAL, "oeqb_tp_forward: negative batch");
     if (batch == 0) return OEQB_OK;
     if (int rc = check_ptrs({x, y, W, z}, "oeqb_tp_forward")) return rc;
-    std::lock_guard<std::mutex> lock(g_mutex);
+    std::unique_lock<std::mutex> lock(g_mutex);
     Entry* e;
     if (int rc = get_entry(desc, desc_len, key, &e)) return rc;
     if (use_fast(e->d) && aligned16({x, W})) {
@@ -2134,6 +2165,7 @@ int oeqb_tp_forward(const void* desc, size_t desc_len, int64_t key, int64_t batc
         return fast_launch(e, 0, f, (cudaStream_t)stream);
     }
     if (e->d.tc && !g_force_generic && !g_no_tc && aligned16({x, z})) {
+        if (int rc = tc_prepare(lock, e, true, false, batch)) return rc;
         return tc_launch(e, x, y, W, z, nullptr, nullptr, batch, 0, (cudaStream_t)stream, 0);
     }
     if (f64_route(e->d, batch)) return f64_forward(e, x, y, W, z, batch, 0, (cudaStream_t)stream);
@@ -2146,7 +2178,7 @@ int oeqb_tp_backward(const void* desc, size_t desc_len, int64_t key, int64_t bat
                      const void* W, const void* g, void* dx, void* dy, void* dW, void* stream) {
     if (batch < 0) return fail(OEQB_EINVAL, "oeqb_tp_backward: negative batch");
     if (int rc = check_ptrs({x, y, W, g, dx, dy, dW}, "oeqb_tp_backward")) return rc;
-    std::lock_guard<std::mutex> lock(g_mutex);
+    std::unique_lock<std::mutex> lock(g_mutex);
     Entry* e;
     if (int rc = get_entry(desc, desc_len, key, &e)) return rc;
     cudaStream_t st = (cudaStream_t)stream;
@@ -2160,6 +2192,8 @@ int oeqb_tp_backward(const void* desc, size_t desc_len, int64_t key, int64_t bat
     if (f64_route(d, batch)) return f64_backward(e, x, y, y, W, g, dx, dy, dW, batch, 0, st);
     if (item_backward_pays(d, batch) && aligned16({W, dW})) return item_backward(e, x, y, y, W, g, dx, dy, dW, batch, 0, st);
     const int tcb = (d.tc_bwd && !g_force_generic && !g_no_tc && aligned16({x, dx, g})) ? g_tc_backward : 0;
+    if (tcb)
+        if (int rc = tc_prepare(lock, e, false, true, batch)) return rc;
     if (tcb != 7) {
         CUDA_TRY(cudaMemsetAsync(dy, 0, batch * d.dim[1] * d.elt(), st));
         BwdParams p{x, y, y, W, g, dx, dy, dW, nullptr, nullptr, nullptr, batch, batch, UNIT_ITEM, 0};
@@ -2173,7 +2207,7 @@ int oeqb_tp_double_backward(const void* desc, size_t desc_len, int64_t key, int6
                             const void* W2, void* dx, void* dy, void* dW, void* dg, void* stream) {
     if (batch < 0) return fail(OEQB_EINVAL, "oeqb_tp_double_backward: negative batch");
     if (int rc = check_ptrs({x, y, W, g, x2, y2, W2, dx, dy, dW, dg}, "oeqb_tp_double_backward")) return rc;
-    std::lock_guard<std::mutex> lock(g_mutex);
+    std::unique_lock<std::mutex> lock(g_mutex);
     Entry* e;
     if (int rc = get_entry(desc, desc_len, key, &e)) return rc;
     cudaStream_t st = (cudaStream_t)stream;
@@ -2202,6 +2236,7 @@ int oeqb_tp_double_backward(const void* desc, size_t desc_len, int64_t key, int6
     }
     if (d.tc_bwd && !g_force_generic && !g_no_tc && g_tc_backward == 7 && aligned16({x, x2, dx, dg, g})) {
         // the same five passes on the tensor-core kernels (the second and later ones add to their outputs)
+        if ((rc = tc_prepare(lock, e, true, true, batch))) return rc;
         if ((rc = tc_launch(e, x2, y, W, dg, nullptr, nullptr, batch, 0, st, 0))) return rc;
         if ((rc = tc_launch(e, x, y2, W, dg, nullptr, nullptr, batch, 1, st, 0))) return rc;
         if ((rc = tc_launch(e, x, y, W2, dg, nullptr, nullptr, batch, 1, st, 0))) return rc;
@@ -2850,10 +2885,7 @@ std::string emit_sym(const SymPlan& p, int dtype, const SymTerm* t) {
 
 std::map<std::pair<uint64_t, int>, std::unique_ptr<Program>> g_sym_programs;   // by (key of the terms, dtype)
 
-std::mutex g_sym_compile_mutex;
-
 // Takes g_mutex, and leaves it while it compiles (about a second per hundred terms): the other operators of the process go on.
-// Threads that want new programs wait for one another, so that each is compiled once.
 int symcon_program(const SymPlan& p, int dtype, const int32_t* terms, Program** out) {
     const std::pair<uint64_t, int> key{p.key, dtype};
     auto known = [&] {
@@ -2863,7 +2895,7 @@ int symcon_program(const SymPlan& p, int dtype, const int32_t* terms, Program** 
         return it != g_sym_programs.end();
     };
     if (known()) return OEQB_OK;
-    std::lock_guard<std::mutex> compiling(g_sym_compile_mutex);
+    std::lock_guard<std::mutex> compiling(g_compile_mutex);
     if (known()) return OEQB_OK;
     if (int rc = check_ptrs({terms}, "oeqb_symcon")) return rc;
     const SymTerm* t = (const SymTerm*)terms;

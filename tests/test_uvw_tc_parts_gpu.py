@@ -114,3 +114,51 @@ def test_a_thread_whose_first_use_of_the_device_is_a_product():
         thread.start()
         thread.join()
     assert len(found) == 2 and torch.equal(found[0], want) and all(t.isfinite().all() for t in found[1])
+
+
+def test_other_operators_run_while_a_program_compiles(tmp_path):
+    import os
+    import threading
+    import time
+
+    import torch
+
+    import openequivariance_b200 as oeq
+    from openequivariance_b200 import native
+    from openequivariance_b200.core import problems as P
+    small = P.readme_problem()
+    tp = oeq.TensorProduct(small)
+    rnd = lambda *s: torch.randn(*s, device="cuda")  # noqa: E731
+    operands = [rnd(100, small.irreps_in1.dim), rnd(100, small.irreps_in2.dim), rnd(100, small.weight_numel)]
+    tp(*operands)
+    feats = "32x0e+32x1e+64x2o+32x3e"                        # (a product of no other test)
+    p = P.FullyConnectedTPProblem(feats, "1x0e+1x1o+1x2e", feats, shared_weights=True)
+    wide = oeq.TensorProduct(p)
+    leaves = [t.requires_grad_() for t in (rnd(50, p.irreps_in1.dim), rnd(50, p.irreps_in2.dim), rnd(p.weight_numel))]
+    gate, done, times = threading.Event(), threading.Event(), []
+
+    def first_use():
+        gate.set()
+        times.append(time.perf_counter())
+        try:
+            wide(*leaves).sum().backward()
+        finally:
+            times.append(time.perf_counter())
+            done.set()
+
+    native.set_option("cache_dir", str(tmp_path))            # empty: the programs have to be compiled
+    thread = threading.Thread(target=first_use)
+    thread.start()
+    gate.wait()
+    longest, calls = 0.0, 0
+    while not done.is_set():
+        start = time.perf_counter()
+        tp(*operands)
+        if not done.is_set():
+            longest, calls = max(longest, time.perf_counter() - start), calls + 1
+        time.sleep(0.001)
+    thread.join()
+    native.set_option("cache_dir", os.path.join(os.path.dirname(oeq.__file__), "csrc", "_cubin_cache"))
+    assert times[1] - times[0] > 0.5                         # it was compiled here
+    assert calls > 10 and longest < 0.25 * (times[1] - times[0]), (calls, longest, times)
+    assert all(t.grad.isfinite().all() for t in leaves)
