@@ -1202,8 +1202,8 @@ struct Program {
     std::map<std::string, cudaKernel_t> kernels;
     std::map<std::string, int> smem_set;  // kernel -> bitmask of devices whose smem attribute was raised
     std::string cubin;                    // kept alive for lazy per-context loading
-    std::set<std::string> regs_ok;        // tensor-core kernels whose register count was verified
-    bool regs_checked = false;            // multi-stream kernels: register count verified against the hand-over scheme
+    bool regs_ok = false;                 // tensor-core kernels: register count verified against the hand-over scheme
+    bool regs_checked = false;            // multi-stream kernels: the same
 };
 
 // How the work on a tile is cut into parts (TcParams::parts, TcDwParams::splits): for S parts the boundaries that make the
@@ -1225,6 +1225,7 @@ struct Entry {
     std::unique_ptr<Program> prog[FAM_COUNT];
     std::unique_ptr<TcCuts> tc_cuts[5];                 // how the tensor-core kernels' work is cut: large and small sets of mode 0, of mode 1, dW
     std::unique_ptr<Program> prog_single[FAM_COUNT];   // the same families built with one edge stream per CTA
+    bool tc_off = false;                                // a tensor-core program did not compile to what the host expects
     bool streams_off = false;                           // a multi-stream kernel came out with the wrong register count
 };
 
@@ -1272,7 +1273,10 @@ int load_program(const std::string& src, const char* label, Program* p) {
         if ((rc = compile_cubin(src, label, p->cubin, nullptr))) return rc;
         ce = cudaLibraryLoadData(&p->lib, p->cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0);
     }
-    if (ce != cudaSuccess) return fail(OEQB_ECOMPILE, "cudaLibraryLoadData(%s): %s", label, cudaGetErrorString(ce));
+    if (ce != cudaSuccess) {
+        cudaGetLastError();
+        return fail(OEQB_ECOMPILE, "cudaLibraryLoadData(%s): %s", label, cudaGetErrorString(ce));
+    }
     return OEQB_OK;
 }
 
@@ -1315,7 +1319,10 @@ int get_kernel(Program* p, const char* name, size_t smem, cudaKernel_t* out) {
     if (it == p->kernels.end()) {
         cudaKernel_t k;
         cudaError_t ce = cudaLibraryGetKernel(&k, p->lib, name);
-        if (ce != cudaSuccess) return fail(OEQB_ECOMPILE, "kernel %s not found: %s", name, cudaGetErrorString(ce));
+        if (ce != cudaSuccess) {
+            cudaGetLastError();   // (not for the next caller to find: this problem may be served by other kernels)
+            return fail(OEQB_ECOMPILE, "kernel %s not found: %s", name, cudaGetErrorString(ce));
+        }
         it = p->kernels.emplace(name, k).first;
         g_kernel_names[k] = name;
     }
@@ -1819,6 +1826,7 @@ int tc_parts(Entry* e, int mode, long long tiles, int* list) {
 }
 
 int keep_pool_memory();
+void note_slow_path(const char* where, const char* why);
 
 // The map of a [rows, cols] array of floats for copies of 32 columns x box_rows rows (cols a multiple of 32, 16-byte aligned).
 int encode_map(CUtensorMap* map, const void* data, long long rows, long long cols, unsigned box_rows, bool swizzled) {
@@ -1849,21 +1857,44 @@ int encode_map(CUtensorMap* map, const void* data, long long rows, long long col
     return OEQB_OK;
 }
 
-// Compiles what a call on `batch` items needs before anything of it is launched, without g_mutex (`lock`, held).
-int tc_prepare(std::unique_lock<std::mutex>& lock, Entry* e, bool forward, bool backward, long long batch) {
-    for (int mode = forward ? 0 : 1; mode <= (backward ? 1 : 0); ++mode) {
-        int list;
-        const int parts = tc_parts(e, mode, (batch + 127) / 128, &list);
-        if (int rc = program_off_lock(lock, e, tc_family(mode, list, parts > 1))) return rc;
+// The kernel of a program, and whether it is what the host expects.  The warpgroups hand registers over (setmaxnreg): the shares only add up when the
+// launch gives every thread 65536 / 512 of them.
+int tc_kernel(Entry* e, int mode, int list, bool parts, cudaKernel_t* k, Program** prog) {
+    static const char* names[2][2] = {{"oeq_uvw_tc_forward", "oeq_uvw_tc_forward_parts"}, {"oeq_uvw_tc_backward_dx", "oeq_uvw_tc_backward_dx_parts"}};
+    const char* name = names[mode][parts];
+    if (int rc = get_program(e, tc_family(mode, list, parts), prog)) return rc;
+    if (int rc = get_kernel(*prog, name, e->d.tc_plan[mode]->smem, k)) return rc;
+    if (!(*prog)->regs_ok) {
+        cudaFuncAttributes attr;
+        CUDA_TRY(cudaFuncGetAttributes(&attr, (const void*)*k));
+        if (attr.numRegs != 128) return fail(OEQB_ECOMPILE, "%s was compiled to %d registers instead of 128: its register hand-over would not end", name, attr.numRegs);
+        (*prog)->regs_ok = true;
     }
-    if (!backward) return OEQB_OK;
-    if (int rc = program_off_lock(lock, e, FAM_UVW_TC_DW)) return rc;
-    return program_off_lock(lock, e, FAM_DW_REDUCE);
+    return OEQB_OK;
+}
+// Compiles what a call on `batch` items needs before anything of it is launched, without g_mutex (`lock`, held).  OEQB_ECOMPILE: there is no usable
+// program (noted once); the general kernels serve the problem from then on.
+int tc_prepare(std::unique_lock<std::mutex>& lock, Entry* e, bool forward, bool backward, long long batch) {
+    if (e->tc_off) return OEQB_ECOMPILE;
+    int rc = OEQB_OK;
+    for (int mode = forward ? 0 : 1; mode <= (backward ? 1 : 0) && !rc; ++mode) {
+        int list;
+        cudaKernel_t k;
+        Program* prog;
+        const bool parts = tc_parts(e, mode, (batch + 127) / 128, &list) > 1;
+        if (!(rc = program_off_lock(lock, e, tc_family(mode, list, parts)))) rc = tc_kernel(e, mode, list, parts, &k, &prog);
+    }
+    if (backward && !rc) rc = program_off_lock(lock, e, FAM_UVW_TC_DW);
+    if (backward && !rc) rc = program_off_lock(lock, e, FAM_DW_REDUCE);
+    if (rc == OEQB_ECOMPILE) {
+        e->tc_off = true;
+        note_slow_path("uvw on the tensor cores", g_err.c_str());
+    }
+    return rc;
 }
 
 // mode 0: dst = z from (src = x, y, W); mode 1: dst = dx from (src = g, y, W), and dy with x
 int tc_launch(Entry* e, const void* src, const void* y, const void* W, void* dst, const void* x, void* dy, long long batch, int accum, cudaStream_t st, int mode) {
-    static const char* names[2][2] = {{"oeq_uvw_tc_forward", "oeq_uvw_tc_forward_parts"}, {"oeq_uvw_tc_backward_dx", "oeq_uvw_tc_backward_dx_parts"}};
     const Desc& d = e->d;
     TcParams p{{}, y, W, dst, x, dy, batch, accum, nullptr, 1, {0}};
     int rc = encode_map(&p.src, src, batch, d.dim[mode == 0 ? 0 : 2], 128, true);
@@ -1871,7 +1902,6 @@ int tc_launch(Entry* e, const void* src, const void* y, const void* W, void* dst
     if (!accum && (mode == 0 ? d.tc_zero_z : d.tc_zero_dx))
         CUDA_TRY(cudaMemsetAsync(dst, 0, (size_t)batch * d.dim[mode == 0 ? 2 : 0] * sizeof(float), st));
     if ((rc = status_word(&p.status))) return rc;
-    Program* prog;
     const size_t smem = d.tc_plan[mode]->smem;
     const long long tiles = (batch + 127) / 128;
     int list = 0;
@@ -1879,17 +1909,9 @@ int tc_launch(Entry* e, const void* src, const void* y, const void* W, void* dst
     const TcCuts& c = tc_cuts(e, 2 * mode + list);
     for (int i = 0; i <= p.parts; ++i) p.cut[i] = c.cut[p.parts][i];
     const bool parts = p.parts > 1;
-    const char* name = names[mode][parts];
-    if ((rc = get_program(e, tc_family(mode, list, parts), &prog))) return rc;
+    Program* prog;
     cudaKernel_t k, ks = nullptr;
-    if ((rc = get_kernel(prog, name, smem, &k))) return rc;
-    // The warpgroups hand registers over (setmaxnreg): the shares only add up when the launch gives every thread 65536 / 512 of them.
-    if (!prog->regs_ok.count(name)) {
-        cudaFuncAttributes attr;
-        CUDA_TRY(cudaFuncGetAttributes(&attr, (const void*)k));
-        if (attr.numRegs != 128) return fail(OEQB_ECOMPILE, "%s was compiled to %d registers instead of 128: its register hand-over would not end", name, attr.numRegs);
-        prog->regs_ok.insert(name);
-    }
+    if ((rc = tc_kernel(e, mode, list, parts, &k, &prog))) return rc;
     const unsigned grid = (unsigned)std::min<long long>(sm_count(), tiles * p.parts);
     // stream-ordered scratch: an aligned copy of weights that start at an odd place (the kernel's loads are of 16 bytes), and the parts' sums of
     // dy, rows that a second kernel adds in order
@@ -2165,8 +2187,8 @@ int oeqb_tp_forward(const void* desc, size_t desc_len, int64_t key, int64_t batc
         return fast_launch(e, 0, f, (cudaStream_t)stream);
     }
     if (e->d.tc && !g_force_generic && !g_no_tc && aligned16({x, z})) {
-        if (int rc = tc_prepare(lock, e, true, false, batch)) return rc;
-        return tc_launch(e, x, y, W, z, nullptr, nullptr, batch, 0, (cudaStream_t)stream, 0);
+        const int rc = tc_prepare(lock, e, true, false, batch);
+        if (rc != OEQB_ECOMPILE) return rc ? rc : tc_launch(e, x, y, W, z, nullptr, nullptr, batch, 0, (cudaStream_t)stream, 0);
     }
     if (f64_route(e->d, batch)) return f64_forward(e, x, y, W, z, batch, 0, (cudaStream_t)stream);
     if (item_forward_pays(e->d, batch) && aligned16({W})) return item_forward(e, x, y, W, z, batch, 0, (cudaStream_t)stream);
@@ -2191,9 +2213,12 @@ int oeqb_tp_backward(const void* desc, size_t desc_len, int64_t key, int64_t bat
     }
     if (f64_route(d, batch)) return f64_backward(e, x, y, y, W, g, dx, dy, dW, batch, 0, st);
     if (item_backward_pays(d, batch) && aligned16({W, dW})) return item_backward(e, x, y, y, W, g, dx, dy, dW, batch, 0, st);
-    const int tcb = (d.tc_bwd && !g_force_generic && !g_no_tc && aligned16({x, dx, g})) ? g_tc_backward : 0;
+    int tcb = (d.tc_bwd && !g_force_generic && !g_no_tc && aligned16({x, dx, g})) ? g_tc_backward : 0;
     if (tcb)
-        if (int rc = tc_prepare(lock, e, false, true, batch)) return rc;
+        if (int rc = tc_prepare(lock, e, false, true, batch)) {
+            if (rc != OEQB_ECOMPILE) return rc;
+            tcb = 0;
+        }
     if (tcb != 7) {
         CUDA_TRY(cudaMemsetAsync(dy, 0, batch * d.dim[1] * d.elt(), st));
         BwdParams p{x, y, y, W, g, dx, dy, dW, nullptr, nullptr, nullptr, batch, batch, UNIT_ITEM, 0};
@@ -2234,9 +2259,10 @@ int oeqb_tp_double_backward(const void* desc, size_t desc_len, int64_t key, int6
         b.X2 = x2; b.Y2 = y2; b.W2 = W2;   // both second-order backward terms in one pass
         return fast_launch(e, 3, b, st, nullptr, true);
     }
-    if (d.tc_bwd && !g_force_generic && !g_no_tc && g_tc_backward == 7 && aligned16({x, x2, dx, dg, g})) {
+    if (d.tc_bwd && !g_force_generic && !g_no_tc && g_tc_backward == 7 && aligned16({x, x2, dx, dg, g}) &&
+        (rc = tc_prepare(lock, e, true, true, batch)) != OEQB_ECOMPILE) {
         // the same five passes on the tensor-core kernels (the second and later ones add to their outputs)
-        if ((rc = tc_prepare(lock, e, true, true, batch))) return rc;
+        if (rc) return rc;
         if ((rc = tc_launch(e, x2, y, W, dg, nullptr, nullptr, batch, 0, st, 0))) return rc;
         if ((rc = tc_launch(e, x, y2, W, dg, nullptr, nullptr, batch, 1, st, 0))) return rc;
         if ((rc = tc_launch(e, x, y, W2, dg, nullptr, nullptr, batch, 1, st, 0))) return rc;

@@ -2,6 +2,7 @@
 tiles (every cut of the schedule), one tile more than there are SMs (a ragged last wave), against the fp64 oracle."""
 import pytest
 
+from openequivariance_b200.core.problem import TPProblem
 from test_uvw_f64_gpu import orders_0_to_2, shared_problem
 
 pytestmark = pytest.mark.gpu
@@ -162,3 +163,49 @@ def test_other_operators_run_while_a_program_compiles(tmp_path):
     assert times[1] - times[0] > 0.5                         # it was compiled here
     assert calls > 10 and longest < 0.25 * (times[1] - times[0]), (calls, longest, times)
     assert all(t.grad.isfinite().all() for t in leaves)
+
+
+@pytest.mark.parametrize("family", ["uvw_tc", "uvw_tc_dx_parts"])      # (what 50 items of these problems run)
+def test_general_kernels_serve_a_problem_whose_program_is_unusable(family, tmp_path):
+    """A cubin without the kernel stands in the cache where the program's should be."""
+    import ctypes
+    import os
+    import shutil
+    import subprocess
+
+    import torch
+
+    import openequivariance_b200 as oeq
+    from helpers import kernels_launched, rel_l2, uniform_inputs
+    from openequivariance_b200 import native
+    from openequivariance_b200.core.descriptor import build_descriptor
+    from oracle import tp_oracle
+    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+    if not shutil.which(nvcc):
+        pytest.skip("needs nvcc")
+    p = TPProblem("32x1e", "1x1e", "32x1e" if family == "uvw_tc" else "32x2e", [(0, 0, 0, "uvw", True)], shared_weights=True, internal_weights=False)
+    # (the name of a cubin in the cache: a hash of the source, the compiler's options and its version)
+    major, minor = ctypes.c_int(), ctypes.c_int()
+    native.load()
+    ctypes.CDLL("libnvrtc.so.12").nvrtcVersion(ctypes.byref(major), ctypes.byref(minor))
+    key = 1469598103934665603
+    for c in (native.emit_source(build_descriptor(p).encode(), family) + "--gpu-architecture=sm_100a--std=c++17-lineinfo-default-device--extra-device-vectorization"
+              + str(major.value * 100 + minor.value)).encode():
+        key = (key ^ c) * 1099511628211 % 2 ** 64
+    (tmp_path / "t.cu").write_text('extern "C" __global__ void nothing() {}\n')
+    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-cubin", "-o", str(tmp_path / f"{key:016x}.cubin"), str(tmp_path / "t.cu")], check=True)
+    native.set_option("cache_dir", str(tmp_path))
+    try:
+        x, y, w, g, x2, y2, w2 = uniform_inputs(p, 50)
+        tp = oeq.TensorProduct(p)
+        t = [torch.tensor(a, device="cuda") for a in (x, y, w, g, x2, y2, w2)]
+        ops = torch.ops.libtorch_tp_jit
+        got, ran = kernels_launched(lambda: [ops.jit_tp_forward(tp.kernel, tp.hash, *t[:3], p.irreps_out.dim), *ops.jit_tp_backward(tp.kernel, tp.hash, *t[:4]),
+                                             *ops.jit_tp_double_backward(tp.kernel, tp.hash, *t)])
+    finally:
+        native.set_option("cache_dir", os.path.join(os.path.dirname(oeq.__file__), "csrc", "_cubin_cache"))
+    assert {"oeq_generic_backward_shared", "oeq_generic_forward"} <= ran and "oeq_uvw_tc_backward_dw" not in ran, ran
+    we, we2 = tp.reorder_weights_to_e3nn(w), tp.reorder_weights_to_e3nn(w2)
+    want = [tp_oracle.forward(p, x, y, we), *tp_oracle.backward(p, x, y, we, g), *tp_oracle.double_backward(p, x, y, we, g, x2, y2, we2)]
+    for n, (a, b) in enumerate(zip(got, want)):
+        assert rel_l2(a.cpu().numpy(), tp.reorder_weights_from_e3nn(b) if n in (3, 6) else b) <= 1e-5
