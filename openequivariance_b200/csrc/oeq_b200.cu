@@ -133,7 +133,7 @@ std::vector<std::vector<int>> tc_dw_groups(const Desc& d);
 size_t tc_dw_smem_bytes(const Desc& d);
 
 // The tensor-core kernels of mode 0 (forward) and 1 (gradients of x and y): see kernels/uvw_tc.cuh for the words.
-constexpr int kTcMaxParts = 16;
+constexpr int kTcMaxParts = kMaxParts;
 struct TcPlan {
     struct Visit { int src; std::vector<int> ins; };   // source block, instructions from it into the set (one weight tile each)
     struct Set {
@@ -1206,16 +1206,6 @@ struct Program {
     bool regs_checked = false;            // multi-stream kernels: the same
 };
 
-// How the work on a tile is cut into parts (TcParams::parts, TcDwParams::splits): for S parts the boundaries that make the
-// costliest part cheapest, a group (an instance of a one-tile set, or a stack of paths for dW) never being cut.
-struct TcCuts {
-    std::vector<int> begin;                   // first instance (mode 3: first group) of every group, and the end
-    std::vector<double> cost;
-    int n[kTcMaxParts + 1] = {0};             // parts that S asks for (fewer when there are fewer groups)
-    int cut[kTcMaxParts + 1][kTcMaxParts + 1] = {{0}};
-    double part[kTcMaxParts + 1][kTcMaxParts] = {{0}};
-};
-
 struct Entry {
     Desc d;
     uint64_t desc_hash = 0;     // of the descriptor text this entry was built from: a key reused for another problem is refused
@@ -1223,7 +1213,7 @@ struct Entry {
     const void* seen_ptr = nullptr;   // last caller buffer whose contents were compared (callers pass the same buffer again)
     std::string header;
     std::unique_ptr<Program> prog[FAM_COUNT];
-    std::unique_ptr<TcCuts> tc_cuts[5];                 // how the tensor-core kernels' work is cut: large and small sets of mode 0, of mode 1, dW
+    std::unique_ptr<Cuts> tc_cuts[5];                     // how the tensor-core kernels' work is cut: large and small sets of mode 0, of mode 1, dW
     std::unique_ptr<Program> prog_single[FAM_COUNT];   // the same families built with one edge stream per CTA
     bool tc_off = false;                                // a tensor-core program did not compile to what the host expects
     bool streams_off = false;                           // a multi-stream kernel came out with the wrong register count
@@ -1740,29 +1730,6 @@ struct TcDwParams {
     int cut[kTcMaxParts + 1];
 };
 
-void tc_cut(TcCuts& c, int most) {
-    const int G = (int)c.cost.size();
-    double total = 0, big = 0;
-    for (double v : c.cost) { total += v; big = std::max(big, v); }
-    for (int S = 1; S <= most; ++S) {
-        double lo = big, hi = total + 1;
-        auto fill = [&](double cap, bool keep) {
-            int parts = 0;
-            for (int g = 0; g < G;) {
-                if (parts == S) return false;
-                double sum = 0;
-                if (keep) c.cut[S][parts] = c.begin[g];
-                do sum += c.cost[g++]; while (g < G && sum + c.cost[g] <= cap);
-                if (keep) { c.part[S][parts] = sum; c.cut[S][parts + 1] = c.begin[g]; }
-                ++parts;
-            }
-            if (keep) c.n[S] = parts;
-            return true;
-        };
-        for (int it = 0; it < 24; ++it) (fill((lo + hi) / 2, false) ? hi : lo) = (lo + hi) / 2;
-        fill(hi, true);
-    }
-}
 // SM cycles of an instance of a set (mode 0 and 1): per chunk the slowest of MMAs (12 of N / 2 cycles each), conversion and sums.
 double tc_instance_cost(const Desc& d, int mode, int n) {
     const TcPlan& p = *d.tc_plan[mode];
@@ -1779,27 +1746,19 @@ double tc_instance_cost(const Desc& d, int mode, int n) {
     return cost;
 }
 constexpr int kTcCutsDw = 4;
-TcCuts& tc_cuts(Entry* e, int which) {   // 2 * mode + (0 large sets, 1 small ones), or kTcCutsDw
-    std::unique_ptr<TcCuts>& slot = e->tc_cuts[which];
+Cuts& tc_cuts(Entry* e, int which) {   // 2 * mode + (0 large sets, 1 small ones), or kTcCutsDw: of the groups, whose costs alone are used
+    std::unique_ptr<Cuts>& slot = e->tc_cuts[which];
     if (slot) return *slot;
-    slot = std::make_unique<TcCuts>();
+    slot = std::make_unique<Cuts>();
     const Desc& d = e->d;
     if (which == kTcCutsDw) {
         const std::vector<TcSub> subs = tc_subpaths(d);
-        const auto groups = tc_dw_groups(d);
-        for (size_t g = 0; g < groups.size(); ++g) {
-            slot->begin.push_back((int)g);
-            slot->cost.push_back(2 * 600.0 * d.L[2][d.ins[subs[groups[g][0]].ins].o].d() + 1000);   // two halves of a tile, a chunk per component
-        }
-        slot->begin.push_back((int)groups.size());
+        for (auto& g : tc_dw_groups(d)) slot->cost.push_back(2 * 600.0 * d.L[2][d.ins[subs[g[0]].ins].o].d() + 1000);   // two halves of a tile, a chunk per component
     } else {
-        const int mode = which / 2;
-        const TcPlan& p = *d.tc_plan[mode];
-        const int n0 = which % 2 ? p.ncoarse : 0, n1 = which % 2 ? (int)p.inst.size() : p.ncoarse;
-        for (int n = n0; n < n1; ++n) { slot->begin.push_back(n - n0); slot->cost.push_back(tc_instance_cost(d, mode, n)); }
-        slot->begin.push_back(n1 - n0);
+        const TcPlan& p = *d.tc_plan[which / 2];
+        for (int n = which % 2 ? p.ncoarse : 0; n < (which % 2 ? (int)p.inst.size() : p.ncoarse); ++n) slot->cost.push_back(tc_instance_cost(d, which / 2, n));
+        cut_into_parts(*slot);
     }
-    tc_cut(*slot, which == kTcCutsDw ? 8 : kTcMaxParts);
     return *slot;
 }
 int tc_family(int mode, int list, bool parts) {
@@ -1811,18 +1770,10 @@ int tc_family(int mode, int list, bool parts) {
 // 30 paths of 32 x 32, 20 tiles on 148 SMs: 20 us a forward in parts where a tile takes one CTA 40 us; 391 tiles: 119 us in one part.
 int tc_parts(Entry* e, int mode, long long tiles, int* list) {
     const int sms = sm_count();
-    int best = 1;
     *list = 0;
-    if (tiles >= 16LL * sms) return best;
-    double best_time = 0;
-    for (int l = 0; l < 2; ++l) {
-        const TcCuts& c = tc_cuts(e, 2 * mode + l);
-        for (int S = 1 + l; S <= kTcMaxParts && c.n[S] == S; ++S) {
-            const double t = busiest_load(tiles * S, S, c.part[S], 3000.0, sms) + (mode == 1 && S > 1 ? 1500.0 : 0.0);
-            if ((l == 0 && S == 1) || t < 0.95 * best_time) { best = S; *list = l; best_time = t; }
-        }
-    }
-    return best;
+    if (tiles >= 16LL * sms) return 1;
+    const Cuts* lists[2] = {&tc_cuts(e, 2 * mode), &tc_cuts(e, 2 * mode + 1)};
+    return best_parts(lists, tiles, 3000.0, mode == 1 ? 1500.0 : 0.0, sms, list);
 }
 
 int keep_pool_memory();
@@ -1906,7 +1857,7 @@ int tc_launch(Entry* e, const void* src, const void* y, const void* W, void* dst
     const long long tiles = (batch + 127) / 128;
     int list = 0;
     p.parts = tc_parts(e, mode, tiles, &list);
-    const TcCuts& c = tc_cuts(e, 2 * mode + list);
+    const Cuts& c = tc_cuts(e, 2 * mode + list);
     for (int i = 0; i <= p.parts; ++i) p.cut[i] = c.cut[p.parts][i];
     const bool parts = p.parts > 1;
     Program* prog;

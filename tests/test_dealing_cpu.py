@@ -46,3 +46,27 @@ def _timed(busiest, units, part):
     start = time.perf_counter()
     busiest(units, part, 8.0, 148)
     return time.perf_counter() - start
+
+
+@pytest.fixture(scope="module")
+def best(tmp_path_factory):
+    """(parts, list) for two lists of costs, tiles and workers."""
+    d = tmp_path_factory.mktemp("parts")
+    (d / "t.cpp").write_text('#include "dealing.h"\nextern "C" int f(int n0, const double* c0, int n1, const double* c1, long long t, double each, double extra,'
+                             " int w, int* list) { Cuts a, b; a.cost.assign(c0, c0 + n0); b.cost.assign(c1, c1 + n1); cut_into_parts(a); cut_into_parts(b);"
+                             " const Cuts* l[2] = {&a, &b}; return best_parts(l, t, each, extra, w, list); }\n")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-I{CSRC}", str(d / "t.cpp"), "-o", str(d / "t.so")], check=True)
+    f = ctypes.CDLL(str(d / "t.so")).f
+    array = lambda v: (ctypes.c_double * len(v))(*v)  # noqa: E731
+
+    def call(c0, c1, tiles, each=3000.0, extra=0.0, workers=148):
+        which = ctypes.c_int()
+        return f(len(c0), array(c0), len(c1), array(c1), ctypes.c_longlong(tiles), ctypes.c_double(each), ctypes.c_double(extra), workers,
+                 ctypes.byref(which)), which.value
+    return call
+
+
+def test_a_number_of_parts_that_makes_no_cut_does_not_hide_the_next(best):
+    assert best([7000.0] * 4, [7000.0] * 4, 20) == (4, 0)             # three parts of four equal pieces are two
+    assert best([48000.0], [4000.0] * 12, 4) == (12, 1)               # seven to eleven of twelve are six
+    assert best([7000.0] * 4, [7000.0] * 4, 148) == (1, 0)            # a tile for each worker
