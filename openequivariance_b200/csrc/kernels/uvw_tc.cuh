@@ -887,7 +887,7 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) oeq_uvw_tc_backward_
         const int w2 = warp - TCW_AW - 3;
         constexpr int LD = L2_DIM | 1;
         float* ys = sh.ys[w2];
-        unsigned ns = 0;
+        unsigned ns = 0, nload = 0;   // stages, and those whose boxes are requested
         float tc[TCW_PPL][TCW_TERMS];
         int tj[TCW_PPL][TCW_TERMS];
         ok = walk(
@@ -899,6 +899,7 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) oeq_uvw_tc_backward_
                     if (lane == 0) tc_mbar_expect_tx(&sh.xs_full[buf], 4096u * (unsigned)nbox);
                     __syncwarp();
                     if (lane < nbox) tc_tile_load(sh.xg[buf] + lane * 1024, lane < gbox ? &p.x : &p.g, TCW_BOX[grp * 32 + lane], (int)(tile * TCW_TILE + 32 * half), &sh.xs_full[buf]);
+                    ++nload;
                 }
                 if (grp == g0 && half == 0) {      // the tile's harmonics (no item: zeros, and T = 0)
                     __syncwarp();
@@ -949,7 +950,7 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) oeq_uvw_tc_backward_
         if (!ok && w2 == 0) {   // given up: the copies in flight end before the CTA does
             if (lane == 0) tc_give_up(&sh.abort_flag, p.status, 61 + warp);
             __syncwarp();
-            for (unsigned s = ns >= 1 ? ns - 1 : 0; s <= ns; ++s) tc_mbar_wait(&sh.xs_full[s & 1u], (s >> 1) & 1u, &sh.never);
+            for (unsigned s = nload > 2 ? nload - 2 : 0; s < nload; ++s) tc_mbar_wait(&sh.xs_full[s & 1u], (s >> 1) & 1u, &sh.never);
         }
     }
     if (!ok && lane == 0) tc_give_up(&sh.abort_flag, p.status, 61 + warp);
