@@ -6,8 +6,9 @@
 //
 // The weights are applied first, to the raw components of the input, and the Clebsch-Gordan sums run over the products.  The other order
 // (Clebsch-Gordan sums into the A operand, one per path and output component) needs an operand of 128 x 32 per (path, k), 102 for the 30
-// paths of 32x(0+1+2, both parities); this one needs one per input component and pass, 18 or 36, and its sums in tensor memory are 32
-// products long (the tensor cores add with truncation, so the error of a sum grows with its length).
+// paths of 32x(0+1+2, both parities); this one needs one per set and input component, 36 a tile in the forward (two sets) and 68 for the
+// gradients (four), and its sums in tensor memory are 32 products long (the tensor cores add with truncation, so the error of a sum grows with
+// its length).
 // The gradient of x is the same computation on the cotangent with the weights transposed, and the gradient of y takes its products
 // from the same accumulators:
 //   V_p[b][u, k] = sum_w W_p[u, w] g[b, o][w, k]      dx[b, a][u, i] = sum cy_p[b][i, k] V_p[b][u, k]
@@ -29,8 +30,8 @@
 // (both agree, so the products do not change): with it the conversion's reads fall into 32 different banks.
 // Registers: 512 threads start with 128; the conversion and issue warpgroups hand theirs to the two that keep the sums (setmaxnreg).
 // Every mbarrier wait is bounded; on time-out the CTA leaves after its copies and MMAs have ended and its tensor memory is free.
-// What bounds it: instruction latency (0.38 instructions a cycle and scheduler, long-scoreboard stalls first; tensor pipe 27 % forward, 14 %
-// gradients).  50,000 items of 32x(0+1+2, both parities): forward 455 us with the Clebsch-Gordan sums first, 119 us; gradients of x and y
+// What bounds it: instruction latency (0.41 instructions a cycle and scheduler, long-scoreboard stalls first; tensor pipe 29 % forward, 15 %
+// gradients).  50,000 items of 32x(0+1+2, both parities): forward 455 us with the Clebsch-Gordan sums first, 117 us; gradients of x and y
 // 1,070 us in two kernels of that kind, 219 us.
 #pragma once
 #if OEQ_TC
@@ -457,7 +458,7 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) TC_KERNEL_NAME(const
 #pragma unroll
                         for (int q = 0; q < 8; ++q) {
                             const float r = tc_tf32(hi[q]);
-                            lo[q] = hi[q] - r;   // the tensor core reads the top 19 bits: truncation of the low part is below 2^-21
+                            lo[q] = hi[q] - r;   // 12 bits, of which the tensor core reads 11: what is lost is below 2^-23
                             hi[q] = r;
                         }
                         tc_st_a(dst + ((unsigned)(16 * h) << 16) + 16u * g, hi);
@@ -628,7 +629,7 @@ extern "C" __global__ void __launch_bounds__(256) oeq_uvw_tc_backward_dy_parts(c
 //   warp 16      12 MMAs (128 x 32 x 8) a chunk
 // A in tensor memory: lane = (slot, channel), column = item, which is how the T of a warp lie in its registers; through shared memory it would be
 // stored twice and read three times.  50,000 items of 32x(0+1+2, both parities): 596 us with T formed from tables by all warps for
-// operands in shared memory, 325 us.
+// operands in shared memory, 325 us.  What bounds it: instruction latency (0.51 instructions a cycle and scheduler, tensor pipe 12 %).
 constexpr int TCW_AW = 16;                      // warps of T
 constexpr int TC_THREADS = 32 * 21;
 constexpr int TCW_TILE = 64;
@@ -766,7 +767,7 @@ extern "C" __global__ void __launch_bounds__(TC_THREADS, 1) oeq_uvw_tc_backward_
                         for (int e = 0; e < 8; ++e) {
                             const float v = tc_half(t[e >> 1], e & 1);
                             hi[e] = tc_tf32(v);
-                            lo[e] = v - hi[e];   // truncated by the tensor core: below 2^-21
+                            lo[e] = v - hi[e];   // (12 bits, of which the tensor core reads 11)
                         }
                         tcw_st(ta + 64u * ring, hi);
                         tcw_st(ta + 64u * ring + 32u, lo);

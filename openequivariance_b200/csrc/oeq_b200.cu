@@ -318,12 +318,12 @@ bool parse_desc(const char* text, size_t len, Desc& d, std::string& why) {
         d.tc_zero_z = d.tc_zero_dx = false;
         for (int h : hit) d.tc_zero_z = d.tc_zero_z || !h;
         for (int h : read) d.tc_zero_dx = d.tc_zero_dx || !h;
-        long long npath = 0;   // 32 x 32 weight tiles: the per-path tables live in constant memory
+        long long npath = 0;   // 32 x 32 weight tiles: what the index tables and the weight gradient's partial rows grow with
         if (ok) for (auto& I : d.ins) npath += (long long)(d.L[0][I.a].mul / 32) * (d.L[2][I.o].mul / 32);
         ok = ok && npath <= 1024 && !d.ins.empty();
-        // The tensor cores add into their accumulators with truncation: measured ~1e-6 + 5.5e-9 per accumulated product.  The
-        // sums of the forward (per output channel: the channels of every path into its block) and of the gradient of x (per
-        // input channel) are kept below 1,280 products, which stays inside the 1e-5 bound.
+        // At most 1,280 products per output channel (and per input channel, for the gradients).  Accuracy does not ask for it: the tensor cores,
+        // which add with truncation, sum 32 of them at a time.  It is how far the kernels are tested and how much code a program may
+        // become (straight-line sums: 4 to 9 s to compile near the limit); wider problems run on the general kernels.
         if (ok) {
             std::vector<long long> into(d.L[2].size(), 0), from(d.L[0].size(), 0);
             for (auto& I : d.ins) { into[I.o] += d.L[0][I.a].mul; from[I.a] += d.L[2][I.o].mul; }
